@@ -19,6 +19,7 @@
 #include "gemm.cuh"
 #include "gemm32.cuh"
 #include "qr_blocked.cuh"
+#include "qr_cols.cuh"
 #include "kernels_misc.cuh"
 #include "linalg.cuh"
 #include "update.cuh"
@@ -58,6 +59,10 @@ struct alfgpu_s {
   zd *lo_acc[2] = {nullptr, nullptr}, *lo_acc0[2] = {nullptr, nullptr};
   double* lo_cnt[2] = {nullptr, nullptr};
   int oz = 0, eexp_complex = 0;
+  // a vertex table with a complex exponential or transition factor was uploaded (or
+  // ALFGPU_FLAG_COMPLEX_ARITH): otherwise every matrix of the sweep is real and the FP64 kernels
+  // that have a real form run it (ArRe; the matrices stay complex128 in memory)
+  int model_complex = 0;
   int oz_narrow = 0;  // small grids: BN = 16 tiles; the flush keeps the double-float GEMM (measured faster there)
   int oz_stab = 0;    // the stabilisation's complex products on the tensor-core GEMM too
   zd *ozGm = nullptr, *ozTm = nullptr, *ozWm = nullptr, *ozXm = nullptr;  // compact-WY explicit Q work
@@ -79,6 +84,8 @@ struct alfgpu_s {
   int CLr = 1;                       // k_qrp_rows cluster size (CL, or CL / 2 on batched grids)
   zd* qrr_ws = nullptr;              // row workspace of k_qrp_rows<ArD, true> (qrr_ok == 2)
   int qr2_mode = 0, CL2 = 1;         // CGR2_2's 2N x 2N QR: 0 k_qrp, 1 / 2 as qrr_ok; its cluster size
+  // cluster size of k_qrp_cols, [0] complex, [1] real; 0: not used.  qrc_cl: N x N, qrc2_cl: 2N x 2N
+  int qrc_cl[2] = {0, 0}, qrc2_cl[2] = {0, 0};
   zd* qr2_ws = nullptr;
   // time-displaced Green functions (ltau = 1)
   int ltau = 0;
@@ -364,6 +371,81 @@ static int qrr_plan(int N, int CL, int B, int flags, int dev, int* CLout) {
   return best;
 }
 
+// Cluster size of the exact pivoted QR with columns in shared memory (k_qrp_cols) for B matrices
+// N x N, 0 where it is not used: the columns do not fit, or (complex) the clusters of a batched
+// launch need a second wave, where k_qrp_rows' global rows win (32 matrices, N = 256: 5.7 ms
+// against 6.7 ms).  Measured (ms, one QR, real unless said otherwise):
+//   2 matrices   N = 64: CL 4 0.200, 8 0.199;  144: 4 0.574, 8 0.513, 16 0.574;  256: 8 1.19, 16 1.17;
+//                288: 8 1.53, 16 1.40;  complex 256: 8 2.68, 16 2.23
+//   8 matrices   144: 8 0.512, 16 0.619;  256: 8 1.19, 16 1.33;  288: 8 1.53, 16 1.61
+//   32 matrices  144: 4 0.577, 8 0.626;  196: 8 1.05, 16 1.58;  256: 8 1.64, 16 2.23
+// so: eight CTAs, sixteen for a few large matrices, four where eight would need more CTAs than
+// SMs and four hold the work (N <= 160), fewer for small N.
+static int qrc_plan(int N, int B, int real, int flags, int dev) {
+  if (flags & (ALFGPU_FLAG_QR_GLOBAL_ROWS | ALFGPU_FLAG_QR_HALF_CLUSTER | ALFGPU_FLAG_QR_FULL_CLUSTER |
+               ALFGPU_FLAG_QR_TWO_PASS))
+    return 0;  // options of the row-distributed kernel
+  int nsm = 152;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int zb = real ? 8 : 16;
+  int cl = N >= 96 ? 8 : (N >= 32 ? 4 : (N >= 16 ? 2 : 1));
+  if (cl == 8 && N <= 160 && 8 * B > nsm) cl = 4;
+  if (N > 224 && 16 * B <= nsm / 2) cl = 16;
+  for (; cl <= 16; cl *= 2) {
+    const size_t sm = qrc_smem_bytes(N, cl, zb);
+    if (sm > 227 * 1024) continue;
+    const void* fn = real ? (const void*)k_qrp_cols<ArRe> : (const void*)k_qrp_cols<ArD>;
+    cudaError_t e = real ? raise_smem_limit(k_qrp_cols<ArRe>, sm) : raise_smem_limit(k_qrp_cols<ArD>, sm);
+    if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    int n = 0;
+    if (e == cudaSuccess) {
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(cl, 1, 1);
+      cfg.blockDim = dim3(QRC_THREADS, 1, 1);
+      cfg.dynamicSmemBytes = sm;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cl; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      cfg.attrs = at; cfg.numAttrs = 1;
+      e = real ? cudaOccupancyMaxActiveClusters(&n, k_qrp_cols<ArRe>, &cfg)
+               : cudaOccupancyMaxActiveClusters(&n, k_qrp_cols<ArD>, &cfg);
+    }
+    cudaGetLastError();
+    if (e != cudaSuccess || n <= 0) continue;
+    if (!real && n < B && cl < 16) continue;
+    if (!real && n < B) return 0;
+    return cl;
+  }
+  return 0;
+}
+
+static int launch_qrc(alfgpu_s* h, const zd* Ain, zd* A, int N, int CL, int real, zd* tau, int* jpvt, double* D,
+                      QRInfo* info, const double* colscale) {
+  const long long NN = (long long)N * N;
+  QRColsParams q;
+  memset(&q, 0, sizeof(q));
+  q.Ain = Ain; q.A = A; q.lda = N; q.sA = NN; q.N = N;
+  q.colscale = colscale; q.sCS = N;
+  q.tau = tau; q.sT = N; q.jpvt = jpvt; q.sP = N; q.D = D; q.sD = N; q.info = info;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(CL, h->B, 1);
+  cfg.blockDim = dim3(QRC_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = qrc_smem_bytes(N, CL, real ? 8 : 16);
+  cfg.stream = h->st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  h->launches++;
+  if (real) CK(cudaLaunchKernelEx(&cfg, k_qrp_cols<ArRe>, q));
+  else CK(cudaLaunchKernelEx(&cfg, k_qrp_cols<ArD>, q));
+  k_bqr_finish<<<dim3((N + 7) / 8, h->B), 256, (size_t)N * sizeof(double), h->st>>>(A, N, NN, N, tau, N, D, N, info);
+  CKL();
+  return 0;
+}
+
 // One launch of the exact pivoted QR on clusters of CL CTAs (rows in shared memory, or in ws when
 // grows), then k_bqr_finish: R (normalised rows) above, reflectors below, tau, jpvt, D, info.
 static int launch_qrr(alfgpu_s* h, const zd* Ain, zd* A, int N, int CL, bool grows, zd* ws, zd* tau, int* jpvt,
@@ -400,6 +482,9 @@ static int launch_qrr(alfgpu_s* h, const zd* Ain, zd* A, int N, int CL, bool gro
 // ---------------------------------------------------------------------------
 // Kernel launch helpers
 // ---------------------------------------------------------------------------
+// The FP64 kernels may take every matrix as real.
+static int real_model(const alfgpu_s* h) { return h->vert_ok && !h->model_complex; }
+
 static int launch_qr(alfgpu_s* h, zd* A, const double* colscale, int nb) {
   prof_begin(h, ALFGPU_PROF_QR);
   QRParams q;
@@ -665,6 +750,13 @@ static int qr_any(alfgpu_s* h, const zd* Ain, const double* colscale, zd* Aout, 
   h->exact_qrp = exact;
   h->qr_df = 0;
   const dim3 g8((N + 7) / 8, B);
+  const int real = real_model(h), qrc = h->qrc_cl[real];
+  if (exact && qrc && !df) {
+    prof_begin(h, ALFGPU_PROF_QR);
+    RET(launch_qrc(h, Ain, Aout, N, qrc, real, h->tau, h->jpvt, h->DUP, h->info, colscale));
+    prof_end(h);
+    return 0;
+  }
   if (exact && !h->qrr_ok) {
     RET(copy_mats(h, Aout, Ain, (size_t)B * NN));
     return launch_qr(h, Aout, colscale, B);
@@ -1226,6 +1318,8 @@ static int obs_tau(alfgpu_s* h, alfgpu_obs_cb cb, void* ctx, int nt) {
 // ---- CGR2_2 ---------------------------------------------------------------------------------
 // Column-pivoted QR (ZGEQP3 semantics, cluster kernel) of the N2 x N2 matrices A in place.
 static int qrp_n(alfgpu_s* h, zd* A, int N2, zd* tau, int* jpvt, double* D, double* vn, QRInfo* info) {
+  const int real = real_model(h);
+  if (h->qrc2_cl[real]) return launch_qrc(h, A, A, N2, h->qrc2_cl[real], real, tau, jpvt, D, info, nullptr);
   if (h->qr2_mode)  // the row-distributed cluster QR, in place (rows read before any output is written)
     return launch_qrr(h, A, A, N2, h->CL2, h->qr2_mode == 2, h->qr2_ws, tau, jpvt, D, info, nullptr, 0);
   QRParams q;
@@ -1803,6 +1897,7 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   h->df_stab = h->mixed && (d.reserved[0] & ALFGPU_FLAG_DF_STAB_GEMM);
   h->df_qr = h->mixed && (d.reserved[0] & ALFGPU_FLAG_DF_STAB_QR);
   h->use_graph = !(d.reserved[0] & ALFGPU_FLAG_NO_GRAPH);
+  h->model_complex = (d.reserved[0] & ALFGPU_FLAG_COMPLEX_ARITH) ? 1 : 0;
   fill_tables(h->ft);
   auto fail = [&](int code) { alfgpu_destroy(h); return code; };
   if (cudaSetDevice(d.device) != cudaSuccess) return fail(ALFGPU_ERROR_CUDA);
@@ -1852,6 +1947,10 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   // workspace per CTA (mode 2) instead of falling back to the column-distributed k_qrp.
   h->CLr = h->CL;
   h->qrr_ok = qrr_plan(h->N, h->CL, h->B, d.reserved[0], h->dev, &h->CLr);
+  for (int real = 0; real < 2; ++real) {
+    h->qrc_cl[real] = qrc_plan(h->N, h->B, real, d.reserved[0], h->dev);
+    if (d.ltau) h->qrc2_cl[real] = qrc_plan(2 * h->N, h->B, real, d.reserved[0], h->dev);
+  }
   if (d.ltau) h->qr2_mode = qrr_plan(2 * d.ndim, cluster_size(2 * d.ndim), h->B, d.reserved[0], h->dev, &h->CL2);
   // the blocked QR keeps at most BQR_ROWS panel rows per CTA and BQR_LROWS rows per lane
   if (h->N > 32 * BQR_LROWS || (h->N + h->CL - 1) / h->CL > BQR_ROWS) h->exact_dec = h->exact_cgr = 1;
@@ -2088,7 +2187,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
       for (int s = 0; s < 5; ++s)
         ee[k * 10 + m * 5 + s] = zmk(v->op_Eexp[(k * 10 + m * 5 + s) * 2], v->op_Eexp[(k * 10 + m * 5 + s) * 2 + 1]);
     for (int s = 0; s < 10; ++s)
-      if (ee[k * 10 + s].y != 0.0) h->eexp_complex = 1;
+      if (ee[k * 10 + s].y != 0.0) h->eexp_complex = h->model_complex = 1;
     if (!std::isfinite(g[k].x) || !std::isfinite(g[k].y)) return ALFGPU_ERROR_HAMILTONIAN;
   }
   // the vertices of every flavour act on the same sites
@@ -2182,6 +2281,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
         }
         const std::complex<double> ea = std::exp(Z1 * std::complex<double>(al[k].x, al[k].y));
         e.expal = zmk(ea.real(), ea.imag());
+        if (e.myexp[0].y != 0.0 || e.myexp[1].y != 0.0 || e.expal.y != 0.0) h->model_complex = 1;
       }
   }
   // positions of each site, ascending (vertex n, eigen-index I) -> 2n + I, per flavour

@@ -10,7 +10,7 @@
 struct ArD {
   typedef zd Z;
   typedef double R;
-  static constexpr bool kDoubleFloat = false;
+  static constexpr bool kDoubleFloat = false, kReal = false;
   static ALF_DEV Z mk(zd a) { return a; }
   static ALF_DEV zd wide(Z a) { return a; }
   static ALF_DEV R mkr(double a) { return a; }
@@ -53,6 +53,8 @@ struct ArD {
   static ALF_DEV Z mkz(R r, R i) { return zmk(r, i); }
   static ALF_DEV R im(Z a) { return a.y; }
   static ALF_DEV R abs2(Z a) { return a.x * a.x + a.y * a.y; }
+  static ALF_DEV R abs2add(Z a, R s) { return fma(a.x, a.x, fma(a.y, a.y, s)); }
+  static ALF_DEV R abs2sub(R s, Z a) { return fma(-a.x, a.x, fma(-a.y, a.y, s)); }
   static ALF_DEV R rzero() { return 0.0; }
   static ALF_DEV R radd(R a, R b) { return a + b; }
   static ALF_DEV R rsub(R a, R b) { return a - b; }
@@ -75,7 +77,7 @@ struct ArD {
 struct ArF {
   typedef dfz Z;
   typedef dff R;
-  static constexpr bool kDoubleFloat = true;
+  static constexpr bool kDoubleFloat = true, kReal = false;
   static ALF_DEV Z mk(zd a) { return dz_make(a); }
   static ALF_DEV zd wide(Z a) { return dz_wide(a); }
   static ALF_DEV R mkr(double a) { return df_make(a); }
@@ -130,3 +132,48 @@ struct ArF {
   }
 };
 
+// Real FP64: the plain form on models whose vertex exponentials and transition factors are all
+// real (the hopping exponentials always are).  Every matrix of the sweep then has zero imaginary
+// parts, and ArD's complex products spend three of four FP64 instructions on them; the real
+// parts come out of the same operations in the same order.  Matrices stay complex128 in memory
+// (mk takes the real part, wide writes a zero imaginary part).
+struct ArRe {
+  typedef double Z;
+  typedef double R;
+  static constexpr bool kDoubleFloat = false, kReal = true;
+  static ALF_DEV Z mk(zd a) { return a.x; }
+  static ALF_DEV zd wide(Z a) { return zmk(a, 0.0); }
+  static ALF_DEV R mkr(double a) { return a; }
+  static ALF_DEV Z one() { return 1.0; }
+  static ALF_DEV Z zero() { return 0.0; }
+  static ALF_DEV Z mul(Z a, Z b) { return a * b; }
+  static ALF_DEV Z sub(Z a, Z b) { return a - b; }
+  static ALF_DEV Z add(Z a, Z b) { return a + b; }
+  static ALF_DEV Z neg(Z a) { return -a; }
+  static ALF_DEV Z mac(Z c, Z a, Z b) { return fma(a, b, c); }
+  static ALF_DEV Z scale(Z a, R s) { return a * s; }
+  static ALF_DEV R re(Z a) { return a; }
+  static ALF_DEV R im(Z) { return 0.0; }
+  static ALF_DEV R mulr(R a, R b) { return a * b; }
+  static ALF_DEV bool gt(R a, R b) { return a > b; }
+  static ALF_DEV Z rcp(Z a) { return ArD::rrcp(a); }
+  static ALF_DEV Z shfl(Z a, int src) { return __shfl_sync(0xffffffffu, a, src); }
+  static ALF_DEV Z shfl_xor(Z a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+  static ALF_DEV Z conj(Z a) { return a; }
+  static ALF_DEV Z mkz(R r, R) { return r; }
+  static ALF_DEV R abs2(Z a) { return a * a; }
+  static ALF_DEV R abs2add(Z a, R s) { return fma(a, a, s); }
+  static ALF_DEV R abs2sub(R s, Z a) { return fma(-a, a, s); }
+  static ALF_DEV R rzero() { return 0.0; }
+  static ALF_DEV R radd(R a, R b) { return a + b; }
+  static ALF_DEV R rsub(R a, R b) { return a - b; }
+  static ALF_DEV R rneg(R a) { return -a; }
+  static ALF_DEV R rsqrt_(R a) { return sqrt(a); }
+  static ALF_DEV R rrcp(R a) { return ArD::rrcp(a); }
+  static ALF_DEV R rmax0(R a) { return a > 0.0 ? a : 0.0; }
+  static ALF_DEV bool rzero_p(R a) { return a == 0.0; }
+  static ALF_DEV bool rneg_p(R a) { return a < 0.0; }
+  static ALF_DEV double rwide(R a) { return a; }
+  static ALF_DEV R rcopysign(R mag, R sgn) { return copysign(mag, sgn); }
+  static ALF_DEV R rshfl_xor(R a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+};

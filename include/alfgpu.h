@@ -145,6 +145,10 @@ enum { ALFGPU_FLAG_OZ_FLUSH_RESIDENT = 262144 };
 /* The exact pivoted QR applies each step's reflector and forms the next step's partial sums in
  * two passes over the rows (by default one pass does both, the next pivot chosen first). */
 enum { ALFGPU_FLAG_QR_TWO_PASS = 524288 };
+/* Models whose vertex exponentials and transition factors are all real keep every matrix of the
+ * sweep real (the hopping exponentials are), and the FP64 kernels then skip the products with the
+ * zero imaginary parts.  This flag keeps the complex products. */
+enum { ALFGPU_FLAG_COMPLEX_ARITH = 1048576 };
 
 /* dims.reserved[1] / dims.reserved[2] (mixed form, tensor-core products only): target bits of
  * the digit-sliced products of the G wraps and TAU_M's propagation (reserved[1]) and of the

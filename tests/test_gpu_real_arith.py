@@ -1,0 +1,72 @@
+"""The real forms of the FP64 kernels (models whose vertices are all real) and the
+column-distributed pivoted QR, at sizes around their tiles, against the CPU oracle and against
+the complex products of the same model (FLAG_COMPLEX_ARITH).
+
+G at every stabilisation point within 1e-10 relative of the oracle's, the plain form's bound;
+D of a decomposition within 1e-10 relative and its reconstruction within 1e-10 (the bounds of
+the parity tests)."""
+import numpy as np
+import pytest
+
+import oracle
+from alf_gb300 import model as mdl, rng
+from alf_gb300.sweep import FLAG_COMPLEX_ARITH, Chains, decompose as gpu_decompose
+from parity_util import compare_record
+
+pytestmark = pytest.mark.gpu
+
+
+def _relmax(a, b):
+    return np.max(np.abs(a - b)) / max(np.max(np.abs(b)), 1e-300)
+
+
+def _record(m, flags, f0, u, precision="fp64", chains=1):
+    g = Chains(m, n_chains=chains, precision=precision, flags=flags)
+    for c in range(chains):
+        g.set_fields(c, f0)
+    g.init_state()
+    g.set_recording(True)
+    g.sweep(np.stack([u] * chains))
+    r = [g.record(c) for c in range(chains)]
+    f = g.fields(chains - 1)
+    g.close()
+    return r, f
+
+
+# N = 9 .. 225: one to sixteen columns per CTA, row counts around 8, 16, 32, 64, 128, 224
+@pytest.mark.parametrize("L1,L2", [(3, 3), (4, 4), (5, 3), (3, 11), (8, 8), (5, 13), (9, 11), (15, 15)])
+def test_real_sweep_matches_oracle_and_complex_products(L1, L2):
+    m = mdl.hubbard("square", L1, L2, U=4.0, beta=0.8, dtau=0.1, nwrap=3)
+    f0 = rng.initial_fields(5, 0, m.n_op, m.ltrot)
+    u = rng.sweep_uniforms(5, 0, m.n_op, m.ltrot, 0)
+    (rr,), fr = _record(m, 0, f0, u)
+    (rc,), fc = _record(m, FLAG_COMPLEX_ARITH, f0, u)
+    o = oracle.Oracle(m)
+    o.set_fields(f0)
+    o.init_state()
+    o.record(1)
+    o.sweep(u)
+    ro = o.recorded()
+    compare_record(rr, ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=1e-10, relative=True, exact_sequence=True,
+                   ratio_median=1e-12)
+    assert np.array_equal(rr["acc"], rc["acc"]) and np.array_equal(fr, fc)
+    assert _relmax(rr["G"], rc["G"]) <= 1e-10
+    assert np.all(rr["G"].imag == 0.0)
+
+
+# the QR's cluster sizes (1, 2, 4, 8, 16 CTAs) and its column and row remainders
+@pytest.mark.parametrize("N", [1, 2, 15, 16, 17, 31, 33, 95, 97, 130, 225, 321])
+@pytest.mark.parametrize("side", ["r", "l"])
+def test_decompose_sizes(N, side):
+    rs = np.random.default_rng(N)
+    X = rs.standard_normal((N, N)) + 1j * rs.standard_normal((N, N))
+    D = 10.0 ** rs.uniform(-8, 8, N)
+    V = np.eye(N) + np.triu(rs.standard_normal((N, N)), 1) * (0.3 / np.sqrt(N))
+    # copies: a 1 x 1 transpose is a view, and the wrappers decompose in place
+    U, d, W = gpu_decompose(side, X.copy(), D.astype(complex), V.astype(complex))
+    _, do, _ = oracle.decompose(side, X.copy(), D.astype(complex), V.astype(complex))
+    A = (X * D) @ (V if side == "r" else V.conj().T)
+    R = U @ np.diag(d) @ (W if side == "r" else W.conj().T)
+    assert np.max(np.abs(d / do - 1.0)) < 1e-10
+    assert _relmax(R, A) < 1e-10
+    assert np.max(np.abs(U.conj().T @ U - np.eye(N))) < 1e-12
