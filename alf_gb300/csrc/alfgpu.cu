@@ -479,12 +479,12 @@ static int launch_qrr(alfgpu_s* h, const zd* Ain, zd* A, int N, int CL, bool gro
   return 0;
 }
 
-// ---------------------------------------------------------------------------
-// Kernel launch helpers
-// ---------------------------------------------------------------------------
 // The FP64 kernels may take every matrix as real.
 static int real_model(const alfgpu_s* h) { return h->vert_ok && !h->model_complex; }
 
+// ---------------------------------------------------------------------------
+// Kernel launch helpers
+// ---------------------------------------------------------------------------
 static int launch_qr(alfgpu_s* h, zd* A, const double* colscale, int nb) {
   prof_begin(h, ALFGPU_PROF_QR);
   QRParams q;
@@ -535,17 +535,25 @@ static int launch_orgqr(alfgpu_s* h, zd* A, int nb) {
 }
 
 
-// Triangular solves (ZTRSM) of p.nvec right-hand sides per matrix: TRSV_V vectors per CTA
-// when their shared memory fits, else one per CTA.
-static int trsv(alfgpu_s* h, const TrsvParams& t) {
-  const size_t sm = trsv_v_smem(t.N);
-  if (sm <= 200 * 1024 && raise_smem_limit(k_trsv_v<TRSV_V>, sm) == cudaSuccess) {
-    k_trsv_v<TRSV_V><<<dim3((t.nvec + TRSV_V - 1) / TRSV_V, h->B), 256, sm, h->st>>>(t);
-  } else {
-    cudaGetLastError();
-    k_trsv<<<dim3(t.nvec, h->B), 256, 3 * (size_t)t.N * sizeof(zd), h->st>>>(t);
-  }
+// Triangular solves (ZTRSM) of t.nvec right-hand sides per matrix: eight vectors per CTA once
+// that fills the SMs, else four or two (each halving shortens a CTA's share of the products).
+template <class A, int V>
+static int trsv_launch(alfgpu_s* h, const TrsvParams& t) {
+  const size_t sm = trsv_b_smem(t.N, V, (int)sizeof(typename A::Z));
+  CK(raise_smem_limit(k_trsv_b<A, V>, sm));
+  k_trsv_b<A, V><<<dim3((t.nvec + V - 1) / V, h->B), 256, sm, h->st>>>(t);
   return 0;  // the caller checks the launch (CKL)
+}
+template <class A>
+static int trsv_any(alfgpu_s* h, const TrsvParams& t) {
+  const long long vecs = (long long)t.nvec * h->B;
+  const size_t zb = sizeof(typename A::Z), cap = 200 * 1024;
+  if (vecs >= 8 * 152 && trsv_b_smem(t.N, 8, (int)zb) <= cap) return trsv_launch<A, 8>(h, t);
+  if (vecs >= 4 * 76 && trsv_b_smem(t.N, 4, (int)zb) <= cap) return trsv_launch<A, 4>(h, t);
+  return trsv_launch<A, 2>(h, t);
+}
+static int trsv(alfgpu_s* h, const TrsvParams& t) {
+  return real_model(h) ? trsv_any<ArRe>(h, t) : trsv_any<ArD>(h, t);
 }
 
 static int gemm(alfgpu_s* h, const GemmParams& p) {
@@ -796,7 +804,8 @@ static int qr_any(alfgpu_s* h, const zd* Ain, const double* colscale, zd* Aout, 
       ap.V = Aout; ap.ldv = N; ap.sV = NN; ap.tau = h->tau; ap.sT = N;
       ap.C = Aout; ap.ldc = N; ap.sC = NN;
       ap.N = N; ap.j0 = j0; ap.nb = w; ap.c0 = j0 + w; ap.conj_tau = 1; ap.init = 0;
-      bqr_apply<ArD>(ap, dim3(N - j0 - w, B), h->st);
+      if (real_model(h)) bqr_apply<ArRe>(ap, dim3(N - j0 - w, B), h->st);
+      else bqr_apply<ArD>(ap, dim3(N - j0 - w, B), h->st);
       CKL();
     }
   }
@@ -877,8 +886,10 @@ static int orgqr_wy(alfgpu_s* h, const zd* F, zd* Q) {
 static int orgqr_any(alfgpu_s* h, const zd* F, zd* Q) {
   const int N = h->N, B = h->B;
   const long long NN = (long long)N * N;
-  // compact WY pays on batched grids; one chain's grid is too small for its launch chain
-  if (h->oz_stab && !h->oz_narrow && !h->qr_df && N <= 32 * BQR_LROWS) return orgqr_wy(h, F, Q);
+  // compact WY pays on batched grids of complex matrices; one chain's grid is too small for its
+  // launch chain, and real columns take a quarter of the FP64 instructions (16 chains, N = 256,
+  // per sweep: compact WY 110 ms, real columns 70 ms)
+  if (h->oz_stab && !h->oz_narrow && !h->qr_df && !real_model(h) && N <= 32 * BQR_LROWS) return orgqr_wy(h, F, Q);
   if (N > 32 * BQR_LROWS) {  // beyond the rows a lane of k_bqr_apply holds
     RET(copy_mats(h, Q, F, (size_t)B * NN));
     return launch_orgqr(h, Q, B);
@@ -891,6 +902,7 @@ static int orgqr_any(alfgpu_s* h, const zd* F, zd* Q) {
     ap.C = Q; ap.ldc = N; ap.sC = NN;
     ap.N = N; ap.j0 = j0; ap.nb = w; ap.c0 = j0; ap.conj_tau = 0; ap.init = 1;
     if (h->qr_df) bqr_apply<ArF>(ap, dim3(N - j0, B), h->st);
+    else if (real_model(h)) bqr_apply<ArRe>(ap, dim3(N - j0, B), h->st);
     else bqr_apply<ArD>(ap, dim3(N - j0, B), h->st);
     CKL();
   }
@@ -1351,7 +1363,8 @@ static int unmqr_n(alfgpu_s* h, const zd* F, const zd* tau, zd* Cm, int N2) {
     ap.V = F; ap.ldv = N2; ap.sV = NN2; ap.tau = tau; ap.sT = N2;
     ap.C = Cm; ap.ldc = N2; ap.sC = NN2;
     ap.N = N2; ap.j0 = j0; ap.nb = w; ap.c0 = 0; ap.conj_tau = 0; ap.init = 0;
-    bqr_apply<ArD>(ap, dim3(N2, h->B), h->st);
+    if (real_model(h)) bqr_apply<ArRe>(ap, dim3(N2, h->B), h->st);
+    else bqr_apply<ArD>(ap, dim3(N2, h->B), h->st);
     CKL();
   }
   return 0;
@@ -1389,11 +1402,14 @@ static int cgr2_2(alfgpu_s* h, const UDVSet& udv2, const UDVSet& udv1) {
   k_cgr22_hlp<<<gN2, 256, 0, h->st>>>(h->HB2, h->jpvt2, h->HLP, N);
   CKL();
   {
-    TrsvParams t{};
-    t.T = h->HB1; t.ldt = N2; t.sT = NN2; t.B = h->HLP; t.vstride = N2; t.estride = 1; t.sB = NN2;
-    t.N = N2; t.nvec = N2; t.lower = 1; t.conj_io = 0; t.trans = 1;
-    t.oscale = nullptr;
+    // R^H as a stored lower triangle: its columns are then contiguous for the solve
     prof_begin(h, ALFGPU_PROF_SOLVE);
+    k_transpose<<<dim3((N2 + 31) / 32, (N2 + 31) / 32, B), dim3(32, 8), 0, h->st>>>(h->HB1, N2, NN2, h->HB2, N2, NN2, N2,
+                                                                                    1);
+    CKL();
+    TrsvParams t{};
+    t.T = h->HB2; t.ldt = N2; t.sT = NN2; t.B = h->HLP; t.vstride = N2; t.estride = 1; t.sB = NN2;
+    t.N = N2; t.nvec = N2; t.lower = 1; t.conj_io = 0;
     RET(trsv(h, t));
     prof_end(h);
     CKL();

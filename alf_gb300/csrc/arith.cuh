@@ -12,6 +12,9 @@ struct ArD {
   typedef double R;
   static constexpr bool kDoubleFloat = false, kReal = false;
   static ALF_DEV Z mk(zd a) { return a; }
+  typedef zd S;  // element of a matrix held in this arithmetic in memory
+  static ALF_DEV Z ld(S a) { return a; }
+  static ALF_DEV Z inv(Z a) { return zinv(a); }
   static ALF_DEV zd wide(Z a) { return a; }
   static ALF_DEV R mkr(double a) { return a; }
   static ALF_DEV Z one() { return zmk(1.0, 0.0); }
@@ -79,6 +82,8 @@ struct ArF {
   typedef dff R;
   static constexpr bool kDoubleFloat = true, kReal = false;
   static ALF_DEV Z mk(zd a) { return dz_make(a); }
+  typedef dfz S;
+  static ALF_DEV Z ld(S a) { return a; }
   static ALF_DEV zd wide(Z a) { return dz_wide(a); }
   static ALF_DEV R mkr(double a) { return df_make(a); }
   static ALF_DEV Z one() { return dfz{{1.f, 0.f}, {0.f, 0.f}}; }
@@ -142,6 +147,9 @@ struct ArRe {
   typedef double R;
   static constexpr bool kDoubleFloat = false, kReal = true;
   static ALF_DEV Z mk(zd a) { return a.x; }
+  typedef zd S;
+  static ALF_DEV Z ld(S a) { return a.x; }
+  static ALF_DEV Z inv(Z a) { return 1.0 / a; }
   static ALF_DEV zd wide(Z a) { return zmk(a, 0.0); }
   static ALF_DEV R mkr(double a) { return a; }
   static ALF_DEV Z one() { return 1.0; }

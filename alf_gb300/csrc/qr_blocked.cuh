@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(32 * WPC) k_bqr_apply(BQRApply p) {
   if (c >= p.N) return;
   const int N = p.N, j0 = p.j0, nb = p.nb;
   const int nblk = (N - j0 + 31) >> 5;  // 32-row blocks
-  const Z* V = reinterpret_cast<const Z*>(p.V) + b * p.sV;
+  const typename A::S* V = reinterpret_cast<const typename A::S*>(p.V) + b * p.sV;
   constexpr int NWc = WPC;
   const zd* tau = p.tau + b * p.sT;
   zd* col = p.C + b * p.sC + (long long)c * p.ldc;
@@ -273,13 +273,13 @@ __global__ void __launch_bounds__(32 * WPC) k_bqr_apply(BQRApply p) {
   }
   auto load_v = [&](int k) {
     const int kc = j0 + k, blo = (kc - j0) >> 5;
-    const Z* v = V + (long long)kc * p.ldv;
+    const typename A::S* v = V + (long long)kc * p.ldv;
 #pragma unroll
     for (int q = 0; q < BQR_QW; ++q) {
       const int blk = w + NWc * q;
       if (blk < blo || blk >= nblk) continue;
       const int r = j0 + lane + 32 * blk;
-      vn[q] = (r < kc || r >= N) ? A::zero() : (r == kc ? A::one() : v[r]);
+      vn[q] = (r < kc || r >= N) ? A::zero() : (r == kc ? A::one() : A::ld(v[r]));
     }
   };
   load_v(p.conj_tau ? 0 : nb - 1);
@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(32 * WPC) k_bqr_apply(BQRApply p) {
     if (NWc > 1) {
       if (lane == 0) red[par][w] = s;
       __syncthreads();
-      tot = A::add(A::add(red[par][0], red[par][1]), A::add(red[par][2], red[par][3]));
+      tot = A::add(red[par][0], red[par][1]);
+      if (NWc > 2) tot = A::add(tot, A::add(red[par][2], red[par][3]));
       par ^= 1;
     }
     const Z f = A::neg(A::mul(A::mk(t), tot));
@@ -333,7 +334,28 @@ template <class A>
 static inline void bqr_apply(const BQRApply& ap, dim3 grid, cudaStream_t st) {
   const int rows = ap.N - ap.j0;
   const long long cols = (long long)grid.x * grid.y;
-  if (cols >= 4 * 152 && rows <= 256) {  // (more rows per lane would spill)
+  if (A::kReal) {
+    // The FP64 instructions per reflector of the busiest sub-partition, for w warps per column:
+    // ceil(cols w / 608) warps, each 2 ceil(blocks / w) products, five shuffle additions, w - 1
+    // additions over the warps and the factor (one column's registers hold any number of rows).
+    const int blocks = (rows + 31) / 32;
+    long long best = 0;
+    int wpc = 1;
+    for (int w = 1; w <= 4; w *= 2) {
+      const long long cost = ((cols * w + 607) / 608) * (2 * ((blocks + w - 1) / w) + 5 + w);
+      if (w == 1 || cost < best) { best = cost; wpc = w; }
+    }
+    if (wpc == 1) {
+      if (blocks <= 8) k_bqr_apply<A, 8, 1><<<grid, 32, 0, st>>>(ap);
+      else k_bqr_apply<A, BQR_LROWS, 1><<<grid, 32, 0, st>>>(ap);
+    } else if (wpc == 2) {
+      if (blocks <= 8) k_bqr_apply<A, 4, 2><<<grid, 64, 0, st>>>(ap);
+      else k_bqr_apply<A, BQR_LROWS / 2, 2><<<grid, 64, 0, st>>>(ap);
+    } else {
+      if (blocks <= 8) k_bqr_apply<A, 2, 4><<<grid, 128, 0, st>>>(ap);
+      else k_bqr_apply<A, BQR_LROWS / 4, 4><<<grid, 128, 0, st>>>(ap);
+    }
+  } else if (cols >= 4 * 152 && rows <= 256) {  // (more rows per lane would spill)
     k_bqr_apply<A, 8, 1><<<grid, 32, 0, st>>>(ap);
   } else {
     if (rows <= 256) k_bqr_apply<A, 2, 4><<<grid, 128, 0, st>>>(ap);

@@ -70,3 +70,45 @@ def test_decompose_sizes(N, side):
     assert np.max(np.abs(d / do - 1.0)) < 1e-10
     assert _relmax(R, A) < 1e-10
     assert np.max(np.abs(U.conj().T @ U - np.eye(N))) < 1e-12
+
+
+# right-hand sides per CTA (2, 4, 8), row blocks of 32 and their remainders, both solve
+# directions, complex factors
+@pytest.mark.parametrize("N", [1, 5, 31, 32, 33, 64, 100, 257, 320])
+@pytest.mark.parametrize("nvar", [1, 2])
+def test_cgr_sizes(N, nvar):
+    from alf_gb300.sweep import cgr as gpu_cgr
+    rs = np.random.default_rng(1000 + N)
+    q = lambda: np.linalg.qr(rs.standard_normal((N, N)) + 1j * rs.standard_normal((N, N)))[0]
+    UR, UL = q(), q()
+    VR, VL = (np.eye(N) + np.triu(rs.standard_normal((N, N)) + 1j * rs.standard_normal((N, N)), 1) * (0.3 / np.sqrt(N))
+              for _ in range(2))
+    DR = np.sort(10.0 ** rs.uniform(-6, 6, N))[::-1].astype(complex)
+    DL = np.sort(10.0 ** rs.uniform(-6, 6, N))[::-1].astype(complex)
+    G, ph = gpu_cgr(nvar, UR.copy(), DR, VR.copy(), UL.copy(), DL, VL.copy())
+    Go, pho = oracle.cgr(nvar, UR.copy(), DR, VR.copy(), UL.copy(), DL, VL.copy())
+    assert _relmax(G, Go) < 1e-10
+    assert abs(ph - pho) < 1e-10
+
+
+# batched real solves and Q columns (eight vectors per CTA, one warp per column), and TAU_M's 2N
+# system, against the complex products: the quartets within 1e-10 of their largest entry
+@pytest.mark.parametrize("chains,L1,L2", [(1, 4, 3), (6, 7, 5), (9, 9, 8)])
+def test_real_tau_matches_complex_products(chains, L1, L2):
+    m = mdl.hubbard("square", L1, L2, U=4.0, beta=0.8, dtau=0.1, nwrap=3)
+    u = np.stack([rng.sweep_uniforms(7, c, m.n_op, m.ltrot, 0) for c in range(chains)])
+    out = []
+    for flags in (0, FLAG_COMPLEX_ARITH):
+        g = Chains(m, n_chains=chains, ltau=1, flags=flags)
+        for c in range(chains):
+            g.set_fields(c, rng.initial_fields(7, c, m.n_op, m.ltrot))
+        g.init_state()
+        _, tau = g.sweep(u, measure=True, keep=lambda k, c, nt: k == 1 and c in (0, chains - 1))
+        out.append((tau, [g.fields(c) for c in range(chains)]))
+        g.close()
+    (ta, fa), (tb, fb) = out
+    assert all(np.array_equal(x, y) for x, y in zip(fa, fb)) and len(ta) == len(tb) > 0
+    for (c, nt, qa, _), (c2, nt2, qb, _) in zip(ta, tb):
+        assert (c, nt) == (c2, nt2)
+        for a, b in zip(qa, qb):
+            assert _relmax(a, b) <= 1e-10
