@@ -177,7 +177,7 @@ struct alfgpu_s {
   QRInfo* info = nullptr;
   // delayed update
   int *m = nullptr, *sites = nullptr;
-  zd *W = nullptr, *X = nullptr, *Y = nullptr, *dlt = nullptr;
+  zd *W = nullptr, *X = nullptr, *Y = nullptr;
   // per chain
   zd* phase = nullptr;
   long long* cnt = nullptr;
@@ -1654,7 +1654,10 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
   // them (one CTA per SM by shared memory and TMEM), the paired tiles leave room for k_update
   const bool ozf = h->mixed && h->oz && !h->oz_narrow && !(h->d.reserved[0] & ALFGPU_FLAG_DF_FLUSH);
   const bool ov = h->overlap && (!ozf || h->ozf_pairs) && !h->pairblock && !h->profiling && nblk > 1;
-  const bool dfv = h->mixed && !(h->d.reserved[0] & ALFGPU_FLAG_FP64_VISITS);  // visits in double-float
+  // Visits in real FP64 on real models in both forms (28 us for 32 positions, 59 us in
+  // double-float), else in double-float in the mixed form.
+  const int real = real_model(h);
+  const bool dfv = h->mixed && !(h->d.reserved[0] & ALFGPU_FLAG_FP64_VISITS);
   const long long msz = (long long)h->C + h->B;
   VertexDev V;
   V.site = h->v_site; V.site2 = h->v_site2; V.nsite = h->v_nsite; V.type = h->v_type; V.sK = (long long)F * M;
@@ -1670,7 +1673,8 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       // (double-float here raised the mixed form's largest Precision Green from 9e-6 to 6e-5)
       const int* mprev = h->m + (long long)((blk - 1) & 1) * msz;
       const dim3 gs((UPD_KMAX + 7) / 8, h->B), bs(32, 8);
-      k_sub_stage<ArD><<<gs, bs, 0, su>>>(h->Gsnap, h->posn, h->npos, mprev, N, F, h->X, h->Y, h->Gsub);
+      if (real) k_sub_stage<ArRe><<<gs, bs, 0, su>>>(h->Gsnap, h->posn, h->npos, mprev, N, F, h->X, h->Y, h->Gsub);
+      else k_sub_stage<ArD><<<gs, bs, 0, su>>>(h->Gsnap, h->posn, h->npos, mprev, N, F, h->X, h->Y, h->Gsub);
       CKL();
     }
     UpdParams u;
@@ -1686,7 +1690,7 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
     u.fields = h->fields;
     u.draws = draws_dev; u.sDraws = 6ll * M * h->L;
     u.rngkey = h->rngkey; u.rngctr = h->rngctr;
-    u.phase = h->phase; u.m_out = mb; u.W = h->W; u.sites_out = h->sites; u.delta_out = h->dlt; u.cnt = h->cnt;
+    u.phase = h->phase; u.m_out = mb; u.W = h->W; u.sites_out = h->sites; u.cnt = h->cnt;
     u.Gsub = (ov && blk > 0) ? h->Gsub : nullptr;
     if (h->recording) { u.rec_acc = h->rec_acc; u.rec_ratio = h->rec_ratio; u.sRec = 2ll * M * h->L; }
     u.ft = h->ft;
@@ -1694,7 +1698,8 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       u.vsite2 = h->v_blk2; u.vcoef = h->v_vc; u.sites2_out = h->sites2_out; u.coef_out = h->coef_out;
     }
     prof_begin(h, ALFGPU_PROF_UPDATE);
-    if (dfv) k_update<ArF><<<h->C, UPD_THREADS, upd_smem_bytes(), su>>>(u);
+    if (real) k_update<ArRe><<<h->C, UPD_THREADS, upd_smem_bytes(8), su>>>(u);
+    else if (dfv) k_update<ArF><<<h->C, UPD_THREADS, upd_smem_bytes(), su>>>(u);
     else k_update<ArD><<<h->C, UPD_THREADS, upd_smem_bytes(), su>>>(u);
     prof_end(h);
     CKL();
@@ -1705,12 +1710,13 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
     prof_begin(h, ALFGPU_PROF_FLUSH);
     const int* s2o = h->pairblock ? h->sites2_out : nullptr;
     const double* co = h->pairblock ? h->coef_out : nullptr;
-    if (dfv)
-      k_flush_xy<ArF><<<dim3((N + 7) / 8, h->B), dim3(32, 8), 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W,
-                                                                         h->X, h->Y, s2o, co);
+    const dim3 gxy((N + 7) / 8, h->B);
+    if (real)
+      k_flush_xy<ArRe><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
+    else if (dfv)
+      k_flush_xy<ArF><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
     else
-      k_flush_xy<ArD><<<dim3((N + 7) / 8, h->B), dim3(32, 8), 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W,
-                                                                         h->X, h->Y, s2o, co);
+      k_flush_xy<ArD><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
     CKL();
     if (ov && blk + 1 < nblk) {  // snapshot for the next block, then let its visits start
       k_sub_gather<<<h->B, 256, 0, h->st>>>(h->G, F * NN, N, F, M, V, dir, h->blk_start[dir][blk + 1],
@@ -1868,6 +1874,8 @@ static int oz_setup(alfgpu_s* h) {
     // with its largest shared-memory carveout while the flush runs
     if (cudaFuncSetAttribute(k_oz_gemm<16, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaFuncSetAttribute(k_update<ArRe>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(k_update<ArF>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(k_update<ArD>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1929,7 +1937,8 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
         cudaFuncSetAttribute(k_bqr_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       return fail(ALFGPU_ERROR_CUDA);
   }
-  if (raise_smem_limit(k_update<ArD>, upd_smem_bytes()) != cudaSuccess ||
+  if (raise_smem_limit(k_update<ArRe>, upd_smem_bytes(8)) != cudaSuccess ||
+      raise_smem_limit(k_update<ArD>, upd_smem_bytes()) != cudaSuccess ||
       raise_smem_limit(k_update<ArF>, upd_smem_bytes()) != cudaSuccess)
     return fail(ALFGPU_ERROR_CUDA);
   // shrink the QR cluster until at least one cluster fits on the device
@@ -2022,7 +2031,7 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   r |= dalloc(h, &h->m, 2 * (C + B)); r |= dalloc(h, &h->sites, C * UPD_KMAX);  // m: one set per block parity
   r |= dalloc(h, &h->Gsnap, B * UPD_KMAX * UPD_KMAX); r |= dalloc(h, &h->Gsub, B * UPD_KMAX * UPD_KMAX);
   r |= dalloc(h, &h->posn, C * UPD_KMAX); r |= dalloc(h, &h->npos, C);
-  r |= dalloc(h, &h->W, C * 2 * UPD_KMAX * UPD_KMAX); r |= dalloc(h, &h->dlt, C * 2 * UPD_KMAX);
+  r |= dalloc(h, &h->W, C * 2 * UPD_KMAX * UPD_KMAX);
   r |= dalloc(h, &h->X, C * 2 * N * UPD_KMAX); r |= dalloc(h, &h->Y, C * 2 * N * UPD_KMAX);
   r |= dalloc(h, &h->phase, C); r |= dalloc(h, &h->cnt, 4 * C); r |= dalloc(h, &h->stat, 8 * C);
   r |= dalloc(h, &h->err, 1);

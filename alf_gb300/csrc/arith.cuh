@@ -2,6 +2,31 @@
 #include "common.cuh"
 #include "dfloat.cuh"
 
+// |x| well inside the normal range (2^-900 .. 2^900), x / 2 and -x, on the integer pipes.
+ALF_DEV bool alf_normal(double x) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ff;
+  return e - 123u < 1800u;
+}
+ALF_DEV double alf_half(double x) { return __hiloint2double(__double2hiint(x) - (1 << 20), __double2loint(x)); }
+ALF_DEV double alf_flip(double x) { return __hiloint2double(__double2hiint(x) ^ (int)0x80000000u, __double2loint(x)); }
+// 1/sqrt(t) and 1/y from the hardware's approximations (about 20 bits) and one cubic step each:
+// with e = 1 - t r^2 (1 - y r) the corrected value r (1 + e/2 + 3/8 e^2) (r (1 + e + e^2)) is off
+// by e^3 < 2^-57 before its rounding.  The arguments are in alf_normal's range.
+ALF_DEV double alf_rsqrt_n(double t) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(t));
+  const double e = fma(-t * r, r, 1.0);
+  return fma(r * e, fma(0.375, e, 0.5), r);
+}
+ALF_DEV double alf_rcp_n(double y) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+  const double e = fma(-y, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+// 1/y: seven dependent FP64 instructions fewer than a division.
+ALF_DEV double alf_rcp(double y) { return alf_normal(y) ? alf_rcp_n(y) : 1.0 / y; }
+
 // Scalar arithmetic shared by the update and QR kernels.  ArD: FP64 complex (the
 // plain form: ratios must agree with an FP64 reference to ~1e-10 even where
 // 1 + Delta (1 - G_jj) cancels).  ArF: double-float on the FP32 pipes (the mixed
@@ -30,16 +55,8 @@ struct ArD {
   static ALF_DEV R absr(R a) { return fabs(a); }
   static ALF_DEV R mulr(R a, R b) { return a * b; }
   static ALF_DEV bool gt(R a, R b) { return a > b; }
-  // 1/d, d > 0 real: float seed, two Newton-Raphson steps r <- r + r (1 - d r) (quadratic
-  // convergence, 2^-24 -> 2^-48 -> below 2^-53); an FP64 division costs ~560 cycles here.
-  static ALF_DEV double rcp_pos(double d) {
-    if (!(d > 1e-30 && d < 1e30)) return 1.0 / d;
-    double r = (double)__frcp_rn(__double2float_rn(d));
-    r = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-  }
   static ALF_DEV Z rcp(Z a) {
-    const double s = rcp_pos(a.x * a.x + a.y * a.y);
+    const double s = alf_rcp(a.x * a.x + a.y * a.y);
     return zmk(a.x * s, -a.y * s);
   }
   // FP64 range holds the unnormalised phase of a block (<= 32 ratio factors); it is
@@ -63,13 +80,7 @@ struct ArD {
   static ALF_DEV R rsub(R a, R b) { return a - b; }
   static ALF_DEV R rneg(R a) { return -a; }
   static ALF_DEV R rsqrt_(R a) { return sqrt(a); }
-  static ALF_DEV R rrcp(R a) {
-    const double m = fabs(a);
-    if (!(m > 1e-30 && m < 1e30)) return 1.0 / a;
-    double r = (double)__frcp_rn(__double2float_rn(a));
-    r = fma(r, fma(-a, r, 1.0), r);
-    return fma(r, fma(-a, r, 1.0), r);
-  }
+  static ALF_DEV R rrcp(R a) { return alf_rcp(a); }
   static ALF_DEV R rmax0(R a) { return a > 0.0 ? a : 0.0; }
   static ALF_DEV bool rzero_p(R a) { return a == 0.0; }
   static ALF_DEV bool rneg_p(R a) { return a < 0.0; }
@@ -164,7 +175,7 @@ struct ArRe {
   static ALF_DEV R im(Z) { return 0.0; }
   static ALF_DEV R mulr(R a, R b) { return a * b; }
   static ALF_DEV bool gt(R a, R b) { return a > b; }
-  static ALF_DEV Z rcp(Z a) { return ArD::rrcp(a); }
+  static ALF_DEV Z rcp(Z a) { return alf_rcp(a); }
   static ALF_DEV Z shfl(Z a, int src) { return __shfl_sync(0xffffffffu, a, src); }
   static ALF_DEV Z shfl_xor(Z a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
   static ALF_DEV Z conj(Z a) { return a; }
@@ -177,7 +188,7 @@ struct ArRe {
   static ALF_DEV R rsub(R a, R b) { return a - b; }
   static ALF_DEV R rneg(R a) { return -a; }
   static ALF_DEV R rsqrt_(R a) { return sqrt(a); }
-  static ALF_DEV R rrcp(R a) { return ArD::rrcp(a); }
+  static ALF_DEV R rrcp(R a) { return alf_rcp(a); }
   static ALF_DEV R rmax0(R a) { return a > 0.0 ? a : 0.0; }
   static ALF_DEV bool rzero_p(R a) { return a == 0.0; }
   static ALF_DEV bool rneg_p(R a) { return a < 0.0; }

@@ -36,28 +36,6 @@ static inline size_t qrc_smem_bytes(int N, int CL, int zb) {
   return nc * qrc_ld(N, zb) * zb + ((size_t)N + 3 * nc + 2) * zb + (3 * nc) * 8 + (3 * nc) * sizeof(int) + 64;
 }
 
-// |x| well inside the normal range (2^-900 .. 2^900), and x / 2, on the integer pipes.
-ALF_DEV bool qrc_normal(double x) {
-  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ff;
-  return e - 123u < 1800u;
-}
-ALF_DEV double qrc_half(double x) { return __hiloint2double(__double2hiint(x) - (1 << 20), __double2loint(x)); }
-// 1/sqrt(t) and 1/y from the hardware's approximations (about 20 bits) and one cubic step each:
-// with e = 1 - t r^2 (1 - y r) the corrected value r (1 + e/2 + 3/8 e^2) (r (1 + e + e^2)) is off
-// by e^3 < 2^-57 before its rounding.  The caller keeps the arguments in the normal range.
-ALF_DEV double qrc_rsqrt(double t) {
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(t));
-  const double e = fma(-t * r, r, 1.0);
-  return fma(r * e, fma(0.375, e, 0.5), r);
-}
-ALF_DEV double qrc_rcp(double y) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
-  const double e = fma(-y, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 template <class Z>
 ALF_DEV Z qrc_peer(const Z* p, unsigned rank) {  // a value in a peer CTA's shared memory
   const uint32_t a = dsmem_addr(p, rank);
@@ -248,10 +226,10 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
       const double ar = A::re(alpha);
       const double t2 = A::abs2add(alpha, xn2);
       double s, ib, iy = 0.0, yy;
-      if (qrc_normal(t2)) {
-        ib = qrc_rsqrt(t2);
+      if (alf_normal(t2)) {
+        ib = alf_rsqrt_n(t2);
         s = t2 * ib;
-        s = fma(fma(-s, s, t2), qrc_half(ib), s);
+        s = fma(fma(-s, s, t2), alf_half(ib), s);
       } else {
         s = sqrt(t2);
         ib = 1.0 / s;
@@ -261,7 +239,7 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
       const Z tau = A::mkz(fma(-ar, ib, 1.0), -A::im(alpha) * ib);  // (beta - alpha) / beta
       const Z y = A::sub(alpha, A::mkz(beta, 0.0));
       yy = A::kReal ? A::re(y) : A::abs2(y);
-      iy = qrc_normal(yy) ? qrc_rcp(yy) : 1.0 / yy;
+      iy = alf_normal(yy) ? alf_rcp_n(yy) : 1.0 / yy;
       const Z scal = A::kReal ? A::mkz(iy, 0.0) : A::scale(A::conj(y), iy);
       for (int t = tid; t < nact; t += QRC_WORK) {
         const int lc = act[t];

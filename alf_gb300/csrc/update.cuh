@@ -63,9 +63,8 @@ struct UpdParams {
   const unsigned long long* rngctr;      // [chain] counter of draw 0 of this sweep
   zd* phase;            // [chain]
   int* m_out;           // [chain], then [chain][F] (per-GEMM-batch rank)
-  zd* W;                // [chain][2][UPD_KMAX][UPD_KMAX]  Delta_S Gamma^-1
+  zd* W;                // [chain][2][UPD_KMAX][UPD_KMAX]  C, x and P of the accepted positions
   int* sites_out;       // [chain][UPD_KMAX]  accepted sites, accept order
-  zd* delta_out;        // [chain][2][UPD_KMAX] Delta of accepted sites
   long long* cnt;       // [chain][4] n_prop, n_acc, n_prop_eff, n_acc_eff
   int8_t* rec_acc; zd* rec_ratio; long long sRec;
   FieldTables ft;
@@ -168,44 +167,48 @@ struct UpdTab {
 
 // One CTA of UPD_THREADS threads per chain.  Dynamic shared memory:
 //   Gh[F][KMAX][KMAX+1]  the block Ghat over the block's positions, updated in place
-//   G0[F][KMAX][KMAX+1]  Ghat at block entry; reused as the ping-pong buffer of the
-//                        Gauss-Jordan inversion of Gamma.
+//   Tc[F][KMAX][KMAX]    x_q Ghat(:, q) of every position q at its step (0 on the rows up to q)
 // A position is one non-zero eigenvalue of a vertex (its site in the diagonal basis);
 // single-site vertices have one, two-site vertices two consecutive positions whose
 // joint ratio is Upgrade2's 2x2 determinant, computed as D_a (1 + Delta_b (1 - G'_bb))
 // with G' after the tentative Sherman-Morrison update of position a; an accepted
 // two-site vertex is applied as two rank-1 updates, the second decided with the first.
-// Warp 0 runs the sequential Metropolis chain (all lanes compute the same scalars;
-// lane a handles row a of a column).  While warps 1..7 apply the rank-1 update of an
-// accepted position q to rows a > q and the columns beyond those warp 0 needs next,
-// warp 0 updates the next one or two columns itself and already decides the next
-// position from them: one block barrier per position.  At block end, W = Delta_S Gamma^-1
-// is formed by Gauss-Jordan elimination without pivoting: the pivots in accept order
-// are the accepted positions' own 1 + Delta (1 - G_jj) factors (the Sherman-Morrison
-// sequence is the LU factorisation of Gamma in that order), non-zero because a zero
-// factor gives weight 0 and is rejected.
+//
+// One block barrier per position v.  Between two barriers, with the previous position's decision
+// and Tc column known, four parts run on different sub-partitions (an FP64 instruction holds its
+// sub-partition ~64 cycles, so the chain per position is counted in them):
+//   warp 0       the ratio and its test, from the diagonal element (scalars only)
+//   warp 1 + f   flavour f's column v, 1 / D and Tc(v), whether or not v is accepted
+//   the others   the previous position's rank-1 update of the columns beyond v
+// Column v is not written back: nothing reads it after its own step (the column that follows the
+// first position of a pair is left out of that step's update and takes two at its own step).
+// The flush needs no inverse of Gamma: the accepted updates are G0 - sum_l x_l u_l w_l^T with
+//   w_l = b_l + sum_{k<l} C_lk w_k,  C_lk = x_k u_k(s_l),      b_l = e_{s_l} - G0(s_l, :)
+//   u_l = G0(:, s_l) + sum_{k<l} u_k P_kl,  P_kl = x_k G^{(k-1)}(s_k, s_l),
+// so G0 - X Y with X = G0(:, S), Y = (1 - P)^-1 diag(x) (1 - C)^-1 b: two triangular
+// substitutions per column in k_flush_xy.  C, P and x are entries of Tc and Ghat.
+// Measured, 32 positions, two flavours: FP64 complex 105 us, double-float 79 us (one warp for the
+// chain, Gauss-Jordan at the end) -> 28 us real, 65 us complex, 59 us double-float (with about 8 us of
+// timing events).
 template <class A>
 __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
   typedef typename A::Z Z;
-  typedef typename A::R R;
   constexpr int KM = UPD_KMAX, LD = UPD_KMAX + 1, NW = UPD_THREADS / 32;
   const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = p.N, F = p.F, M = p.M, nq = p.nq;
   extern __shared__ __align__(16) unsigned char upd_raw[];
-  Z* Gh = reinterpret_cast<Z*>(upd_raw);
-  Z* G0 = Gh + 2 * KM * LD;
+  Z* Gh = reinterpret_cast<Z*>(upd_raw);  // [F][KM][LD]
+  Z* Tc = Gh + 2 * KM * LD;               // [F][KM][KM]
   // per position
-  __shared__ Z s_mye[2][KM], s_dlt[2][KM], s_tcol[2][2][KM], s_rowt[2][KM], s_piv[2][2];
-  __shared__ zd s_dlt64[2][KM];
-  __shared__ int s_psite[KM], s_pvis[KM], s_pkind[KM], s_accq[KM], s_acc[2];
+  __shared__ Z s_mye[2][KM], s_dlt[2][KM], s_rD[2][KM];
+  __shared__ Z s_myk[2][A::kReal ? KM : 1], s_dlk[2][A::kReal ? KM : 1];  // real: K folded in
+  __shared__ int s_psite[KM], s_pvis[KM], s_pkind[KM], s_acc[KM], s_accq[NW][KM];
   __shared__ int s_psite2[KM];      // vector positions: site b, else -1
   __shared__ double s_pc[KM][2];    // vector positions: (c_a, c_b)
   // per visit (FP64 in both forms: the ratio accumulation)
   __shared__ zd s_K[KM];
   __shared__ double s_u2[KM], s_gr[KM];
   __shared__ int s_vtx[KM], s_snew[KM], s_prop[KM];
-  __shared__ short s_ij[KM * KM];
-  __shared__ int s_m, s_np;
 
   const double2* G = reinterpret_cast<const double2*>(p.G) + (long long)c * p.sG;
   const int* site = p.V.site + (long long)c * p.V.sK;
@@ -216,339 +219,328 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
   int8_t* fl = p.fields + (long long)c * p.L * M + (long long)(p.nt1 - 1) * M;
   const long long NN = (long long)N * N;
 
-  // Prologue (warp 0, lane q = visit): each vertex is visited once per block, so its old
-  // field is the field at block start and every visit's proposal, draws and transition
-  // factors are known; positions by an exclusive prefix sum of the vertex sizes.
-  if (warp == 0) {
-    const int q = lane;
-    int w = 0, n = 0;
-    if (q < nq) {
-      const int pos = p.q0 + q;
-      n = p.dir == 0 ? pos : M - 1 - pos;
-      w = nsite[n];
-    }
-    int incl = w;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const int p0 = incl - w;
-    if (lane == 31) s_np = incl;
-    if (q < nq) {
-      s_vtx[q] = n;
-      const int v = p.visit_base + p.q0 + q;
-      double u0, u1, uu2;
-      if (p.draws) {
-        const double* d = p.draws + (long long)c * p.sDraws + 3ll * v;
-        u0 = d[0]; u1 = d[1]; uu2 = d[2];
-      } else {
-        unsigned long long key = p.rngkey[c], ctr = p.rngctr[c] + 3ull * v;
-        u0 = alf_uniform(key, ctr); u1 = alf_uniform(key, ctr + 1); uu2 = alf_uniform(key, ctr + 2);
+  // Positions (every warp, lane q = visit): an exclusive prefix sum of the vertex sizes.
+  const int q = lane;
+  int w = 0, n = 0;
+  if (q < nq) {
+    const int pos = p.q0 + q;
+    n = p.dir == 0 ? pos : M - 1 - pos;
+    w = nsite[n];
+  }
+  int incl = w;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const int p0 = incl - w, np = __shfl_sync(0xffffffffu, incl, 31);
+  if (warp == 1 && q < nq) {
+    const int vb = p.vsite2 ? p.vsite2[(long long)c * p.V.sK + n] : -1;
+    for (int I = 0; I < w; ++I) {
+      s_psite[p0 + I] = I ? site2[n] : site[n];
+      s_pvis[p0 + I] = q;
+      s_pkind[p0 + I] = (w == 2) ? (I ? 2 : 1) : 0;  // 0 single, 1 first of a pair, 2 second
+      s_psite2[p0 + I] = (w == 1) ? vb : -1;
+      if (vb >= 0) {
+        s_pc[p0 + I][0] = p.vcoef[2 * ((long long)c * p.V.sK + n)];
+        s_pc[p0 + I][1] = p.vcoef[2 * ((long long)c * p.V.sK + n) + 1];
       }
-      const int so = fl[n], tp = ty[n];
-      const int ch = (tp == 1) ? 0 : nranf3(u0) - 1;
-      const int sn = (tp == 1) ? -so : (int)p.ft.flip[so + 2][ch];
-      s_snew[q] = sn;
-      s_prop[q] = 1.5 > u1;  // T0_proposal (Wrapgr_mod.F90:123,133); always true
-      s_u2[q] = uu2;
-      s_gr[q] = p.ft.grat[tp - 1][so + 2][sn + 2];
-      zd K = zmk(1.0, 0.0);
-      for (int f = 0; f < F; ++f) {
-        const UpdTab e = tab[((long long)(f * M + n) * 5 + so + 2) * 3 + ch];
-        for (int I = 0; I < w; ++I) {
-          s_mye[f][p0 + I] = A::mk(e.myexp[I]);
-          s_dlt[f][p0 + I] = A::mk(e.dlt[I]);
-          s_dlt64[f][p0 + I] = e.dlt[I];
-        }
-        K = (f == 0) ? e.expal : zmul(K, e.expal);
-      }
-      // [prod_f exp(Z1 alpha)]^N_SUN gamma'/gamma: with N_SUN = 1 the gamma ratio joins K
-      if (p.NSUN == 1) K = zscale(K, p.ft.grat[tp - 1][so + 2][sn + 2]);
-      s_K[q] = K;
-      const int vb = p.vsite2 ? p.vsite2[(long long)c * p.V.sK + n] : -1;
+    }
+  }
+  if (warp == 0 && q < nq) {
+    // each vertex is visited once per block, so its old field is the field at block start and
+    // every visit's proposal, draws and transition factors are known
+    s_vtx[q] = n;
+    const int v = p.visit_base + p.q0 + q;
+    const int so = fl[n], tp = ty[n];
+    double u0, u1, uu2;
+    if (p.draws) {
+      const double* d = p.draws + (long long)c * p.sDraws + 3ll * v;
+      u0 = d[0]; u1 = d[1]; uu2 = d[2];
+    } else {
+      unsigned long long key = p.rngkey[c], ctr = p.rngctr[c] + 3ull * v;
+      u0 = alf_uniform(key, ctr); u1 = alf_uniform(key, ctr + 1); uu2 = alf_uniform(key, ctr + 2);
+    }
+    const int ch = (tp == 1) ? 0 : nranf3(u0) - 1;
+    const int sn = (tp == 1) ? -so : (int)p.ft.flip[so + 2][ch];
+    const UpdTab* e = tab + ((long long)n * 5 + so + 2) * 3 + ch;
+    s_snew[q] = sn;
+    s_prop[q] = 1.5 > u1;  // T0_proposal (Wrapgr_mod.F90:123,133); always true
+    s_u2[q] = uu2;
+    const double gr = p.ft.grat[tp - 1][so + 2][sn + 2];
+    s_gr[q] = gr;
+    zd K = e->expal;
+    if (F == 2) K = zmul(K, e[(long long)M * 15].expal);
+    // [prod_f exp(Z1 alpha)]^N_SUN gamma'/gamma: with N_SUN = 1 the gamma ratio joins K
+    if (p.NSUN == 1) K = zscale(K, gr);
+    s_K[q] = K;
+    for (int f = 0; f < F; ++f)
       for (int I = 0; I < w; ++I) {
-        s_psite[p0 + I] = I ? site2[n] : site[n];
-        s_pvis[p0 + I] = q;
-        s_pkind[p0 + I] = (w == 2) ? (I ? 2 : 1) : 0;  // 0 single, 1 first of a pair, 2 second
-        s_psite2[p0 + I] = (w == 1) ? vb : -1;
-        if (vb >= 0) {
-          s_pc[p0 + I][0] = p.vcoef[2 * ((long long)c * p.V.sK + n)];
-          s_pc[p0 + I][1] = p.vcoef[2 * ((long long)c * p.V.sK + n) + 1];
+        const Z me = A::mk(e[(long long)f * M * 15].myexp[I]), dl = A::mk(e[(long long)f * M * 15].dlt[I]);
+        s_mye[f][p0 + I] = me;
+        s_dlt[f][p0 + I] = dl;
+        // real: K joins the first flavour's factor of a single position (the last factor of a pair)
+        if (A::kReal && I == w - 1) {
+          s_myk[f][p0 + I] = f == 0 ? A::mul(me, A::mk(K)) : me;
+          s_dlk[f][p0 + I] = f == 0 ? A::mul(dl, A::mk(K)) : dl;
         }
       }
-    }
   }
-  __syncthreads();
-  const int np = s_np;
-  for (int a = warp; a < np; a += NW)
-    if (lane < np)
-      for (int f = 0; f < F; ++f) {
-        zd g = p.Gsub ? p.Gsub[(((long long)c * F + f) * KM + a) * KM + lane]
-                      : G[f * NN + s_psite[a] + (long long)s_psite[lane] * N];
-        if (p.vsite2 && (s_psite2[a] >= 0 || s_psite2[lane] >= 0)) {
-          // Ghat(a, l) = v_a^T G v_l over the (up to two) sites of each position
-          const int ia[2] = {s_psite[a], s_psite2[a]}, il[2] = {s_psite[lane], s_psite2[lane]};
-          const double ca[2] = {s_psite2[a] >= 0 ? s_pc[a][0] : 1.0, s_psite2[a] >= 0 ? s_pc[a][1] : 0.0};
-          const double cl[2] = {s_psite2[lane] >= 0 ? s_pc[lane][0] : 1.0, s_psite2[lane] >= 0 ? s_pc[lane][1] : 0.0};
-          g = zmk(0.0, 0.0);
-          for (int x = 0; x < 2; ++x)
-            for (int y = 0; y < 2; ++y)
-              if (ia[x] >= 0 && il[y] >= 0 && ca[x] != 0.0 && cl[y] != 0.0)
-                g = zadd(g, zscale(G[f * NN + ia[x] + (long long)il[y] * N], ca[x] * cl[y]));
-        }
-        const Z v = A::mk(g);
-        Gh[(f * KM + a) * LD + lane] = v;
-        G0[(f * KM + a) * LD + lane] = v;
-      }
-  __syncthreads();
-
-  // warp-0 state (identical in all lanes)
-  zd ph = p.phase[c];  // FP64, kept unnormalised within a block (only its direction enters the weight)
-  int m = 0, nacc = 0, pend = 0;
-  long long n_prop = 0;
-  auto accept_pos = [&](int v) {
-    if (lane == 0) {
-      s_accq[m] = v;
-      p.sites_out[(long long)c * KM + m] = s_psite[v];
-      if (p.sites2_out) {
-        p.sites2_out[(long long)c * KM + m] = s_psite2[v];
-        if (s_psite2[v] >= 0) {
-          p.coef_out[2 * ((long long)c * KM + m)] = s_pc[v][0];
-          p.coef_out[2 * ((long long)c * KM + m) + 1] = s_pc[v][1];
-        }
-      }
-      for (int f = 0; f < F; ++f) p.delta_out[((long long)c * 2 + f) * KM + m] = s_dlt64[f][v];
-    }
-    m += 1;
-  };
-  // Decide position v from the current column v (gc, diagonal gd) and, for the first
-  // position of a pair, column v+1 (gc2).  Second positions follow their pair's decision.
-  auto decide = [&](int v, const Z* gd, const Z* gc, const Z* gc2) {
-    const int kind = s_pkind[v];
-    int acc = 0;
-    const int fo = (F == 2) ? (lane & 1) : 0;  // flavour of this lane's scalar work
-    if (kind == 2) {  // second position of an accepted / rejected pair
-      acc = pend;
-      if (acc) {
-        const Z D = A::sub(s_mye[fo][v], A::mul(s_dlt[fo][v], fo ? gd[1] : gd[0]));
-        const Z xm = A::mul(s_dlt[fo][v], A::rcp(D));
-        const Z x[2] = {A::shfl(xm, 0), A::shfl(xm, 1)};
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-          if (f < F && lane > v && lane < np) s_tcol[v & 1][f][lane] = A::mul(x[f], gc[f]);
-        accept_pos(v);
-      }
-      if (lane == 0) s_acc[v & 1] = acc;
-      return;
-    }
-    const int q = s_pvis[v];
-    zd Rt = zmk(0.0, 0.0);
-    if (s_prop[q]) {
-      // lane parity carries flavour fo: Mat(1,1) = myexp - Delta G(P,P), and for the first
-      // position of a pair the 2x2 determinant D_a (myexp_b - Delta_b G'_bb)
-      const Z D = A::sub(s_mye[fo][v], A::mul(s_dlt[fo][v], fo ? gd[1] : gd[0]));
-      Z Rm = D, xm = A::zero();
-      if (kind == 1) {
-        xm = A::mul(s_dlt[fo][v], A::rcp(D));
-        const int w = v + 1;
-        const Z c2 = fo ? gc2[1] : gc2[0], c1 = fo ? gc[1] : gc[0];
-        const Z gww = A::shfl(c2, w), gvw = A::shfl(c2, v), gwv = A::shfl(c1, w);
-        const Z gp = A::mac(gww, A::mul(xm, gwv), gvw);
-        Rm = A::mul(D, A::sub(s_mye[fo][w], A::mul(s_dlt[fo][w], gp)));
-      }
-      // the ratio is accumulated in FP64: flavour product, exp(Z1 alpha), N_SUN power
-      const zd Rm64 = A::wide(Rm);
-      Rt = (F == 2) ? zmul(ArD::shfl(Rm64, 0), ArD::shfl(Rm64, 1)) : Rm64;
-      if (p.NSUN == 1) {
-        Rt = zmul(Rt, s_K[q]);  // K carries the gamma ratio (prologue)
-      } else {
-        Rt = zmul(Rt, s_K[q]);
-        zd Rp = Rt;
-        for (int e = 1; e < p.NSUN; ++e) Rp = zmul(Rp, Rt);
-        Rt = zscale(Rp, s_gr[q]);
-      }
-      // weight = |Re(phase R) / Re(phase)| > u  (Wrapgr_mod.F90:141-143), division-free, FP64
-      const double num = fabs(ph.x * Rt.x - ph.y * Rt.y);
-      const double den = fabs(ph.x) * s_u2[q];
-      acc = num > den;
-      if (acc) {
-        ph = zmul(ph, Rt);
-        if (kind != 1) xm = A::mul(s_dlt[fo][v], A::rcp(D));  // Delta / Mat(1,1)
-        const Z x[2] = {A::shfl(xm, 0), A::shfl(xm, 1)};
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-          if (f < F && lane > v && lane < np) s_tcol[v & 1][f][lane] = A::mul(F == 2 ? x[f] : xm, gc[f]);
-      }
-    }
-    n_prop += s_prop[q];
-    if (lane == 0) {
-      if (p.rec_acc) {
-        const long long r = (long long)c * p.sRec + p.visit_base + p.q0 + q;
-        p.rec_acc[r] = (int8_t)acc;
-        p.rec_ratio[r] = Rt;
-      }
-      if (acc) fl[s_vtx[q]] = (int8_t)s_snew[q];
-      s_acc[v & 1] = acc;
-    }
-    if (acc) { accept_pos(v); nacc += 1; }
-    pend = acc;
-  };
-
-  if (warp == 0) {
-    Z gd[2], gc[2], gc2[2];
-#pragma unroll
-    for (int f = 0; f < 2; ++f)
-      if (f < F) {
-        gc[f] = (lane < np) ? Gh[(f * KM + lane) * LD] : A::zero();
-        gc2[f] = (lane < np && np > 1) ? Gh[(f * KM + lane) * LD + 1] : A::zero();
-        gd[f] = Gh[f * KM * LD];
-      }
-    decide(0, gd, gc, gc2);
-  }
-  __syncthreads();
-  for (int q = 0; q < np; ++q) {
-    const int acc = s_acc[q & 1];
-    const int v = q + 1;
-    // columns warp 0 brings up to date for its next decision: v, and v+1 if v opens a pair
-    const int wc = (v < np && s_pkind[v] == 1) ? 2 : 1;
-    if (warp == 0) {
-      if (v < np) {
-        Z gd[2], gc[2], gc2[2];
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-          if (f < F) {
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              if (t >= wc) continue;
-              const int col_i = v + t;
-              Z col = (lane < np) ? Gh[(f * KM + lane) * LD + col_i] : A::zero();
-              if (acc && lane > q && lane < np) {  // column col_i of the rank-1 update of position q
-                col = A::mac(col, s_tcol[q & 1][f][lane], Gh[(f * KM + q) * LD + col_i]);
-                Gh[(f * KM + lane) * LD + col_i] = col;
-              }
-              if (t == 0) gc[f] = col; else gc2[f] = col;
+  if (warp != 0) {
+    asm volatile("bar.sync 1, 224;" ::: "memory");  // positions (warps 1..7); warp 0 joins below
+    if (p.Gsub) {
+      for (int a = warp - 1; a < np; a += NW - 1)
+        if (lane < np)
+          for (int f = 0; f < F; ++f)
+            Gh[(f * KM + a) * LD + lane] = A::mk(p.Gsub[(((long long)c * F + f) * KM + a) * KM + lane]);
+    } else {
+      for (int l = warp - 1; l < np; l += NW - 1)  // lane = row: consecutive sites are contiguous in G
+        if (lane < np)
+          for (int f = 0; f < F; ++f) {
+            zd g;
+            if (p.vsite2 && (s_psite2[lane] >= 0 || s_psite2[l] >= 0)) {
+              // Ghat(a, l) = v_a^T G v_l over the (up to two) sites of each position
+              const int ia[2] = {s_psite[lane], s_psite2[lane]}, il[2] = {s_psite[l], s_psite2[l]};
+              const double ca[2] = {s_psite2[lane] >= 0 ? s_pc[lane][0] : 1.0, s_psite2[lane] >= 0 ? s_pc[lane][1] : 0.0};
+              const double cl[2] = {s_psite2[l] >= 0 ? s_pc[l][0] : 1.0, s_psite2[l] >= 0 ? s_pc[l][1] : 0.0};
+              g = zmk(0.0, 0.0);
+              for (int x = 0; x < 2; ++x)
+                for (int y = 0; y < 2; ++y)
+                  if (ia[x] >= 0 && il[y] >= 0 && ca[x] != 0.0 && cl[y] != 0.0)
+                    g = zadd(g, zscale(G[f * NN + ia[x] + (long long)il[y] * N], ca[x] * cl[y]));
+            } else {
+              g = G[f * NN + s_psite[lane] + (long long)s_psite[l] * N];
             }
-            gd[f] = A::shfl(gc[f], v);
-          }
-        decide(v, gd, gc, gc2);
-      }
-    } else if (acc && warp != 4) {
-      // Ghat(a,b) += x Ghat(a,q) Ghat(q,b), rows a > q, columns b > q + wc.  Warp 4 shares
-      // warp 0's SM sub-partition (FP64 unit) and stays idle so the chain is not delayed.
-      const int wk = warp < 4 ? warp : warp - 1;  // 1..6
-      const int b = lane;
-      if (b > q + wc && b < np)
-        for (int f = 0; f < F; ++f)
-          for (int a = q + wk; a < np; a += NW - 2) {
-            Z* g = Gh + (f * KM + a) * LD + b;
-            *g = A::mac(*g, s_tcol[q & 1][f][a], Gh[(f * KM + q) * LD + b]);
+            Gh[(f * KM + lane) * LD + l] = A::mk(g);
           }
     }
-    __syncthreads();
   }
-  if (tid == 0) s_m = m;
   __syncthreads();
-  m = s_m;
-  if (m > 0) {
-    const int FMM = F * m * m;
-    for (int e = tid; e < m * m; e += UPD_THREADS) s_ij[e] = (short)(((e / m) << 6) | (e % m));
-    // Gamma(l,l') = delta_ll' + (delta_ll' - G0(s_l, s_l')) Delta_l'  in Gh (accept order)
-    for (int l = warp; l < m; l += NW)
-      if (lane < m)
-        for (int f = 0; f < F; ++f) {
-          const int l2 = lane;
-          const Z g = G0[(f * KM + s_accq[l]) * LD + s_accq[l2]];
-          Z v = A::mul(A::sub(l == l2 ? A::one() : A::zero(), g), s_dlt[f][s_accq[l2]]);
-          if (l == l2) v = A::add(v, A::one());
-          Gh[(f * KM + l) * LD + l2] = v;
+
+  // scalar state of warp 0 (identical in all lanes)
+  zd ph = p.phase[c];  // FP64, kept unnormalised within a block (only its direction enters the weight)
+  long long n_prop = 0;
+  int nacc = 0;
+  const int fo = (F == 2) ? (lane & 1) : 0;  // flavour of this lane's scalar work
+  for (int v = 0; v < np; ++v) {
+    const int kind = s_pkind[v];
+    const int q = v - 1, qs = v > 0 ? q : 0;
+    const int acc = v > 0 ? s_acc[q] : 0;
+    if (warp == 0) {
+      int a = 0;
+      if (kind == 2) {  // second position: decided with the first
+        a = acc;
+        if (lane == 0) s_acc[v] = a;
+      } else {
+        const int vi = s_pvis[v], prop = s_prop[vi];
+        zd Rt = zmk(0.0, 0.0);
+        // Mat(1,1) = myexp - Delta G(P,P), and for the first position of a pair the 2x2
+        // determinant D_a (myexp_b - Delta_b G'_bb); the real form has K in its last factor
+        Z Rm;
+        if (kind == 0) {
+          const Z me = A::kReal ? s_myk[fo][v] : s_mye[fo][v], dl = A::kReal ? s_dlk[fo][v] : s_dlt[fo][v];
+          Z g = Gh[(fo * KM + v) * LD + v];
+          const Z tq = Tc[(fo * KM + qs) * KM + v], row = Gh[(fo * KM + qs) * LD + v];
+          if (acc) g = A::mac(g, tq, row);
+          Rm = A::mac(me, A::neg(dl), g);
+        } else {
+          const int w = v + 1, ra = v + ((lane >> 1) & 1), rb = v + ((lane >> 2) & 1);
+          const Z me = A::kReal ? s_myk[fo][w] : s_mye[fo][w], dl = A::kReal ? s_dlk[fo][w] : s_dlt[fo][w];
+          Z g = Gh[(fo * KM + ra) * LD + rb];
+          if (acc) g = A::mac(g, Tc[(fo * KM + q) * KM + ra], Gh[(fo * KM + q) * LD + rb]);
+          const Z gvv = A::shfl(g, fo), gwv = A::shfl(g, fo + 2), gvw = A::shfl(g, fo + 4), gww = A::shfl(g, fo + 6);
+          const Z D = A::mac(s_mye[fo][v], A::neg(s_dlt[fo][v]), gvv);
+          const Z xm = A::mul(s_dlt[fo][v], A::rcp(D));
+          const Z gp = A::mac(gww, A::mul(xm, gwv), gvw);
+          Rm = A::mul(D, A::mac(me, A::neg(dl), gp));
         }
-    __syncthreads();
-    if (tid < F) s_piv[0][tid] = A::rcp(Gh[(tid * KM) * LD]);
-    // in-place Gauss-Jordan inversion, ping-pong between Gh and G0
-    Z* Ga = Gh;
-    Z* Gb = G0;
-    for (int k = 0; k < m; ++k) {
-      __syncthreads();
-      if (warp < F && lane < m) s_rowt[warp][lane] = A::mul(Ga[(warp * KM + lane) * LD + k], s_piv[k & 1][warp]);
-      __syncthreads();
-      for (int e = tid; e < FMM; e += UPD_THREADS) {
-        const int f = e >= m * m, r = e - f * m * m;
-        const int i = s_ij[r] >> 6, j = s_ij[r] & 63;
-        const Z pinv = s_piv[k & 1][f];
-        Z v;
-        if (i == k && j == k) v = pinv;
-        else if (i == k) v = A::mul(Ga[(f * KM + k) * LD + j], pinv);
-        else if (j == k) v = A::neg(s_rowt[f][i]);
-        else v = A::mac(Ga[(f * KM + i) * LD + j], A::neg(s_rowt[f][i]), Ga[(f * KM + k) * LD + j]);
-        Gb[(f * KM + i) * LD + j] = v;
-        if (i == k + 1 && j == k + 1) s_piv[(k + 1) & 1][f] = A::rcp(v);
+        if (prop) {
+          // the ratio is accumulated in FP64: flavour product, exp(Z1 alpha), N_SUN power
+          if (A::kReal) {
+            // the weight |Re(phase R) / Re(phase)| (Wrapgr_mod.F90:141-143) of a real ratio is |R|;
+            // non-negative numbers compare like their bits
+            double r = A::wide(Rm).x;
+            if (F == 2) r *= __shfl_xor_sync(0xffffffffu, r, 1);
+            if (p.NSUN != 1) {
+              double rp = r;
+              for (int e = 1; e < p.NSUN; ++e) rp *= r;
+              r = rp * s_gr[vi];
+            }
+            Rt.x = r;
+            const long long rb = __double_as_longlong(r) & 0x7fffffffffffffffll;
+            a = rb <= 0x7ff0000000000000ll && rb > __double_as_longlong(s_u2[vi]);
+            if (a && __double_as_longlong(r) < 0) ph = zmk(alf_flip(ph.x), alf_flip(ph.y));
+          } else {
+            const zd Rm64 = A::wide(Rm);
+            Rt = (F == 2) ? zmul(ArD::shfl(Rm64, 0), ArD::shfl(Rm64, 1)) : Rm64;
+            Rt = zmul(Rt, s_K[vi]);
+            if (p.NSUN != 1) {
+              zd Rp = Rt;
+              for (int e = 1; e < p.NSUN; ++e) Rp = zmul(Rp, Rt);
+              Rt = zscale(Rp, s_gr[vi]);
+            }
+            // division-free
+            const double num = fabs(ph.x * Rt.x - ph.y * Rt.y);
+            const double den = fabs(ph.x) * s_u2[vi];
+            a = num > den;
+            if (a) ph = zmul(ph, Rt);
+          }
+        }
+        n_prop += prop;
+        nacc += a;
+        if (lane == 0) {
+          s_acc[v] = a;
+          if (p.rec_acc) {
+            const long long r = (long long)c * p.sRec + p.visit_base + p.q0 + vi;
+            p.rec_acc[r] = (int8_t)a;
+            p.rec_ratio[r] = Rt;
+          }
+        }
       }
-      Z* t = Ga; Ga = Gb; Gb = t;
+    } else if (warp <= F) {
+      const int f = warp - 1;
+      Z* Gf = Gh + f * KM * LD;
+      Z* Tf = Tc + f * KM * KM;
+      const Z dl = s_dlt[f][v], me = s_mye[f][v], tq = Tf[qs * KM + lane];
+      Z col = (lane < np) ? Gf[lane * LD + v] : A::zero();
+      Z row = Gf[qs * LD + v];
+      if (kind == 2) {  // the update before the pair's first position was left out of this column
+        if (v > 1 && s_acc[v - 2] && lane > v - 2 && lane < np)
+          col = A::mac(col, Tf[(v - 2) * KM + lane], Gf[(v - 2) * LD + v]);
+        row = A::shfl(col, q);
+        if (lane == q) Gf[q * LD + v] = col;
+      }
+      if (acc) col = A::mac(col, tq, row);  // Tc is zero on the rows up to its position
+      const Z D = A::mac(me, A::neg(dl), A::shfl(col, v));
+      const Z dc = A::mul(dl, col);
+      const Z r = A::rcp(D);
+      Tf[v * KM + lane] = (lane > v && lane < np) ? A::mul(dc, r) : A::zero();
+      if (lane == 0) s_rD[f][v] = r;
+    } else if (acc) {
+      // Ghat(a,b) += x Ghat(a,q) Ghat(q,b), rows a > q, columns b > v (b > v + 1 if v opens a pair)
+      const int b = lane;
+      if (b > v + (kind == 1) && b < np)
+        for (int f = 0; f < F; ++f) {
+          const Z row = Gh[(f * KM + q) * LD + b];
+          const Z* Tq = Tc + (f * KM + q) * KM;
+          Z* g = Gh + f * KM * LD + b;
+          const int ws = F + 1, st = NW - ws;  // first of these warps, and how many
+          int a = v + (warp - ws);
+          for (; a + st < np; a += 2 * st) {
+            const Z g0 = g[a * LD], g1 = g[(a + st) * LD], t0 = Tq[a], t1 = Tq[a + st];
+            g[a * LD] = A::mac(g0, t0, row);
+            g[(a + st) * LD] = A::mac(g1, t1, row);
+          }
+          if (a < np) g[a * LD] = A::mac(g[a * LD], Tq[a], row);
+        }
     }
     __syncthreads();
-    // W(l, l') = Delta_l Gamma^-1(l, l')
-    for (int l = warp; l < m; l += NW)
-      if (lane < m)
-        for (int f = 0; f < F; ++f)
-          p.W[(((long long)c * 2 + f) * KM + l) * KM + lane] =
-              zmul(s_dlt64[f][s_accq[l]], A::wide(Ga[(f * KM + l) * LD + lane]));
   }
-  if (tid == 0) {
+  // accepted positions in order (every warp for itself)
+  const int myacc = lane < np ? s_acc[lane] : 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, myacc);
+  const int m = __popc(mask), my = __popc(mask & ((1u << lane) - 1u));
+  if (warp == 0 && lane == 0) {
     p.m_out[c] = m;
     for (int f = 0; f < F; ++f) p.m_out[p.nChains + c * F + f] = m;
-    if (m > 0) p.phase[c] = ArD::unit(ph);
-    long long* cn = p.cnt + 4ll * c;
-    cn[0] += n_prop; cn[1] += nacc; cn[2] += nq; cn[3] += nacc;
+    if (m > 0) p.phase[c] = A::kReal ? ph : ArD::unit(ph);
+    unsigned long long* cn = reinterpret_cast<unsigned long long*>(p.cnt) + 4ll * c;
+    atomicAdd(cn, (unsigned long long)n_prop);
+    atomicAdd(cn + 1, (unsigned long long)nacc);
+    atomicAdd(cn + 2, (unsigned long long)nq);
+    atomicAdd(cn + 3, (unsigned long long)nacc);
+  }
+  if (warp == NW - 1 && myacc) {
+    p.sites_out[(long long)c * KM + my] = s_psite[lane];
+    if (p.sites2_out) {
+      p.sites2_out[(long long)c * KM + my] = s_psite2[lane];
+      if (s_psite2[lane] >= 0) {
+        p.coef_out[2 * ((long long)c * KM + my)] = s_pc[lane][0];
+        p.coef_out[2 * ((long long)c * KM + my) + 1] = s_pc[lane][1];
+      }
+    }
+    if (s_pkind[lane] != 2) fl[s_vtx[s_pvis[lane]]] = (int8_t)s_snew[s_pvis[lane]];
+  }
+  // W(l, k): C_lk below the diagonal, x_l on it, P_lk above
+  if (myacc) s_accq[warp][my] = lane;
+  __syncwarp();
+  const int qk = s_accq[warp][lane];  // the lane-th accepted position (lane < m)
+  for (int l = warp; l < m; l += NW) {
+    const int ql = __shfl_sync(0xffffffffu, qk, l);
+    if (lane < m)
+      for (int f = 0; f < F; ++f) {
+        const Z x = A::mul(s_dlt[f][ql], s_rD[f][ql]);
+        const Z w = lane < l ? Tc[(f * KM + qk) * KM + ql] : (lane == l ? x : A::mul(x, Gh[(f * KM + ql) * LD + qk]));
+        p.W[(((long long)c * 2 + f) * KM + l) * KM + lane] = A::wide(w);
+      }
   }
 }
 
-constexpr size_t upd_smem_bytes() { return 2ull * 2 * UPD_KMAX * (UPD_KMAX + 1) * 16; }  // Z is 16 bytes
+// zb: bytes of one element in the kernel's arithmetic (16 complex or double-float, 8 real)
+constexpr size_t upd_smem_bytes(size_t zb = 16) { return 2ull * UPD_KMAX * (2 * UPD_KMAX + 1) * zb; }
 
-// Flush operands for G = G0 - X Y (one launch, spread over the GPU; the m x m x N product of
-// Y in the precision form's arithmetic, double-float in the mixed form):
+// Flush operands for G = G0 - X Y (one launch, spread over the GPU, in the precision form's
+// arithmetic, double-float in the mixed form on complex models):
 //   X(:, l) = G0 v_l
-//   Y(l, :) = sum_l' W(l,l') (v_l'^T - v_l'^T G0)
-// with v_l = e_{s_l}, or c_a e_a + c_b e_b for a vector position (sites2 / coefs, may be null).
-// block 32 x 8 threads = (l, column / row); grid (ceil(N/8), chains*flavours).
+//   Y = (1 - P)^-1 diag(x) (1 - C)^-1 b,  b(l, :) = v_l^T - v_l^T G0
+// with v_l = e_{s_l}, or c_a e_a + c_b e_b for a vector position (sites2 / coefs, may be null), and
+// C, x, P as k_update leaves them in W.  One warp per column of Y (two columns when m <= 16),
+// lane = l: two substitutions, one shuffle and one multiply-add per accepted position each.
+// grid (ceil(N/8), chains*flavours), 256 threads.
 // X: [chain][2][N][KMAX] col-major (ld N); Y: [chain][2][KMAX][N] col-major (ld KMAX).
 template <class A>
-__global__ void k_flush_xy(const zd* Gv, long long sG, int N, int F, const int* m_in, const int* sites, const zd* W,
-                           zd* X, zd* Y, const int* sites2 = nullptr, const double* coefs = nullptr) {
+__global__ void __launch_bounds__(256) k_flush_xy(const zd* Gv, long long sG, int N, int F, const int* m_in,
+                                                  const int* sites, const zd* W, zd* X, zd* Y,
+                                                  const int* sites2 = nullptr, const double* coefs = nullptr) {
   typedef typename A::Z Z;
   const int b = blockIdx.y, c = b / F, f = b % F;
   const int m = m_in[c];
   if (m == 0) return;
+  const int cpw = m <= 16 ? 2 : 1;  // columns per warp
+  const int col0 = blockIdx.x * 8 * cpw;
+  if (col0 >= N) return;
   __shared__ Z Ws[UPD_KMAX][UPD_KMAX + 1];
-  __shared__ Z gb[8][UPD_KMAX];
   __shared__ int st[UPD_KMAX];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int l = tid; l < m; l += 256) st[l] = sites[(long long)c * UPD_KMAX + l];
-  for (int e = tid; e < m * m; e += 256)
-    Ws[e / m][e % m] = A::mk(W[(((long long)c * 2 + f) * UPD_KMAX + e / m) * UPD_KMAX + e % m]);
+  for (int e = tid; e < m * UPD_KMAX; e += 256)
+    if ((e & 31) < m) Ws[e >> 5][e & 31] = A::mk(W[((long long)c * 2 + f) * UPD_KMAX * UPD_KMAX + e]);
   __syncthreads();
-  const int col = blockIdx.x * 8 + ty;
   const zd* Gf = Gv + (long long)c * sG + (long long)f * N * N;
   const long long xy = ((long long)c * 2 + f) * N * UPD_KMAX;
-  if (col < N && tx < m) {
-    const int s = st[tx];
-    const int s2 = sites2 ? sites2[(long long)c * UPD_KMAX + tx] : -1;
-    if (s2 < 0) {
-      X[xy + col + (long long)tx * N] = Gf[col + (long long)s * N];  // row `col` of X
-      gb[ty][tx] = A::mk(zsub(zmk(s == col ? 1.0 : 0.0, 0.0), Gf[s + (long long)col * N]));
-    } else {
-      const double ca = coefs[2 * ((long long)c * UPD_KMAX + tx)], cb = coefs[2 * ((long long)c * UPD_KMAX + tx) + 1];
-      X[xy + col + (long long)tx * N] =
-          zadd(zscale(Gf[col + (long long)s * N], ca), zscale(Gf[col + (long long)s2 * N], cb));
-      const double e = (s == col ? ca : 0.0) + (s2 == col ? cb : 0.0);
-      gb[ty][tx] = A::mk(zsub(zmk(e, 0.0), zadd(zscale(Gf[s + (long long)col * N], ca),
-                                                zscale(Gf[s2 + (long long)col * N], cb))));
+  for (int e = tid; e < m * 8 * cpw; e += 256) {  // rows col0 .. of X
+    const int l = e / (8 * cpw), r = col0 + e % (8 * cpw);
+    if (r >= N) continue;
+    const int s = st[l], s2 = sites2 ? sites2[(long long)c * UPD_KMAX + l] : -1;
+    zd x = Gf[r + (long long)s * N];
+    if (s2 >= 0)
+      x = zadd(zscale(x, coefs[2 * ((long long)c * UPD_KMAX + l)]),
+               zscale(Gf[r + (long long)s2 * N], coefs[2 * ((long long)c * UPD_KMAX + l) + 1]));
+    X[xy + r + (long long)l * N] = x;
+  }
+  const int wd = 32 / cpw, l = lane & (wd - 1);
+  const int col = col0 + warp * cpw + lane / wd;
+  Z y = A::zero();
+  if (col < N && l < m) {
+    const int s = st[l], s2 = sites2 ? sites2[(long long)c * UPD_KMAX + l] : -1;
+    zd g = Gf[s + (long long)col * N];
+    double e = s == col ? 1.0 : 0.0;
+    if (s2 >= 0) {
+      const double ca = coefs[2 * ((long long)c * UPD_KMAX + l)], cb = coefs[2 * ((long long)c * UPD_KMAX + l) + 1];
+      g = zadd(zscale(g, ca), zscale(Gf[s2 + (long long)col * N], cb));
+      e = (s == col ? ca : 0.0) + (s2 == col ? cb : 0.0);
     }
+    y = A::mk(zsub(zmk(e, 0.0), g));
   }
-  __syncthreads();
-  if (col < N && tx < m) {
-    Z y = A::zero();
-    for (int l2 = 0; l2 < m; ++l2) y = A::mac(y, Ws[tx][l2], gb[ty][l2]);
-    Y[xy + tx + (long long)col * UPD_KMAX] = A::wide(y);
+  const int base = lane & ~(wd - 1);
+  const int lr = l < m ? l : 0;
+  for (int k = 0; k + 1 < m; ++k) {
+    const Z yk = A::shfl(y, base + k);
+    if (l > k && l < m) y = A::mac(y, Ws[lr][k], yk);
   }
+  y = A::mul(y, Ws[lr][lr]);
+  for (int k = m - 1; k > 0; --k) {
+    const Z yk = A::shfl(y, base + k);
+    if (l < k) y = A::mac(y, Ws[lr][k], yk);
+  }
+  if (col < N && l < m) Y[xy + l + (long long)col * UPD_KMAX] = A::wide(y);
 }
-

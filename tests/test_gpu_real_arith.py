@@ -112,3 +112,32 @@ def test_real_tau_matches_complex_products(chains, L1, L2):
         assert (c, nt) == (c2, nt2)
         for a, b in zip(qa, qb):
             assert _relmax(a, b) <= 1e-10
+
+
+# the delayed-update block: 2 .. 32 positions, few and nearly all of them accepted (one and two
+# columns of Y per warp in the flush operands), one and several blocks per slice; plain and mixed
+# form, real and complex arithmetic.  Plain form: the oracle's accept sequence and G; mixed form on
+# complex arithmetic runs its visits in double-float: 1e-5, the bound of its parity tests.
+@pytest.mark.parametrize("delay", [2, 7, 17, 32])
+@pytest.mark.parametrize("U", [0.2, 4.0])
+def test_update_blocks(delay, U):
+    m = mdl.hubbard("square", 6, 6, U=U, beta=0.8, dtau=0.1, nwrap=4)
+    f0 = rng.initial_fields(9, 0, m.n_op, m.ltrot)
+    u = rng.sweep_uniforms(9, 0, m.n_op, m.ltrot, 0)
+    o = oracle.Oracle(m)
+    o.set_fields(f0)
+    o.init_state()
+    o.record(1)
+    o.sweep(u)
+    ro = o.recorded()
+    for precision, flags, tol in (("fp64", 0, 1e-10), ("fp64", FLAG_COMPLEX_ARITH, 1e-10), ("mixed", 0, 1e-10),
+                                  ("mixed", FLAG_COMPLEX_ARITH, 1e-5)):
+        g = Chains(m, precision=precision, flags=flags, delay_k=delay)
+        g.set_fields(0, f0)
+        g.init_state()
+        g.set_recording(True)
+        g.sweep(u[None])
+        rg = g.record(0)
+        g.close()
+        compare_record(rg, ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=tol, relative=True,
+                       exact_sequence=precision == "fp64")
