@@ -558,7 +558,7 @@ static int trsv(alfgpu_s* h, const TrsvParams& t) {
 
 static int gemm(alfgpu_s* h, const GemmParams& p) {
   int nl = 1;
-  CK(launch_zgemm(p, h->st, h->gws, h->gws_elems, &nl));
+  CK(launch_zgemm(p, h->st, h->gws, h->gws_elems, &nl, real_model(h)));
   h->launches += nl;
   return 0;
 }

@@ -141,3 +141,25 @@ def test_update_blocks(delay, U):
         g.close()
         compare_record(rg, ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=tol, relative=True,
                        exact_sequence=precision == "fp64")
+
+
+# the real FP64 products: 16 x 16 tiles with one, two and four slices of K (few and many tiles, K
+# remainders of 4 and 64), 64 x 64 tiles (24 chains), every operand form of the sweep with its
+# permutations, triangles and scales: against the complex products, 1e-10 relative
+@pytest.mark.parametrize("chains,L1,L2", [(1, 2, 3), (2, 5, 5), (5, 8, 8), (3, 11, 7), (24, 13, 10)])
+def test_real_products(chains, L1, L2):
+    m = mdl.hubbard("square", L1, L2, U=4.0, beta=0.6, dtau=0.1, nwrap=2)
+    u = np.stack([rng.sweep_uniforms(11, c, m.n_op, m.ltrot, 0) for c in range(chains)])
+    out = []
+    for flags in (0, FLAG_COMPLEX_ARITH):
+        g = Chains(m, n_chains=chains, flags=flags)
+        for c in range(chains):
+            g.set_fields(c, rng.initial_fields(11, c, m.n_op, m.ltrot))
+        g.init_state()
+        g.sweep(u)
+        out.append(([g.green(c) for c in range(chains)], [g.fields(c) for c in range(chains)], g.phase()))
+        g.close()
+    (ga, fa, pa), (gb, fb, pb) = out
+    assert all(np.array_equal(x, y) for x, y in zip(fa, fb))
+    assert all(_relmax(x, y) <= 1e-10 for x, y in zip(ga, gb))
+    assert np.max(np.abs(pa - pb)) <= 1e-10
