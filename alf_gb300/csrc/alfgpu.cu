@@ -571,6 +571,23 @@ static int gemm32(alfgpu_s* h, const GemmParams& g, int tA, int tB, int tC) {
   return 0;
 }
 
+// Whether an N x n x k product of every matrix belongs on the tensor cores: the FP64 GEMM takes at
+// least (N/8)(n/8)(k/4) B DMMAs (zmul of them for one complex product: 2 with a real factor, 4) of
+// 0.30 us on 608 sub-partitions, the tensor-core product a latency of two slicings and a launch.
+// Measured, a wrap of real matrices (two products), FP64 against tensor cores: N = 100, 1 chain 31 / 36 us
+// (4 us of DMMAs each), N = 64, 16 chains 80 / 35 us (16), N = 100, 4 chains 67 / 38 us (17), N = 144, 1 chain
+// 59 / 42 us (12), N = 256, 16 chains 2565 / 171 us; a flush (k = 32): N = 144, 16 chains 42 / 37 us (41),
+// N = 100, 16 chains 24 / 43 us (20).  Mixed form: always, as its arithmetic is.
+#define OZ_MIN_US 8.0
+#define OZ_MIN_FLUSH_US 36.0
+static bool oz_pays(const alfgpu_s* h, int n, int k, int zmul, double min_us) {
+  if (h->d.reserved[0] & ALFGPU_FLAG_TENSOR_WIDE) return true;
+  const int real = real_model(h);
+  if (h->mixed) return true;
+  const double mm = (double)((h->N + 7) / 8) * ((n + 7) / 8) * ((k + 3) / 4) * h->B * (real ? 1 : zmul);
+  return mm * (0.30 / 608.0) >= min_us;
+}
+
 // Digit slices of one operand for k_oz_gemm (see ozaki.cuh for the modes).
 static int oz_slice(alfgpu_s* h, const void* src, int mode, long long sr, long long sk, long long sb, int modb,
                     const zd* ks, long long sks, int srows, int Kc, const int* kdyn, int S, int bits, int Rpad,
@@ -590,13 +607,15 @@ static int oz_gemm(alfgpu_s* h, const CUtensorMap& ta, const CUtensorMap& tb, in
                    int bits, int bn, int nst, int RpadA, int RpadB, int modA, int modB, const int* expA,
                    const int* expB, int omode, int osub, void* out, long long ldr, long long ldc, long long sout,
                    int batch, const zd* rsc = nullptr, long long srsc = 0, int SbA = 0, int SbB = 0,
-                   const zd* csc = nullptr, long long scsc = 0, int persist_ctas = 0) {
+                   const zd* csc = nullptr, long long scsc = 0, int persist_ctas = 0, int kvalid = 0) {
   OzGemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.N = Nn; p.nkc = Kpad / OZ_KC; p.S = S; p.bits = bits; p.nst = nst; p.nd = S + 1;
   p.SbA = SbA > 0 ? SbA : S; p.SbB = SbB > 0 ? SbB : S;
   p.csc = csc; p.scsc = scsc;
-  p.L = oz_shift(Kpad, bits, S, p.nd);
+  p.Kv = ((kvalid > 0 ? kvalid : Kpad) + 15) / 16;
+  oz_words(kvalid > 0 ? kvalid : Kpad, bits, S, p.nd, &p.lg, &p.pair);
+  if (h->mixed && h->oz_narrow && h->oz_Kpad <= 128) p.L = oz_shift(Kpad, bits, S, p.nd);
   p.RpadA = RpadA; p.RpadB = RpadB; p.modA = modA; p.modB = modB; p.expA = expA; p.expB = expB;
   p.omode = omode; p.osub = osub; p.out = out; p.ldr = ldr; p.ldc = ldc; p.sout = sout; p.err = h->err;
   p.rsc = rsc; p.srsc = srsc;
@@ -618,6 +637,30 @@ static int oz_gemm(alfgpu_s* h, const CUtensorMap& ta, const CUtensorMap& tb, in
   h->launches++;
   CKL();
   return 0;
+}
+
+// Real models: the digit slices of the rows of a real matrix (its elements sr, sk, sb doubles apart)
+// and a product of two real slice buffers with N rows each, written to complex128 (zero imaginary
+// parts).
+static int oz_slice_r(alfgpu_s* h, const void* src, long long sr, long long sk, long long sb, const zd* ks, int S,
+                      unsigned short* out, int* expo) {
+  return oz_slice(h, src, OZ_REAL, sr, sk, sb, 0, ks, h->N, h->N, h->N, nullptr, S, h->oz_bits, h->oz_RpN, h->oz_Kpad,
+                  out, expo, h->B);
+}
+// X <- diag(rsc) expT diag(ks) X for the B matrices X (columns sliced first, so in place), S
+// slices; ks or rsc may be null.
+static int oz_left(alfgpu_s* h, zd* X, const zd* ks, const zd* rsc, int S) {
+  const int N = h->N, B = h->B;
+  const long long NN = (long long)N * N;
+  if (real_model(h)) {
+    RET(oz_slice_r(h, X, 2ll * N, 2, 2 * NN, ks, S, h->ozGB, h->ozGBe));
+    return oz_gemm(h, h->tmE[0], h->tmGB, N, N, h->oz_Kpad, S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN, h->oz_RpN,
+                   h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_REALZ, 0, X, 1, N, NN, B, rsc, N, h->oz_S, S, nullptr, 0, 0, N);
+  }
+  RET(oz_slice(h, X, OZ_CROWS, N, 1, NN, 0, ks, N, N, N, nullptr, S, h->oz_bits, h->oz_Rp2N, h->oz_Kpad, h->ozGB,
+               h->ozGBe, B));
+  return oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN, h->oz_Rp2N,
+                 h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, X, 1, N, NN, B, rsc, N, h->oz_S, S, nullptr, 0, 0, N);
 }
 
 // Slices of expT / expTinv (real, per flavour) as the M-side (rows i, K = columns) and
@@ -643,7 +686,7 @@ static int oz_slice_expT(alfgpu_s* h) {
 // products combined in the epilogue.  The real parts of rs / cs are used (the call sites pass
 // real singular values); alpha = 1, beta in {0, 1}, square N x N x N only.
 static bool oz_stab_ok(alfgpu_s* h, const GemmParams& g) {
-  return h->mixed && h->oz && h->oz_stab && !g.realA && !g.realB && !g.ks && !g.kdyn && g.modA == 0 &&
+  return h->oz && h->oz_stab && oz_pays(h, h->N, h->N, 4, OZ_MIN_US) && !g.realA && !g.realB && !g.ks && !g.kdyn && g.modA == 0 &&
          g.modB == 0 && g.alpha.x == 1.0 && g.alpha.y == 0.0 && g.beta.y == 0.0 &&
          (g.beta.x == 0.0 || g.beta.x == 1.0) && g.m == h->N && g.n == h->N && g.k == h->N && g.opA != OP_T &&
          g.opB != OP_T && g.batch == h->B;
@@ -668,6 +711,16 @@ static int oz_zgemm(alfgpu_s* h, const GemmParams& g) {
   bq.rsc = g.cs; bq.srsc = g.sCS; bq.rinv = g.csInv;
   bq.out = h->ozGB; bq.expo = h->ozGBe;
   h->launches += 2;
+  if (real_model(h)) {  // real rows: element strides in doubles
+    for (OzSliceParams* q : {&a, &bq}) {
+      q->mode = OZ_REAL; q->sr *= 2; q->sk *= 2; q->sb *= 2; q->Rpad = h->oz_RpN;
+    }
+    CK(oz_launch_slice(a, h->B, h->st));
+    CK(oz_launch_slice(bq, h->B, h->st));
+    return oz_gemm(h, h->tmGA, h->tmGB, N, N, h->oz_Kpad, h->oz_S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN,
+                   h->oz_RpN, 0, 0, h->ozGAe, h->ozGBe, OZ_OUT_REALZ, g.beta.x == 1.0 ? -1 : 0, g.C, 1, g.ldc, g.sC,
+                   h->B, nullptr, 0, 0, 0, nullptr, 0, 0, N);
+  }
   CK(oz_launch_slice(a, h->B, h->st));
   CK(oz_launch_slice(bq, h->B, h->st));
   return oz_gemm(h, h->tmGA, h->tmGB, 2 * N, 2 * N, h->oz_Kpad, h->oz_S, h->oz_bits, h->oz_bn, h->oz_nst,
@@ -675,10 +728,9 @@ static int oz_zgemm(alfgpu_s* h, const GemmParams& g) {
                  g.ldc, g.sC, h->B);
 }
 
-// The mixed form's UDV propagation runs on the tensor-core GEMM (FP64-accurate) when the
-// slice scales are real.
+// The UDV propagation runs on the tensor-core GEMM (FP64-accurate) when the slice scales are real.
 static bool oz_propagate(alfgpu_s* h) {
-  return h->mixed && h->oz && (!h->eexp_complex || h->pairblock) && !h->mixed_propagate;
+  return h->oz && (!h->eexp_complex || h->pairblock) && !h->mixed_propagate && oz_pays(h, h->N, h->N, 2, OZ_MIN_US);
 }
 
 // Stabilisation products (UDV propagation, decompose, CGR): double-float in the mixed
@@ -889,7 +941,7 @@ static int orgqr_any(alfgpu_s* h, const zd* F, zd* Q) {
   // compact WY pays on batched grids of complex matrices; one chain's grid is too small for its
   // launch chain, and real columns take a quarter of the FP64 instructions (16 chains, N = 256,
   // per sweep: compact WY 110 ms, real columns 70 ms)
-  if (h->oz_stab && !h->oz_narrow && !h->qr_df && !real_model(h) && N <= 32 * BQR_LROWS) return orgqr_wy(h, F, Q);
+  if (h->mixed && h->oz_stab && !h->oz_narrow && !h->qr_df && !real_model(h) && N <= 32 * BQR_LROWS) return orgqr_wy(h, F, Q);
   if (N > 32 * BQR_LROWS) {  // beyond the rows a lane of k_bqr_apply holds
     RET(copy_mats(h, Q, F, (size_t)B * NN));
     return launch_orgqr(h, Q, B);
@@ -1046,11 +1098,7 @@ static int wrapur_u(alfgpu_s* h, UDVSet& u, int ntau, int ntau1) {
     }
     if (h->pairblock) {  // U <- P (expT U): the product, then the slice's explicit vertex phases
       if (oz_propagate(h)) {
-        RET(oz_slice(h, u.U, OZ_CROWS, N, 1, (long long)N * N, 0, nullptr, 0, N, N, nullptr, h->ozp_S, h->oz_bits,
-                     h->oz_Rp2N, h->oz_Kpad, h->ozGB, h->ozGBe, B));
-        RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, h->ozp_S, h->oz_bits, h->oz_bn, h->oz_nst,
-                    h->oz_RpN, h->oz_Rp2N, h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, u.U, 1, N,
-                    (long long)N * N, B, nullptr, 0, h->oz_S, h->ozp_S));
+        RET(oz_left(h, u.U, nullptr, nullptr, h->ozp_S));
       } else {
         GemmParams p = gsq(h, B);
         p.A = h->expT; p.realA = 1; p.modA = h->F;
@@ -1063,11 +1111,7 @@ static int wrapur_u(alfgpu_s* h, UDVSet& u, int ntau, int ntau1) {
     }
     RET(slice_scale(h, nt));
     if (oz_propagate(h)) {  // U <- diag(S) expT U on the tensor cores, in place (U is sliced first)
-      RET(oz_slice(h, u.U, OZ_CROWS, N, 1, (long long)N * N, 0, nullptr, 0, N, N, nullptr, h->ozp_S, h->oz_bits,
-                   h->oz_Rp2N, h->oz_Kpad, h->ozGB, h->ozGBe, B));
-      RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, h->ozp_S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN,
-                  h->oz_Rp2N, h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, u.U, 1, N, (long long)N * N, B, h->S,
-                  N, h->oz_S, h->ozp_S));
+      RET(oz_left(h, u.U, nullptr, h->S, h->ozp_S));
       continue;
     }
     GemmParams p = gsq(h, B);
@@ -1101,11 +1145,7 @@ static int wrapul(alfgpu_s* h, int ntau1, int ntau) {
     if (h->pairblock) {  // U <- expT (P^dagger U): the slice's explicit vertex phases, then the product
       RET(vtx_left_adj(h, h->udvl.U, nt));
       if (oz_propagate(h)) {
-        RET(oz_slice(h, h->udvl.U, OZ_CROWS, N, 1, (long long)N * N, 0, nullptr, 0, N, N, nullptr, h->ozp_S,
-                     h->oz_bits, h->oz_Rp2N, h->oz_Kpad, h->ozGB, h->ozGBe, B));
-        RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, h->ozp_S, h->oz_bits, h->oz_bn, h->oz_nst,
-                    h->oz_RpN, h->oz_Rp2N, h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, h->udvl.U, 1, N,
-                    (long long)N * N, B, nullptr, 0, h->oz_S, h->ozp_S));
+        RET(oz_left(h, h->udvl.U, nullptr, nullptr, h->ozp_S));
       } else {
         GemmParams q = gsq(h, B);
         q.A = h->expT; q.realA = 1; q.modA = h->F;
@@ -1117,11 +1157,7 @@ static int wrapul(alfgpu_s* h, int ntau1, int ntau) {
     }
     RET(slice_scale(h, nt));
     if (oz_propagate(h)) {  // U <- expT diag(conj S) U on the tensor cores (S real), in place
-      RET(oz_slice(h, h->udvl.U, OZ_CROWS, N, 1, (long long)N * N, 0, h->S, N, N, N, nullptr, h->ozp_S, h->oz_bits,
-                   h->oz_Rp2N, h->oz_Kpad, h->ozGB, h->ozGBe, B));
-      RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, h->ozp_S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN,
-                  h->oz_Rp2N, h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, h->udvl.U, 1, N, (long long)N * N, B,
-                  nullptr, 0, h->oz_S, h->ozp_S));
+      RET(oz_left(h, h->udvl.U, h->S, nullptr, h->ozp_S));
       continue;
     }
     GemmParams q = gsq(h, B);
@@ -1434,20 +1470,23 @@ static int cgr2_2(alfgpu_s* h, const UDVSet& udv2, const UDVSet& udv1) {
 // PROPRM1 X <- X expTinv diag(Sinv)    (tau_m_mod.F90:238-263)
 // With vector vertices (pairblock) the slice's vertex product is applied explicitly after the
 // product instead of as a row / column scale.
-static bool oz_tau(alfgpu_s* h) { return h->mixed && h->oz && (!h->eexp_complex || h->pairblock); }
+static bool oz_tau(alfgpu_s* h) {
+  return h->oz && (!h->eexp_complex || h->pairblock) && oz_pays(h, h->N, h->N, 2, OZ_MIN_US);
+}
 static int oz_propr(alfgpu_s* h, zd* X, int nt1) {
-  const int N = h->N, B = h->B, S = h->ozw_S;
-  const long long NN = (long long)N * N;
-  RET(oz_slice(h, X, OZ_CROWS, N, 1, NN, 0, nullptr, 0, N, N, nullptr, S, h->oz_bits, h->oz_Rp2N, h->oz_Kpad,
-               h->ozGB, h->ozGBe, B));
-  RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, h->oz_Kpad, S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN,
-              h->oz_Rp2N, h->F, 0, h->ozEe[0], h->ozGBe, OZ_OUT_COLS, 0, X, 1, N, NN, B,
-              h->pairblock ? nullptr : h->S, N, h->oz_S, S));
+  RET(oz_left(h, X, nullptr, h->pairblock ? nullptr : h->S, h->ozw_S));
   return h->pairblock ? vtx_left(h, X, nt1) : 0;
 }
 static int oz_proprm1(alfgpu_s* h, zd* X, int nt1) {
   const int N = h->N, B = h->B, S = h->ozw_S;
   const long long NN = (long long)N * N;
+  if (real_model(h)) {
+    RET(oz_slice_r(h, X, 2, 2ll * N, 2 * NN, nullptr, S, h->ozGA, h->ozGAe));
+    RET(oz_gemm(h, h->tmGA, h->tmE[3], N, N, h->oz_Kpad, S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_RpN, h->oz_RpN, 0,
+                h->F, h->ozGAe, h->ozEe[3], OZ_OUT_REALZ, 0, X, 1, N, NN, B, nullptr, 0, S, h->oz_S,
+                h->pairblock ? nullptr : h->Sinv, N, 0, N));
+    return h->pairblock ? vtx_right_inv(h, X, nt1) : 0;
+  }
   RET(oz_slice(h, X, OZ_CROWS, 1, N, NN, 0, nullptr, 0, N, N, nullptr, S, h->oz_bits, h->oz_Rp2N, h->oz_Kpad,
                h->ozGA, h->ozGAe, B));
   RET(oz_gemm(h, h->tmGA, h->tmE[3], 2 * N, N, h->oz_Kpad, S, h->oz_bits, h->oz_bn, h->oz_nst, h->oz_Rp2N,
@@ -1561,7 +1600,7 @@ static int hop_impl(alfgpu_s* h, int up, int with_scale) {
     RET(cb_apply(h, h->G, up ? CB_MMTHR : CB_MMTHL));
     return cb_apply(h, h->G, up ? CB_MMTHL_M1 : CB_MMTHR_M1);
   }
-  if (h->mixed && h->oz && !(with_scale && h->eexp_complex)) {
+  if (h->oz && !(with_scale && h->eexp_complex) && oz_pays(h, N, N, 2, OZ_MIN_US)) {
     // up:   T1 = expT diag(S) G (row-major), G = T1 diag(Sinv) expTinv
     // down: T1 = G diag(S) expT (column-major), G = expTinv diag(Sinv) T1
     // the wraps use the first ozw_S digit slices (the expT slices hold oz_S per flavour)
@@ -1570,6 +1609,18 @@ static int hop_impl(alfgpu_s* h, int up, int with_scale) {
     const int bn = h->oz_bn, nst = h->oz_nst;
     const zd* s1 = with_scale ? h->S : nullptr;
     const zd* s2 = with_scale ? h->Sinv : nullptr;
+    if (real_model(h)) {
+      // the left product first in both directions, so that G's columns and the intermediate's rows
+      // are sliced along their storage: T1 = expT diag(S) G (down: expTinv diag(Sinv) G), real rows
+      const int ldt = (N + 1) & ~1;
+      double* T1 = reinterpret_cast<double*>(h->T1);
+      RET(oz_slice_r(h, h->G, 2ll * N, 2, 2 * NN, up ? s1 : s2, S, h->ozGB, h->ozGBe));
+      RET(oz_gemm(h, h->tmE[up ? 0 : 1], h->tmGB, N, N, Kp, S, bits, bn, nst, RpN, RpN, F, 0, h->ozEe[up ? 0 : 1],
+                  h->ozGBe, OZ_OUT_REAL, 0, T1, ldt, 1, (long long)ldt * N, B, nullptr, 0, SE, S, nullptr, 0, 0, N));
+      RET(oz_slice_r(h, T1, ldt, 1, (long long)ldt * N, up ? s2 : s1, S, h->ozGA, h->ozGAe));
+      return oz_gemm(h, h->tmGA, h->tmE[up ? 3 : 2], N, N, Kp, S, bits, bn, nst, RpN, RpN, 0, F, h->ozGAe,
+                     h->ozEe[up ? 3 : 2], OZ_OUT_REALZ, 0, h->G, 1, N, NN, B, nullptr, 0, S, SE, nullptr, 0, 0, N);
+    }
     if (up) {
       RET(oz_slice(h, h->G, OZ_CROWS, N, 1, NN, 0, s1, N, N, N, nullptr, S, bits, Rp2, Kp, h->ozGB, h->ozGBe, B));
       RET(oz_gemm(h, h->tmE[0], h->tmGB, N, 2 * N, Kp, S, bits, bn, nst, RpN, Rp2, F, 0, h->ozEe[0], h->ozGBe,
@@ -1587,7 +1638,7 @@ static int hop_impl(alfgpu_s* h, int up, int with_scale) {
     }
     return 0;
   }
-  if (h->mixed) {
+  if (h->mixed && !(h->oz && real_model(h))) {
     const double* E1 = up ? h->expT : h->expTinv;
     const double* E2 = up ? h->expTinv : h->expT;
     if (up) {
@@ -1652,12 +1703,12 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
   const size_t nblk = h->blk_start[dir].size();
   // the overlap needs room on the SMs next to the flush: the default tensor-core flush tiles fill
   // them (one CTA per SM by shared memory and TMEM), the paired tiles leave room for k_update
-  const bool ozf = h->mixed && h->oz && !h->oz_narrow && !(h->d.reserved[0] & ALFGPU_FLAG_DF_FLUSH);
+  const bool dff = h->d.reserved[0] & ALFGPU_FLAG_DF_FLUSH;
+  const bool ozf = h->oz && !(h->mixed && dff) &&
+                   (h->mixed ? !h->oz_narrow : real_model(h) && oz_pays(h, N, UPD_KMAX, 1, OZ_MIN_FLUSH_US));
   const bool ov = h->overlap && (!ozf || h->ozf_pairs) && !h->pairblock && !h->profiling && nblk > 1;
-  // Visits in real FP64 on real models in both forms (28 us for 32 positions, 59 us in
-  // double-float), else in double-float in the mixed form.
   const int real = real_model(h);
-  const bool dfv = h->mixed && !(h->d.reserved[0] & ALFGPU_FLAG_FP64_VISITS);
+  const bool dfv = h->mixed && !(h->d.reserved[0] & ALFGPU_FLAG_FP64_VISITS);  // visits in double-float
   const long long msz = (long long)h->C + h->B;
   VertexDev V;
   V.site = h->v_site; V.site2 = h->v_site2; V.nsite = h->v_nsite; V.type = h->v_type; V.sK = (long long)F * M;
@@ -1698,7 +1749,8 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       u.vsite2 = h->v_blk2; u.vcoef = h->v_vc; u.sites2_out = h->sites2_out; u.coef_out = h->coef_out;
     }
     prof_begin(h, ALFGPU_PROF_UPDATE);
-    if (real) k_update<ArRe><<<h->C, UPD_THREADS, upd_smem_bytes(8), su>>>(u);
+    if (real && dfv) k_update<ArFRe><<<h->C, UPD_THREADS, upd_smem_bytes(8), su>>>(u);
+    else if (real) k_update<ArRe><<<h->C, UPD_THREADS, upd_smem_bytes(8), su>>>(u);
     else if (dfv) k_update<ArF><<<h->C, UPD_THREADS, upd_smem_bytes(), su>>>(u);
     else k_update<ArD><<<h->C, UPD_THREADS, upd_smem_bytes(), su>>>(u);
     prof_end(h);
@@ -1711,7 +1763,9 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
     const int* s2o = h->pairblock ? h->sites2_out : nullptr;
     const double* co = h->pairblock ? h->coef_out : nullptr;
     const dim3 gxy((N + 7) / 8, h->B);
-    if (real)
+    if (real && dfv)
+      k_flush_xy<ArFRe><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
+    else if (real)
       k_flush_xy<ArRe><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
     else if (dfv)
       k_flush_xy<ArF><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
@@ -1740,8 +1794,17 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
     if (F == 1) { p.sA = 2ll * N * UPD_KMAX; p.sB = 2ll * N * UPD_KMAX; }
     p.kdyn = mb + h->C;  // per-(chain, flavour) rank, written by k_update
     if (ozf) {
-      // G -= X Y as one real product: [Re X | Im X] times the K-doubled complex rows of Y
       const int Kf = 2 * UPD_KMAX;
+      if (real) {  // K = 32: the first half of the slice buffers' K extent
+        RET(oz_slice(h, h->X, OZ_REAL, 2, 2ll * N, 2 * p.sA, 0, nullptr, 0, N, UPD_KMAX, p.kdyn, h->ozf_S, h->ozf_bits,
+                     h->oz_RpN, Kf, h->ozXA, h->ozXAe, h->B));
+        RET(oz_slice(h, h->Y, OZ_REAL, 2ll * UPD_KMAX, 2, 2 * p.sB, 0, nullptr, 0, N, UPD_KMAX, p.kdyn, h->ozf_S,
+                     h->ozf_bits, h->oz_RpN, Kf, h->ozYB, h->ozYBe, h->B));
+        RET(oz_gemm(h, h->tmXA, h->tmYB, N, N, Kf, h->ozf_S, h->ozf_bits, h->ozf_bn, h->ozf_nst, h->oz_RpN, h->oz_RpN,
+                    0, 0, h->ozXAe, h->ozYBe, OZ_OUT_REALZ, 1, h->G, 1, N, NN, h->B, nullptr, 0, 0, 0, nullptr, 0,
+                    h->ozf_grid, UPD_KMAX));
+      } else {
+      // G -= X Y as one real product: [Re X | Im X] times the K-doubled complex rows of Y
       RET(oz_slice(h, h->X, OZ_CKA, 1, N, p.sA, 0, nullptr, 0, N, UPD_KMAX, p.kdyn, h->ozf_S, h->ozf_bits,
                    h->oz_RpN, Kf, h->ozXA, h->ozXAe, h->B));
       RET(oz_slice(h, h->Y, OZ_CKB, UPD_KMAX, 1, p.sB, 0, nullptr, 0, N, UPD_KMAX, p.kdyn, h->ozf_S, h->ozf_bits,
@@ -1749,6 +1812,11 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       RET(oz_gemm(h, h->tmXA, h->tmYB, N, 2 * N, Kf, h->ozf_S, h->ozf_bits, h->ozf_bn, h->ozf_nst, h->oz_RpN,
                   h->oz_Rp2N, 0, 0, h->ozXAe, h->ozYBe, OZ_OUT_COLS, 1, h->G, 1, N, NN, h->B, nullptr, 0, 0, 0,
                   nullptr, 0, h->ozf_grid));
+      }
+    } else if (h->mixed && real) {
+      const int t32 = (N + 31) / 32;
+      k_df_flush<<<dim3(t32, t32, h->B), 256, 0, h->st>>>(h->X, p.sA, h->Y, p.sB, h->G, NN, N, p.kdyn);
+      CKL();
     } else if (h->mixed) RET(gemm32(h, p, ST_C128, ST_C128, ST_C128));
     else RET(gemm(h, p));
     prof_end(h);
@@ -1798,15 +1866,19 @@ static int oz_setup(alfgpu_s* h) {
   const int N = h->N;
   const size_t B = h->B, F = h->F;
   h->oz = 0;
-  h->oz_Kpad = oz_round(N, OZ_KC);
-  h->oz_RpN = oz_round(N, OZ_BM);
-  h->oz_Rp2N = oz_round(2 * N, OZ_BM);
-  if (oz_pick(h->oz_Kpad, &h->oz_bits, &h->oz_S) || oz_pick(2 * UPD_KMAX, &h->ozf_bits, &h->ozf_S)) return 0;
+  h->oz_Kpad = oz_roundup(N, OZ_KC);
+  h->oz_RpN = oz_roundup(N, OZ_BM);
+  h->oz_Rp2N = oz_roundup(2 * N, OZ_BM);
+  // mixed form 55 bits of each row's scale; FP64 form 62, below the roundings of an FP64 product
+  const int bits = h->mixed ? OZ_TARGET_BITS : 61;
+  if (h->N > 512 || oz_pick(h->oz_Kpad, &h->oz_bits, &h->oz_S, bits) ||
+      oz_pick(2 * UPD_KMAX, &h->ozf_bits, &h->ozf_S, bits))
+    return 0;
   // digit slices of the G wraps / TAU_M propagation (reserved[1]) and the UDV propagation
   // (reserved[2]): the target bits rounded up to whole slices, at most oz_S
   auto slices_for = [&](int target) {
-    if (target <= 0) return h->oz_S;
-    const int s = (target + h->oz_bits - 1) / h->oz_bits;
+    if (target <= 0 || !h->mixed) return h->oz_S;
+    const int s = (target + h->oz_bits) / h->oz_bits;  // one bit is the sign
     return std::max(2, std::min(h->oz_S, s));
   };
   h->ozw_S = slices_for(h->d.reserved[1]);
@@ -1817,21 +1889,14 @@ static int oz_setup(alfgpu_s* h) {
   const long long tiles = (long long)((N + OZ_BM - 1) / OZ_BM) * ((2 * N + 31) / 32) * (long long)B;
   const int narrow = tiles < 2ll * nsm && !(h->d.reserved[0] & ALFGPU_FLAG_TENSOR_WIDE);
   h->oz_narrow = narrow;
-  if (oz_pick_tile(h->oz_S, h->oz_Kpad / OZ_KC, &h->oz_bn, &h->oz_nst,
-                   narrow || (h->d.reserved[0] & ALFGPU_FLAG_OZ_DEEP_RING)) ||
+  const int fl = h->d.reserved[0];
+  if (oz_pick_tile(h->oz_S, h->oz_Kpad / OZ_KC, &h->oz_bn, &h->oz_nst, narrow || (fl & ALFGPU_FLAG_OZ_DEEP_RING),
+                   !narrow && !(fl & ALFGPU_FLAG_OZ_DEEP_RING)) ||
       oz_pick_tile(h->ozf_S, 2 * UPD_KMAX / OZ_KC, &h->ozf_bn, &h->ozf_nst, narrow))
     return 0;
-  if (!narrow && (h->d.reserved[0] & ALFGPU_FLAG_OZ_FLUSH_RESIDENT)) {
-    // K = 64 products as persistent CTAs, one per SM, that keep a tile's A digit slices in a ring
-    // of S stages and reuse them for the following tiles of the same M-tile
-    if (oz_smem_bytes(32, h->ozf_S, 1, h->ozf_S) <= 227 * 1024) {
-      h->ozf_bn = 32;
-      h->ozf_nst = h->ozf_S;
-      h->ozf_grid = nsm;
-    }
-  } else if (!narrow && !(h->d.reserved[0] & ALFGPU_FLAG_OZ_FLUSH_SINGLE)) {
+  if (!narrow && !(fl & ALFGPU_FLAG_OZ_FLUSH_SINGLE)) {
     // K = 64 products (flush, compact-WY update) on 16-wide tiles with a ring small enough for
-    // two CTAs per SM ((S + 1) x 16 TMEM columns round to 256 of the SM's 512) and room beside
+    // two CTAs per SM ((S + 1) x 16 TMEM columns round to 128 or 256 of the SM's 512) and room beside
     // them for one k_update CTA, so the next block's visits can overlap the flush
     int st = 8;
     while (st > 2 && 2 * oz_smem_bytes(16, h->ozf_S, 1, st) + upd_smem_bytes() + 16 * 1024 > 227 * 1024) --st;
@@ -1875,6 +1940,8 @@ static int oz_setup(alfgpu_s* h) {
     if (cudaFuncSetAttribute(k_oz_gemm<16, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(k_update<ArRe>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaFuncSetAttribute(k_update<ArFRe>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
         cudaFuncSetAttribute(k_update<ArF>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
@@ -1938,6 +2005,7 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
       return fail(ALFGPU_ERROR_CUDA);
   }
   if (raise_smem_limit(k_update<ArRe>, upd_smem_bytes(8)) != cudaSuccess ||
+      raise_smem_limit(k_update<ArFRe>, upd_smem_bytes(8)) != cudaSuccess ||
       raise_smem_limit(k_update<ArD>, upd_smem_bytes()) != cudaSuccess ||
       raise_smem_limit(k_update<ArF>, upd_smem_bytes()) != cudaSuccess)
     return fail(ALFGPU_ERROR_CUDA);
@@ -2038,10 +2106,10 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   r |= dalloc(h, &h->draws, C * 6 * M * L);
   r |= dalloc(h, &h->rngkey, C); r |= dalloc(h, &h->rngctr, C);
   if (r) return fail(ALFGPU_ERROR_CUDA);
-  if (h->mixed && !(d.reserved[0] & ALFGPU_FLAG_NO_TENSOR_GEMM)) {
+  if (!(d.reserved[0] & ALFGPU_FLAG_NO_TENSOR_GEMM)) {
     const int e = oz_setup(h);
     if (e) return fail(e);
-    h->oz_stab = h->oz && !(d.reserved[0] & ALFGPU_FLAG_FP64_STAB_GEMM) && !h->df_stab;
+    h->oz_stab = h->oz && !(h->mixed && (d.reserved[0] & ALFGPU_FLAG_FP64_STAB_GEMM)) && !h->df_stab;
   }
   h->h_key.assign(C, 0); h->h_ctr.assign(C, 0);
   for (size_t c = 0; c < C; ++c) { h->h_key[c] = alf_chain_key(0, c); h->h_ctr[c] = M * L; }
@@ -2761,7 +2829,8 @@ static int oneshot_handle(int N, alfgpu_s** out) {
   memset(&d, 0, sizeof(d));
   d.ndim = N; d.n_fl = 1; d.n_sun = 1; d.n_op = 1; d.ltrot = 1; d.nwrap = 1; d.n_chains = 1;
   d.precision = ALFGPU_PRECISION_FP64;
-  d.reserved[0] = ALFGPU_FLAG_EXACT_QRP;  // decompose_UDV_state / CGR default branch: ZGEQP3 pivoting
+  // decompose_UDV_state / CGR default branch: ZGEQP3 pivoting; one matrix: no tensor-core buffers
+  d.reserved[0] = ALFGPU_FLAG_EXACT_QRP | ALFGPU_FLAG_NO_TENSOR_GEMM;
   return alfgpu_create(out, &d);
 }
 
@@ -2917,9 +2986,9 @@ extern "C" int alfgpu_decompose_noalloc(int32_t ndim, char side, double* U, doub
 int alfgpu_oz_dgemm(int32_t m, int32_t n, int32_t k, const double* A, int32_t lda, const double* B, int32_t ldb,
                     double* C, int32_t ldc, int32_t device) {
   if (m < 1 || n < 1 || k < 1 || !A || !B || !C || lda < m || ldb < k || ldc < m) return ALFGPU_ERROR_ARGUMENT;
-  const int Kp = oz_round(k, OZ_KC);
+  const int Kp = oz_roundup(k, OZ_KC);
   int bits = 0, S = 0, bn = 0, nst = 0;
-  if (oz_pick(Kp, &bits, &S) || oz_pick_tile(S, Kp / OZ_KC, &bn, &nst)) return ALFGPU_ERROR_SIZE;
+  if (k > 512 || oz_pick(Kp, &bits, &S) || oz_pick_tile(S, Kp / OZ_KC, &bn, &nst)) return ALFGPU_ERROR_SIZE;
   if (!oz_encoder()) return ALFGPU_ERROR_CUDA;
   alfgpu_s* h = new alfgpu_s();
   h->dev = device;
@@ -2927,7 +2996,7 @@ int alfgpu_oz_dgemm(int32_t m, int32_t n, int32_t k, const double* A, int32_t ld
   auto run = [&]() -> int {
     CK(cudaSetDevice(device));
     CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
-    const int RpA = oz_round(m, OZ_BM), RpB = oz_round(n, OZ_BM);
+    const int RpA = oz_roundup(m, OZ_BM), RpB = oz_roundup(n, OZ_BM);
     double *dA = nullptr, *dB = nullptr, *dC = nullptr;
     unsigned short *sa = nullptr, *sb = nullptr;
     int *ea = nullptr, *eb = nullptr;

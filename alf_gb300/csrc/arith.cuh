@@ -196,3 +196,23 @@ struct ArRe {
   static ALF_DEV R rcopysign(R mag, R sgn) { return copysign(mag, sgn); }
   static ALF_DEV R rshfl_xor(R a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
 };
+
+// Real double-float: ArF on real models (the visits and flush operands of the mixed form).
+struct ArFRe {
+  typedef dff Z;
+  typedef dff R;
+  static constexpr bool kDoubleFloat = true, kReal = true;
+  static ALF_DEV Z mk(zd a) { return df_make(a.x); }
+  static ALF_DEV zd wide(Z a) { return zmk(df_wide(a), 0.0); }
+  static ALF_DEV Z one() { return dff{1.f, 0.f}; }
+  static ALF_DEV Z zero() { return dff{0.f, 0.f}; }
+  static ALF_DEV Z mul(Z a, Z b) { return df_mul(a, b); }
+  static ALF_DEV Z sub(Z a, Z b) { return df_sub(a, b); }
+  static ALF_DEV Z add(Z a, Z b) { return df_add(a, b); }
+  static ALF_DEV Z neg(Z a) { return df_neg(a); }
+  static ALF_DEV Z mac(Z c, Z a, Z b) { return df_fma(c, a, b); }
+  static ALF_DEV Z rcp(Z a) { return df_rcp(a); }
+  static ALF_DEV Z shfl(Z a, int src) {
+    return dff{__shfl_sync(0xffffffffu, a.h, src), __shfl_sync(0xffffffffu, a.l, src)};
+  }
+};

@@ -18,21 +18,38 @@ struct dfz {
   dff r, i;
 };
 
-ALF_DEV dff df_make(double x) {
-  dff v;
-  v.h = __double2float_rn(x);
-  v.l = __double2float_rn(x - (double)v.h);
-  return v;
-}
 ALF_DEV dff df_f(float x) { return dff{x, 0.f}; }
-ALF_DEV double df_wide(dff a) { return (double)a.h + (double)a.l; }
-ALF_DEV dfz dz_make(zd z) { return dfz{df_make(z.x), df_make(z.y)}; }
-ALF_DEV zd dz_wide(dfz z) { return zmk(df_wide(z.r), df_wide(z.i)); }
 
 ALF_DEV dff df_qts(float a, float b) {  // |a| >= |b| or a == 0
   const float s = __fadd_rn(a, b);
   return dff{s, __fsub_rn(b, __fsub_rn(s, a))};
 }
+// FP64 <-> double-float.  The conversion instructions run on the FP64 pipe (64 cycles per warp each),
+// so in the range of FP32 the bits are moved on the integer pipes: x = hi (24 bits, truncated) +
+// the other 29 bits as a float; and the exponent of a float rebiased for the way back.
+ALF_DEV dff df_make(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), sg = hi & 0x80000000u;
+  if (((hi << 1) | lo) == 0u) return dff{0.f, 0.f};
+  const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+  if (e < -70 || e > 100) {
+    dff v;
+    v.h = __double2float_rn(x);
+    v.l = __double2float_rn(x - (double)v.h);
+    return v;
+  }
+  const float h = __uint_as_float(sg | ((unsigned)(e + 127) << 23) | (((hi << 3) | (lo >> 29)) & 0x7fffffu));
+  const float l = __uint2float_rn(lo & 0x1fffffffu) * __uint_as_float(sg | ((unsigned)(e + 75) << 23));
+  return df_qts(h, l);
+}
+ALF_DEV double df_f2d(float f) {
+  const unsigned u = (unsigned)__float_as_int(f), e = (u >> 23) & 0xffu;
+  if (e == 0u && (u << 1) == 0u) return 0.0;
+  if (e == 0u || e == 255u) return (double)f;
+  return __hiloint2double((int)((u & 0x80000000u) | ((e + 896u) << 20) | ((u & 0x7fffffu) >> 3)), (int)(u << 29));
+}
+ALF_DEV double df_wide(dff a) { return df_f2d(a.h) + df_f2d(a.l); }
+ALF_DEV dfz dz_make(zd z) { return dfz{df_make(z.x), df_make(z.y)}; }
+ALF_DEV zd dz_wide(dfz z) { return zmk(df_wide(z.r), df_wide(z.i)); }
 ALF_DEV dff df_ts(float a, float b) {
   const float s = __fadd_rn(a, b);
   const float bb = __fsub_rn(s, a);
@@ -65,6 +82,13 @@ ALF_DEV dff df_dot2(dff a, dff b, dff c, dff d) {
   const float e1 = df_perr(a, b, p1), e2 = df_perr(c, d, p2);
   dff s = df_ts(p1, p2);
   return df_qts(s.h, __fadd_rn(s.l, __fadd_rn(e1, e2)));
+}
+// z + a*b
+ALF_DEV dff df_fma(dff z, dff a, dff b) {
+  const float p = __fmul_rn(a.h, b.h);
+  const float e = df_perr(a, b, p);
+  const dff s = df_ts(z.h, p);
+  return df_qts(s.h, __fadd_rn(s.l, __fadd_rn(z.l, e)));
 }
 // z + a*b + c*d
 ALF_DEV dff df_dot2acc(dff z, dff a, dff b, dff c, dff d) {

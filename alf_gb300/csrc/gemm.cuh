@@ -373,12 +373,13 @@ __global__ void k_zgemm_reduce(GemmParams p) {
 
 // Real products: the tile whose busiest sub-partition has the fewest DMMAs.  16 x 16 tiles (WK
 // slices of K inside the CTA) wherever larger ones leave SMs idle, 64 x 64 tiles once they fill
-// the GPU about three times over (fewer operand reads per product).  Measured, one chain's wrap (two
+// the GPU about three times over (fewer operand reads per product) without much padding.  Measured, one chain's wrap (two
 // products, two flavours): N = 16 61 us complex (32 x 32 tiles) -> 14.7 us, N = 256 409 -> 248 us;
 // eight chains, N = 196 2160 -> 622 us.
 static inline cudaError_t launch_rgemm(const GemmParams& p, cudaStream_t st) {
   const long long t64 = (long long)((p.m + 63) / 64) * ((p.n + 63) / 64) * p.batch;
-  if (t64 >= 3 * 152) {
+  const double pad = (double)((p.m + 63) / 64 * 64) * ((p.n + 63) / 64 * 64) / ((double)p.m * p.n);
+  if (t64 >= 3 * 152 && pad < 1.1) {
     k_zgemm<64, 64, 32, true><<<dim3((p.n + 63) / 64, (p.m + 63) / 64, p.batch), 256, 0, st>>>(p);
     return cudaGetLastError();
   }

@@ -4,33 +4,34 @@
 // multiplication and its applications", Numer. Algorithms 59, 2012).
 //
 // Every row of the M-side operand A (and every row of the N-side operand B, i.e. every
-// output column) is scaled by a power of two 2^-e with |x| < 2^e over the row, and its
-// entries are cut into S signed digits of b bits, x = 2^e sum_s d_s 2^(-b s),
-// |d_s| < 2^b.  The digits are integers, exact in BF16 (b <= 7).  For each anti-diagonal
+// output column) is scaled by a power of two 2^-e, rounded to b S - 1 bits below the row's
+// largest entry and cut into S digits of b bits in balanced form, x = 2^e sum_s d_s 2^(-b s),
+// |d_s| <= 2^(b-1).  The digits are integers, exact in BF16 (b <= 8).  For each anti-diagonal
 // D = s + t <= S + 2 of the digit products, sum_{s+t=D} A_s B_t is accumulated on the
-// tensor cores in FP32; b and S are chosen so that every partial sum is an integer below
-// 2^24, so these accumulations are exact.  The diagonals are combined in 64-bit integer
-// arithmetic and rounded once to FP64.  With S b >= 54 the product carries an error below
-// 2^-53 (max_k |A_ik|) (sum_k |B_kj|) + 2^-53 (max_k |B_kj|) (sum_k |A_ik|) (operand
-// truncation; the dropped diagonals D >= S + 3 add < 2^-56 K max|A_i.| max|B_.j|), i.e.
-// FP64-level on the O(1) entries of Green functions and hopping exponentials; FP32
-// products (2^-24) are not enough there (they are amplified by the stabilisation
-// interval).  Complex products are real GEMMs on interleaved real/imaginary rows
-// (k_oz_slice modes) with the complex element assembled in the epilogue.  The first S'
-// digits of an S-digit slicing are the S'-digit slicing of the same element (same row
-// exponent and digit width), so a product may use a prefix of a buffer's slices (SbA /
+// tensor cores in FP32; b and S are chosen so that every partial sum is an integer of at most
+// 2^24, so these accumulations are exact.  The diagonals are combined exactly (two 64-bit words) and
+// rounded once to FP64.  What is lost: the operands' rounding, 2^-(b S) of the row scale per entry
+// (S b = 56: 55 bits and a sign, FP64 entries near their row's maximum keep all their bits), and
+// the dropped diagonals D >= S + 3, K S 2^(2b-2) 2^(-b(S+3)) of the scales at most (below 2^-58 for
+// digits of random sign), i.e. FP64-level on the O(1) entries of Green functions and hopping
+// exponentials; FP32 products (2^-24) are not enough there (they are amplified by the
+// stabilisation interval).  Balanced digits carry one bit more per product than signed magnitudes:
+// 43 digit products at K = 256 (S = 8, b = 7) for the 53 of nine 6-bit magnitudes.
+// Complex products are real GEMMs on interleaved real/imaginary rows
+// (k_oz_slice modes) with the complex element assembled in the epilogue; real models use plain
+// rows (OZ_REAL, OZ_OUT_REALZ).  The first S' digits of an S-digit slicing are the element rounded
+// to S' digits, so a product may use a prefix of a buffer's slices (SbA /
 // SbB give the buffers' own slice counts): fewer slices trade accuracy, 2^-(b S'), for
 // (S' + 1)(S' + 2)/2 - 2 instead of (S + 1)(S + 2)/2 - 2 digit products.
 //
 //   k_oz_slice  FP64 -> BF16 digit slices [batch][S][Rpad][Kpad] (K contiguous) and the
 //               row exponents, integer arithmetic only (the FP64 pipe is 1/64 of FP32)
-//   k_oz_gemm   one CTA per 128 x BN output tile: all B slices of the tile resident in
-//               shared memory (TMA, 128-byte swizzle), A slices streamed through a ring of
-//               64-wide K chunks by a producer warp; an MMA warp issues, per A slice and
-//               K step, one tcgen05.mma (M = 128, N = up to 256, K = 16, BF16 -> FP32)
-//               against all B slices at once, into S + 1 TMEM accumulators (one per
-//               diagonal, the MMA's column base offset by the A slice index), and
-//               tcgen05.commit releases ring stages; eight warps read TMEM back
+//   k_oz_gemm   one CTA per 128 x BN output tile: per 64-wide K chunk, the chunk's B slices (double
+//               buffered) and its A slices (ring of stages) come by TMA with 128-byte swizzle; an MMA
+//               warp issues, per A slice and K step, one tcgen05.mma (M = 128, N = up to 256,
+//               K = 16, BF16 -> FP32) against all B slices at once, into S + 1 TMEM accumulators (one
+//               per diagonal, the MMA's column base offset by the A slice index), and
+//               tcgen05.commit releases the buffers; eight warps read TMEM back
 //               (tcgen05.ld 32x32b), combine, round, and write complex128/float64.
 #pragma once
 #include <cuda.h>
@@ -42,11 +43,11 @@
 #include "common.cuh"
 
 enum { OZ_REAL = 0, OZ_CROWS = 1, OZ_CKA = 2, OZ_CKB = 3 };
-enum { OZ_OUT_COLS = 0, OZ_OUT_ROWS = 1, OZ_OUT_REAL = 2, OZ_OUT_CPLX = 3 };
+enum { OZ_OUT_COLS = 0, OZ_OUT_ROWS = 1, OZ_OUT_REAL = 2, OZ_OUT_CPLX = 3, OZ_OUT_REALZ = 4 };
 #define OZ_KC 64          // K chunk of one TMA box (128 bytes of BF16)
 #define OZ_BM 128         // MMA M
 #ifndef OZ_TARGET_BITS
-#define OZ_TARGET_BITS 54  // digits x bits per slice >= this (an FP64 mantissa and one guard bit)
+#define OZ_TARGET_BITS 54  // digits x bits per slice > this (an FP64 mantissa, one guard bit and a sign)
 #endif
 
 // ---------------------------------------------------------------------------------------
@@ -62,7 +63,7 @@ struct OzSliceParams {
   int srows;                // source rows (complex rows for OZ_C*)
   int Kc;                   // source K extent (complex k for OZ_C*)
   const int* kdyn;          // optional per-batch valid source K (entries beyond are zero)
-  const int* perm; long long sperm;  // optional K remap (OZ_CROWS): element (i, k) is source (i, perm[k])
+  const int* perm; long long sperm;  // optional K remap (OZ_CROWS, OZ_REAL): element (i, k) is source (i, perm[k])
   int tri, trans;           // tri: zero the strictly lower triangle of the source in storage
                             // coordinates (row, col) = trans ? (k', i) : (i, k'), k' the remapped k
   const zd* rsc; long long srsc; int rinv;  // optional real per-row scale (real part), or its inverse
@@ -70,6 +71,7 @@ struct OzSliceParams {
   int unitlow, doff;        // OZ_CROWS: the source is a unit lower trapezoid (Householder vectors of a
                             // QR panel): storage (r, c) is 0 for r < c + doff, 1 for r == c + doff
   int S, bits;
+  unsigned long long cadd;  // sum_s 2^(bits s + bits - 1), set by oz_launch_slice
   int Rpad, Kpad;
   unsigned short* out;      // BF16 bits, [batch][S][Rpad][Kpad]
   int* expo;                // [batch][Rpad]
@@ -126,43 +128,40 @@ ALF_DEV int oz_ebound(double x, const double* s) {
   return e;
 }
 
-// BF16 bits of the integer d, |d| < 2^22 (exact for |d| < 256): d + 1.5 2^23 in FP32 is
-// exact, subtracting the bias leaves (float)d, whose low 16 bits are zero.
-ALF_DEV unsigned oz_bf16_bits(int d) {
-  const float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
-  return (unsigned)__float_as_int(f) >> 16;
-}
-
-// Digits of one element pair of one logical row, one 32-bit word (two BF16) per slice.
+// Digits of one element pair of one logical row, one 32-bit word (two BF16) per slice: the value
+// rounded to v = x s 2^(b S - 1 - e), |v| <= 2^(b S - 1); with C = sum_s 2^(b s + b - 1) added, the b-bit
+// fields of v + C (the top one unmasked) are the balanced digits plus 2^(b-1).  A field f as
+// float: 2^23 + f in FP32 is exact, subtracting 2^23 + 2^(b-1) leaves the digit, whose low 16
+// bits are zero.
 ALF_DEV void oz_write_pair(const OzSliceParams& p, unsigned* o, double x0, double x1, const double* s0,
                            const double* s1, int e, int* bad) {
   const int bS = p.bits * p.S;
   const unsigned mask = (1u << p.bits) - 1u;
+  const float off = 8388608.0f + (float)(1 << (p.bits - 1));
   const size_t sstride = (size_t)p.Rpad * p.Kpad / 2;
   unsigned long long v[2];
-  int ng[2];
   const double xs[2] = {x0, x1};
   const double* ss[2] = {s0, s1};
+  const unsigned long long C = p.cadd;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const OzNum n = oz_num(xs[u], ss[u], bad);
-    ng[u] = n.neg;
-    v[u] = 0ull;
+    v[u] = C;
     if (n.m) {
-      const int sh = n.e2 + bS - e;  // |x s| 2^(bS - e) < 2^bS
-      v[u] = sh >= 0 ? (sh >= 64 ? 0ull : n.m << sh) : (-sh >= 64 ? 0ull : n.m >> (-sh));
+      const int sh = e - n.e2 - bS;  // |x s| 2^(bS - 1 - e) = m 2^(-sh - 1), rounded (sh >= 0: |x s| < 2^e, bS <= 63)
+      const unsigned long long r = sh >= 64 ? 0ull : ((n.m >> sh) + 1ull) >> 1;
+      v[u] = n.neg ? C - r : C + r;
     }
   }
   const unsigned l0 = (unsigned)v[0], h0 = (unsigned)(v[0] >> 32);
   const unsigned l1 = (unsigned)v[1], h1 = (unsigned)(v[1] >> 32);
   for (int s = 0; s < p.S; ++s) {
     const int sh = p.bits * (p.S - 1 - s);
-    const unsigned a = sh >= 32 ? (h0 >> (sh - 32)) : __funnelshift_r(l0, h0, sh);
-    const unsigned c = sh >= 32 ? (h1 >> (sh - 32)) : __funnelshift_r(l1, h1, sh);
-    int d0 = (int)(a & mask), d1 = (int)(c & mask);
-    if (ng[0]) d0 = -d0;
-    if (ng[1]) d1 = -d1;
-    o[(size_t)s * sstride] = oz_bf16_bits(d0) | (oz_bf16_bits(d1) << 16);
+    const unsigned ms = s ? mask : 2u * mask + 1u;
+    const unsigned a = (sh >= 32 ? (h0 >> (sh - 32)) : __funnelshift_r(l0, h0, sh)) & ms;
+    const unsigned c = (sh >= 32 ? (h1 >> (sh - 32)) : __funnelshift_r(l1, h1, sh)) & ms;
+    const float f0 = __uint_as_float(0x4B000000u + a) - off, f1 = __uint_as_float(0x4B000000u + c) - off;
+    o[(size_t)s * sstride] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
   }
 }
 
@@ -199,7 +198,11 @@ __global__ void __launch_bounds__(256) k_oz_slice(OzSliceParams p) {
     if (k >= Kl) continue;
     switch (p.mode) {
       case OZ_REAL:
-        if (k < kd) x0[u] = srd[i * p.sr + k * p.sk];
+        if (k < kd) {
+          const int kq = p.perm ? p.perm[(size_t)b * p.sperm + k] : k;
+          if (p.tri && (p.trans ? kq > i : i > kq)) break;
+          x0[u] = srd[i * p.sr + kq * p.sk];
+        }
         break;
       case OZ_CROWS:
         if (k < kd) {
@@ -242,9 +245,9 @@ __global__ void __launch_bounds__(256) k_oz_slice(OzSliceParams p) {
   if (e0 == -100000) e0 = 0;
   if (e1 == -100000) e1 = 0;
   const int r0 = two ? 2 * i : i;
-  if (tid == 0) {
-    p.expo[(size_t)b * p.Rpad + r0] = e0;
-    if (two) p.expo[(size_t)b * p.Rpad + r0 + 1] = e1;
+  if (tid == 0) {  // the digits' scale is 2^(e + 1): v carries the sign in its top digit
+    p.expo[(size_t)b * p.Rpad + r0] = e0 + 1;
+    if (two) p.expo[(size_t)b * p.Rpad + r0 + 1] = e1 + 1;
   }
   if (k0 >= Kl) return;
   int bad = 0;
@@ -258,7 +261,10 @@ __global__ void __launch_bounds__(256) k_oz_slice(OzSliceParams p) {
 static inline cudaError_t oz_launch_slice(const OzSliceParams& p, int batch, cudaStream_t st) {
   const int Kl = (p.mode == OZ_CKA || p.mode == OZ_CKB) ? 2 * p.Kc : p.Kc;
   if (Kl > 512) return cudaErrorInvalidValue;
-  k_oz_slice<<<dim3(p.srows, batch), 32 * ((Kl + 63) / 64), 0, st>>>(p);
+  OzSliceParams q = p;
+  q.cadd = 0;
+  for (int s = 0; s < p.S; ++s) q.cadd += 1ull << (p.bits * s + p.bits - 1);
+  k_oz_slice<<<dim3(p.srows, batch), 32 * ((Kl + 63) / 64), 0, st>>>(q);
   return cudaGetLastError();
 }
 
@@ -284,10 +290,15 @@ ALF_DEV bool oz_mbar_try(uint32_t bar, uint32_t parity) {
 }
 // Bounded wait: gives up after ~2^31 SM cycles (about one second) and returns false.
 ALF_DEV bool oz_mbar_wait(uint32_t bar, uint32_t parity) {
+  if (oz_mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   while (!oz_mbar_try(bar, parity))
     if (clock64() - t0 > (1ll << 31)) return false;
   return true;
+}
+// The same for a converged warp: one answer for all its lanes.
+ALF_DEV bool oz_mbar_wait_w(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, oz_mbar_wait(bar, parity)) != 0;
 }
 ALF_DEV void oz_tma_2d(uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar) {
   asm volatile(
@@ -310,6 +321,13 @@ ALF_DEV uint64_t oz_desc(uint32_t saddr) {
 ALF_DEV uint32_t oz_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
 }
+ALF_DEV void oz_mma_acc(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc) {  // D += A B
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
+      "l"(ad), "l"(bd), "r"(idesc)
+      : "memory");
+}
 ALF_DEV void oz_mma(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -317,78 +335,62 @@ ALF_DEV void oz_mma(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, ui
       "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
       : "memory");
 }
+// One lane of the converged warp (the same one each time).
+ALF_DEV bool oz_elect() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
 ALF_DEV void oz_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 ALF_DEV void oz_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 ALF_DEV void oz_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 
-template <int BN>
-ALF_DEV void oz_tmem_ld(uint32_t taddr, uint32_t (&r)[BN]);
-template <>
-ALF_DEV void oz_tmem_ld<32>(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-template <>
-ALF_DEV void oz_tmem_ld<16>(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-template <>
-ALF_DEV void oz_tmem_ld<8>(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// (zh 2^sh + zl) 2^sc rounded to the nearest FP64 (ties to even), 0 < sh < 64, |sum| < 2^95: integer
+// arithmetic without branches.
+ALF_DEV double oz_round(long long zh, long long zl, int sh, int sc) {
+  // the 96-bit sum and its magnitude
+  unsigned long long lo = ((unsigned long long)zh << sh) + (unsigned long long)zl;
+  int w2 = (int)(zh >> (64 - sh)) + (int)(zl >> 63) + (lo < (unsigned long long)zl ? 1 : 0);
+  const int neg = w2 >> 31;
+  const unsigned long long nl = (unsigned long long)(long long)neg;
+  lo = (lo ^ nl) - nl;
+  unsigned a2 = (unsigned)((w2 ^ neg) + (neg && lo == 0ull ? 1 : 0));
+  unsigned a1 = (unsigned)(lo >> 32), a0 = (unsigned)lo;
+  // leading word to the top, then the leading bit; what falls off is kept as a sticky bit
+  int T = 0;
+  if (!a2) { a2 = a1; a1 = a0; a0 = 0u; T = 32; }
+  if (!a2) { a2 = a1; a1 = 0u; T += 32; }
+  const int n = __clz(a2);  // 32 only for zero
+  const unsigned mh = __funnelshift_lc(a1, a2, n);
+  unsigned ml = __funnelshift_lc(a0, a1, n);
+  ml |= ((a0 << (n & 31)) != 0u) ? 1u : 0u;
+  // 53 bits with the implicit one, rounded; a carry out of them raises the exponent by itself
+  const unsigned rem = ml & 0x7ffu;
+  unsigned long long r = (((unsigned long long)mh << 32) | ml) >> 11;
+  r += (rem > 0x400u || (rem == 0x400u && (r & 1ull))) ? 1ull : 0ull;
+  const int be = 95 - T - n + sc + 1023;
+  unsigned long long u = ((unsigned long long)(unsigned)(be - 1) << 52) + r;
+  if (be <= 0 || !a2) u = 0ull;
+  if (be >= 2047 && a2) u = 0x7ff0000000000000ull;
+  return __longlong_as_double((long long)(u | ((unsigned long long)(unsigned)neg << 63)));
 }
 
-// An FP32 value that holds an integer of magnitude < 2^31, as int (bit manipulation on the
-// integer pipes).
-ALF_DEV int oz_f2i(uint32_t u) {
-  const int e = (int)((u >> 23) & 0xff);
-  if (e < 127) return 0;  // |x| < 1: the exact integer sum is 0
-  const int m = (int)((u & 0x7fffffu) | 0x800000u);
-  const int sh = 150 - e;
-  const int v = sh >= 0 ? (m >> sh) : (sh > -8 ? (m << -sh) : 0x7fffffff);
-  return (u >> 31) ? -v : v;
-}
-
-// z 2^sc rounded to the nearest FP64 (ties to even), integer arithmetic only.
-ALF_DEV double oz_i64_to_f64(long long z, int sc) {
-  if (z == 0) return 0.0;
-  const unsigned long long sgn = z < 0 ? (1ull << 63) : 0ull;
-  const unsigned long long a = z < 0 ? (unsigned long long)(-z) : (unsigned long long)z;
-  const int p = 63 - __clzll((long long)a);
-  unsigned long long m;
-  int e = p + sc;
-  if (p > 52) {
-    const int r = p - 52;
-    m = a >> r;
-    const unsigned long long rem = a & ((1ull << r) - 1), half = 1ull << (r - 1);
-    if (rem > half || (rem == half && (m & 1))) {
-      ++m;
-      if (m >> 53) { m >>= 1; ++e; }
-    }
-  } else {
-    m = a << (52 - p);
-  }
-  const int be = e + 1023;
-  if (be <= 0) return __longlong_as_double((long long)sgn);
-  if (be >= 2047) return __longlong_as_double((long long)(sgn | 0x7ff0000000000000ull));
-  return __longlong_as_double((long long)(sgn | ((unsigned long long)be << 52) | (m & 0xfffffffffffffull)));
+// z 2^sc rounded to the nearest FP64 (ties to even), |z| < 2^63.
+ALF_DEV double oz_round1(long long z, int sc) {
+  const unsigned long long nl = (unsigned long long)(z >> 63);
+  const unsigned long long a = ((unsigned long long)z ^ nl) - nl;
+  const int n = __clzll((long long)a);
+  const unsigned long long m = a << (n & 63);
+  const unsigned rem = (unsigned)m & 0x7ffu;
+  unsigned long long r = m >> 11;
+  r += (rem > 0x400u || (rem == 0x400u && (r & 1ull))) ? 1ull : 0ull;
+  const int be = 63 - n + sc + 1023;
+  unsigned long long u = ((unsigned long long)(unsigned)(be - 1) << 52) + r;
+  if (be <= 0 || !a) u = 0ull;
+  if (be >= 2047 && a) u = 0x7ff0000000000000ull;
+  return __longlong_as_double((long long)(u | (nl & 0x8000000000000000ull)));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -397,13 +399,15 @@ ALF_DEV double oz_i64_to_f64(long long z, int sc) {
 struct OzGemmParams {
   int M, N;                  // logical rows of A and of B (valid extents)
   int nkc, S, bits, nst;     // K chunks (Kpad / 64), slices, bits per slice, ring stages
-  int nd;                    // diagonals accumulated: s + t < nd (0-based digit indices)
-  int L;                     // fixed-point position of the combined integer (oz_shift)
+  int nd;                    // diagonals accumulated: s + t < nd (0-based digit indices), nd = S + 1
+  int L;                     // > 0: one 64-bit word with 2^-L as its unit instead of two (oz_words)
+  int lg, pair;              // diagonals in the low word (ND - lg even); two diagonals fit 32 bits (oz_words)
+  int Kv;                    // K steps of 16 that hold digits (the rest of Kpad is zero)
   int RpadA, RpadB;
   int modA, modB;            // operand batch = b % mod when > 0
   const int* expA; const int* expB;
-  int omode, osub;           // OZ_OUT_*; osub 1: out -= A B, -1: out += A B (OZ_OUT_CPLX)
-  void* out; long long ldr, ldc, sout;  // element strides (complex128 for _COLS/_ROWS, float64 for _REAL)
+  int omode, osub;           // OZ_OUT_*; osub 1: out -= A B, -1: out += A B (OZ_OUT_CPLX, OZ_OUT_REALZ)
+  void* out; long long ldr, ldc, sout;  // element strides (float64 for _REAL, complex128 otherwise)
   int* err;                  // bit 2: a bounded wait gave up
   const zd* rsc; long long srsc;  // optional real scale of output row m (real part used), per batch
   const zd* csc; long long scsc;  // optional real scale of output column n (OZ_OUT_ROWS; real part), per batch
@@ -415,30 +419,62 @@ struct OzGemmParams {
 };
 
 static inline size_t oz_smem_bytes(int bn, int S, int nkc, int nst) {
-  return (size_t)(S + 1) * nkc * bn * 128 + (size_t)nst * OZ_BM * 128 + 256 + 1024;
+  return (size_t)S * (nkc > 1 ? 2 : 1) * bn * 128 + (size_t)nst * OZ_BM * 128 + 256 + 1024;
 }
 
-// 256 threads.  Warp 0 lane 0 is the TMA producer (B slices once, A chunks into the ring
-// as stages free up), warp 1 lane 0 issues the MMAs and commits each ring stage back to the
-// producer; then all eight warps read TMEM: warp w takes TMEM lanes 32 (w % 4) .. + 31
-// (its sub-partition's) and columns (w / 4) BN/2 .. + BN/2 - 1.
+template <int HB>
+ALF_DEV void oz_tmem_ld_async(uint32_t taddr, uint32_t (&r)[HB]);
+template <>
+ALF_DEV void oz_tmem_ld_async<16>(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+template <>
+ALF_DEV void oz_tmem_ld_async<8>(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// Waits for the warp's TMEM loads; the registers are tied to the wait so that their uses stay behind it.
+template <int HB>
+ALF_DEV void oz_tmem_wait(uint32_t (&r)[HB], uint32_t (&q)[HB]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < HB; ++j) asm volatile("" : "+r"(r[j]), "+r"(q[j]));
+}
+
+// 256 threads.  Warp 0 lane 0 is the TMA producer (per K chunk the B slices into one of two
+// buffers, then the A slices into the ring, as they free up), warp 1 lane 0 issues the MMAs and
+// commits each buffer back to the producer; then all eight warps read TMEM: warp w takes TMEM
+// lanes 32 (w % 4) .. + 31 (its sub-partition's) and columns (w / 4) BN/2 .. + BN/2 - 1.
+// Holding one chunk's B slices instead of all of them leaves room, at 16-wide tiles, for two CTAs per
+// SM, whose epilogues and main loops overlap.  Measured (K = 256, real): 32 matrices N = 256, 16-wide
+// pairs 64 us, 32-wide with nine stages 67 us; two matrices 16 us and 19 us (start: 32-wide tiles with all B
+// slices resident and one issuing thread, 105 us per real half of a complex product).  The ring's depth
+// (2 .. 9) makes no difference: a chunk of 4 K steps takes ~450 cycles to issue.
 template <int BN, bool PERSIST = false>
-__global__ void __launch_bounds__(256, 1) k_oz_gemm(const __grid_constant__ CUtensorMap tmA,
+__global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_constant__ CUtensorMap tmA,
                                                     const __grid_constant__ CUtensorMap tmB, OzGemmParams p) {
   constexpr int HB = BN / 2;  // columns per epilogue thread
   extern __shared__ unsigned char oz_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int S = p.S, nkc = p.nkc, NST = p.nst, ND = p.nd;
+  const int wu = __shfl_sync(0xffffffffu, warp, 0);  // warp index, uniform for the compiler
+  const int S = p.S, nkc = p.nkc, NST = p.nst, ND = p.nd, NB = nkc > 1 ? 2 : 1;
   const uint32_t raw = oz_smem(oz_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t sB = base;                                     // [nkc][S + 1][BN rows x 128 B], block S zero
-  const uint32_t sA = sB + (uint32_t)((S + 1) * nkc * BN * 128);  // [NST][128 rows x 128 B]
-  const uint32_t sBar = sA + (uint32_t)(NST * OZ_BM * 128);     // full[NST], empty[NST], bfull, done
+  const uint32_t sB = base;                                      // [NB][S][BN rows x 128 B]
+  const uint32_t sA = sB + (uint32_t)(NB * S * BN * 128);        // [NST][128 rows x 128 B]
+  const uint32_t sBar = sA + (uint32_t)(NST * OZ_BM * 128);      // full[NST], empty[NST], bfull[2], bempty[2], done
   unsigned char* gbar = oz_raw + (sBar - raw);
-  const uint32_t full0 = sBar, empty0 = sBar + 8u * NST, bfull = sBar + 16u * NST, done = bfull + 8;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(gbar + 16 * NST + 16);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbar + 16 * NST + 20);
-  volatile int* consumed_sh = reinterpret_cast<volatile int*>(gbar + 16 * NST + 24);
+  const uint32_t full0 = sBar, empty0 = sBar + 8u * NST, bfull0 = sBar + 16u * NST, bempty0 = bfull0 + 16,
+                 done = bfull0 + 32;  // tslot, abort flag and consumed count follow
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(gbar + 16 * NST + 40);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbar + 16 * NST + 44);
+  volatile int* consumed_sh = reinterpret_cast<volatile int*>(gbar + 16 * NST + 48);
+  const uint32_t cons = done + 16;  // shared address of *consumed_sh
   int ncols = 32;
   while (ncols < ND * BN) ncols <<= 1;
 
@@ -450,18 +486,13 @@ __global__ void __launch_bounds__(256, 1) k_oz_gemm(const __grid_constant__ CUte
   }
   if (tid == 32) {
     for (int i = 0; i < NST; ++i) { oz_mbar_init(full0 + 8u * i, 1); oz_mbar_init(empty0 + 8u * i, 1); }
-    oz_mbar_init(bfull, 1);
+    for (int i = 0; i < 2; ++i) { oz_mbar_init(bfull0 + 8u * i, 1); oz_mbar_init(bempty0 + 8u * i, 1); }
     oz_mbar_init(done, 1);
     *abort_flag = 0;
     *consumed_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  for (int kc = 0; kc < nkc; ++kc) {  // block t = S of every K chunk: zeros (read by the s = 0 MMAs)
-    uint4* z = reinterpret_cast<uint4*>(oz_raw + (sB - raw) + (size_t)(kc * (S + 1) + S) * BN * 128);
-    for (int i = tid; i < BN * 8; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
   oz_fence_before();
   __syncthreads();
   oz_fence_after();
@@ -469,25 +500,12 @@ __global__ void __launch_bounds__(256, 1) k_oz_gemm(const __grid_constant__ CUte
   const int total = S * nkc;
   const uint32_t chunkA = OZ_BM * 128, chunkB = BN * 128;
   const int ntile = PERSIST ? p.tiles_n * p.tiles_m * p.tiles_b : 1;
-  // ring stage and round of a chunk follow its count over all tiles of this CTA, kept as running
-  // (stage, round) pairs by the producer and the MMA issuer; bfull and done complete once per
-  // tile (parity = tile iteration & 1)
-  int pst = 0, pround = 0, mst = 0, mround = 0;
+  // stage and round of each A chunk and of each B chunk follow their counts over all tiles of this
+  // CTA, kept as running (stage, round) pairs by the producer (p*) and the MMA issuer (m*); done
+  // completes once per tile (parity = tile iteration & 1)
+  int pst = 0, pround = 0, mst = 0, mround = 0, pbst = 0, pbround = 0, mbst = 0, mbround = 0;
   int it = 0;
-  // A-resident mode (persistent, every A chunk of a tile fits the ring): a CTA takes a contiguous
-  // range of tiles, N-tile fastest, so consecutive tiles share their A chunks, which are loaded
-  // into stages 0 .. total - 1 only when the (batch, M-tile) changes; the ring's empty barriers
-  // are not used (the previous tile's MMAs are complete before the next tile starts)
-  const bool resident = PERSIST && total <= NST;
-  int t_begin = 0, t_end = 1, t_step = 1;
-  if (PERSIST && resident) {
-    t_begin = (int)((long long)ntile * blockIdx.x / gridDim.x);
-    t_end = (int)((long long)ntile * (blockIdx.x + 1) / gridDim.x);
-  } else if (PERSIST) {
-    t_begin = (int)blockIdx.x; t_end = ntile; t_step = (int)gridDim.x;
-  }
-  int keyA_prev = -1, aloads = 0;
-  for (int tix = t_begin; tix < t_end; tix += t_step, ++it) {
+  for (int tix = PERSIST ? (int)blockIdx.x : 0; tix < ntile; tix += PERSIST ? (int)gridDim.x : 1, ++it) {
   int b, m0, n0;
   if (PERSIST) {
     n0 = (tix % p.tiles_n) * BN;
@@ -497,130 +515,236 @@ __global__ void __launch_bounds__(256, 1) k_oz_gemm(const __grid_constant__ CUte
     b = blockIdx.z; m0 = blockIdx.y * OZ_BM; n0 = blockIdx.x * BN;
   }
   const int bA = p.modA > 0 ? b % p.modA : b, bB = p.modB > 0 ? b % p.modB : b;
-  const int g0 = it * total;  // count of this tile's first A chunk
   const uint32_t tpar = (uint32_t)(it & 1);
-  const int keyA = bA * p.tiles_m + m0 / OZ_BM;
-  const bool loadA = !resident || keyA != keyA_prev;
-  if (resident && loadA) { keyA_prev = keyA; ++aloads; }
-  const uint32_t apar = (uint32_t)((aloads - 1) & 1);  // resident A: parity of its load
 
-  if (tid == 0) {  // producer
+  // Both loops run on whole warps, with one elected lane issuing: in a one-thread branch the
+  // compiler cannot keep the descriptors in uniform registers, and an MMA took ~325 cycles to issue.
+  if (wu == 0) {  // producer
     const int rowA0 = bA * p.SbA * p.RpadA + m0, rowB0 = bB * p.SbB * p.RpadB + n0;
-    oz_mbar_expect_tx(bfull, (uint32_t)(S * nkc) * chunkB);
-    for (int t = 0; t < S; ++t)
-      for (int kc = 0; kc < nkc; ++kc)
-        oz_tma_2d(sB + (uint32_t)(kc * (S + 1) + t) * chunkB, &tmB, kc * OZ_KC, rowB0 + t * p.RpadB, bfull);
-    int loaded = 0;
+    const int g0 = it * total, gb0 = it * nkc;  // counts of this tile's first A and B chunk
+    int loaded = 0, bloaded = 0;
     bool ok = true;
-    if (resident) {
-      if (loadA)
-        for (int l = 0; l < total; ++l) {
-          oz_mbar_expect_tx(full0 + 8u * l, chunkA);
-          oz_tma_2d(sA + (uint32_t)l * chunkA, &tmA, (l % nkc) * OZ_KC, rowA0 + (l / nkc) * p.RpadA, full0 + 8u * l);
-        }
-      loaded = total;
-    }
-    for (int s = 0, kc = 0; !resident && loaded < total; ++loaded) {
-      const int st = pst;
-      if (pround > 0 && !oz_mbar_wait(empty0 + 8u * st, (uint32_t)((pround - 1) & 1))) { ok = false; break; }
-      if (*abort_flag) break;
-      oz_mbar_expect_tx(full0 + 8u * st, chunkA);
-      oz_tma_2d(sA + (uint32_t)st * chunkA, &tmA, kc * OZ_KC, rowA0 + s * p.RpadA, full0 + 8u * st);
-      if (++pst == NST) { pst = 0; ++pround; }
-      if (++kc == nkc) { kc = 0; ++s; }
-    }
-    if (!ok) { atomicOr(p.err, 4); *abort_flag = 1; }
-    if (*abort_flag) {  // let every copy issued by this thread land before the CTA exits
-      oz_mbar_wait(bfull, tpar);
-      if (resident) {
-        if (loadA)
-          for (int l = 0; l < total; ++l) oz_mbar_wait(full0 + 8u * l, apar);
-      } else {
-        for (int q = g0 + *consumed_sh; q < g0 + loaded; ++q)
-          oz_mbar_wait(full0 + 8u * (uint32_t)(q % NST), (uint32_t)((q / NST) & 1));
+    for (int kc = 0; ok && kc < nkc; ++kc) {
+      if (pbround > 0 && !oz_mbar_wait_w(bempty0 + 8u * pbst, (uint32_t)((pbround - 1) & 1))) { ok = false; break; }
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      if (oz_elect()) {
+        oz_mbar_expect_tx(bfull0 + 8u * pbst, (uint32_t)S * chunkB);
+        for (int t = 0; t < S; ++t)
+          oz_tma_2d(sB + (uint32_t)(pbst * S + t) * chunkB, &tmB, kc * OZ_KC, rowB0 + t * p.RpadB, bfull0 + 8u * pbst);
       }
+      __syncwarp();
+      ++bloaded;
+      if (++pbst == NB) { pbst = 0; ++pbround; }
+      for (int s = 0; s < S; ++s) {
+        if (pround > 0 && !oz_mbar_wait_w(empty0 + 8u * pst, (uint32_t)((pround - 1) & 1))) { ok = false; break; }
+        if (__any_sync(0xffffffffu, *abort_flag)) break;
+        if (oz_elect()) {
+          oz_mbar_expect_tx(full0 + 8u * pst, chunkA);
+          oz_tma_2d(sA + (uint32_t)pst * chunkA, &tmA, kc * OZ_KC, rowA0 + s * p.RpadA, full0 + 8u * pst);
+        }
+        __syncwarp();
+        ++loaded;
+        if (++pst == NST) { pst = 0; ++pround; }
+      }
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
     }
-  } else if (tid == 32) {  // MMA issuer
+    if (!ok && lane == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
+    __syncwarp();
+    if (__any_sync(0xffffffffu, *abort_flag)) {  // let every copy issued by this warp land before the CTA exits
+      for (int q = gb0; q < gb0 + bloaded; ++q) oz_mbar_wait(bfull0 + 8u * (uint32_t)(q % NB), (uint32_t)((q / NB) & 1));
+      for (int q = g0 + *consumed_sh; q < g0 + loaded; ++q)
+        oz_mbar_wait(full0 + 8u * (uint32_t)(q % NST), (uint32_t)((q / NST) & 1));
+    }
+  } else if (wu == 1) {  // MMA issuer
     oz_fence_after();  // the previous tile's TMEM reads are done (barrier below)
-    bool ok = oz_mbar_wait(bfull, tpar);
+    bool ok = true;
     // descriptors differ only in the start-address field: advance them by (bytes >> 4)
     const uint64_t dA0 = oz_desc(sA), dB0 = oz_desc(sB);
     constexpr int TMAX = 256 / BN;  // B blocks per MMA (N <= 256)
     int q = 0;
-    for (int s = 0, kc = 0; ok && q < total; ++q) {
-      const int st = resident ? q : mst;
-      if (!oz_mbar_wait(full0 + 8u * st, resident ? apar : (uint32_t)(mround & 1))) { ok = false; break; }
-      oz_fence_after();
-      const uint64_t dA = dA0 + (uint64_t)((st * chunkA) >> 4);
-      // A_s times the contiguous blocks B_0 .. B_{nt-1} of this K chunk in one MMA (N = nt BN),
-      // into TMEM columns (s + t) BN: each product lands in its diagonal's accumulator.  For
-      // s = 0 the zero block t = S covers the last diagonal, so every accumulator is written
-      // (not accumulated) by the first K step.
-      const int nt = ND - s;
-      for (int kk = 0; kk < OZ_KC / 16; ++kk) {
-        const uint32_t acc = (s == 0 && kc == 0 && kk == 0) ? 0u : 1u;
-        for (int t0 = 0; t0 < nt; t0 += TMAX) {
-          const int n = min(TMAX, nt - t0);
-          const uint64_t dB = dB0 + (uint64_t)(((kc * (S + 1) + t0) * chunkB) >> 4) + 2u * kk;
-          oz_mma(tbase + (uint32_t)((s + t0) * BN), dA + 2u * kk, dB, oz_idesc(n * BN), acc);
+    for (int kc = 0; ok && kc < nkc; ++kc) {
+      if (!oz_mbar_wait_w(bfull0 + 8u * mbst, (uint32_t)(mbround & 1))) { ok = false; break; }
+      const uint64_t dBk = dB0 + (uint64_t)((uint32_t)(mbst * S) * chunkB >> 4);
+      const int nkk = min(OZ_KC / 16, p.Kv - kc * (OZ_KC / 16));
+      for (int s = 0; s < S; ++s) {
+        if (!oz_mbar_wait_w(full0 + 8u * mst, (uint32_t)(mround & 1))) { ok = false; break; }
+        oz_fence_after();
+        // A_s times the contiguous blocks B_0 .. B_{nt-1} of this K chunk in one MMA (N = nt BN),
+        // into TMEM columns (s + t) BN: each product lands in its diagonal's accumulator.  In the
+        // first K step s = 0 writes the diagonals 0 .. S - 1 and the last block of s = 1 diagonal S;
+        // everything else accumulates.
+        const uint64_t dA = dA0 + (uint64_t)(((uint32_t)mst * chunkA) >> 4);
+        const int nt = min(S, ND - s), n1 = min(TMAX, nt), n2 = nt - n1;  // at most two MMAs per K step
+        const uint32_t d1 = tbase + (uint32_t)(s * BN), d2 = d1 + (uint32_t)(n1 * BN);
+        const uint32_t i1 = oz_idesc(n1 * BN), i2 = oz_idesc(n2 * BN);
+        const uint64_t dB2 = dBk + (uint64_t)((uint32_t)n1 * chunkB >> 4);
+        const bool start = kc == 0 && s < 2;
+        if (oz_elect()) {
+          if (start) {
+            for (int kk = 0; kk < nkk; ++kk) {
+              const int tw = (kk == 0 && s == 1) ? nt - 1 : nt;  // blocks that share one accumulate flag
+              for (int t0 = 0; t0 < tw; t0 += TMAX) {
+                const int n = min(TMAX, tw - t0);
+                oz_mma(tbase + (uint32_t)((s + t0) * BN), dA + 2u * kk,
+                       dBk + (uint64_t)((uint32_t)t0 * chunkB >> 4) + 2u * kk, oz_idesc(n * BN),
+                       (kk == 0 && s == 0) ? 0u : 1u);
+              }
+              if (tw < nt)
+                oz_mma(tbase + (uint32_t)((s + tw) * BN), dA + 2u * kk,
+                       dBk + (uint64_t)((uint32_t)tw * chunkB >> 4) + 2u * kk, oz_idesc(BN), 0u);
+            }
+          } else if (n2) {
+#pragma unroll
+            for (int kk = 0; kk < OZ_KC / 16; ++kk)
+              if (kk < nkk) {
+                oz_mma_acc(d1, dA + 2u * kk, dBk + 2u * kk, i1);
+                oz_mma_acc(d2, dA + 2u * kk, dB2 + 2u * kk, i2);
+              }
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < OZ_KC / 16; ++kk)
+              if (kk < nkk) oz_mma_acc(d1, dA + 2u * kk, dBk + 2u * kk, i1);
+          }
+          oz_commit(empty0 + 8u * mst);
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(cons), "r"(q + 1) : "memory");
+          if (s == S - 1) oz_commit(bempty0 + 8u * mbst);
         }
-      }
-      if (!resident) {
-        oz_commit(empty0 + 8u * st);
+        __syncwarp();
+        ++q;
         if (++mst == NST) { mst = 0; ++mround; }
       }
-      *consumed_sh = q + 1;
-      if (++kc == nkc) { kc = 0; ++s; }
+      if (!ok) break;
+      if (++mbst == NB) { mbst = 0; ++mbround; }
     }
-    if (!ok) { atomicOr(p.err, 4); *abort_flag = 1; }
-    oz_commit(done);  // arrives when every MMA issued above has completed
+    if (!ok && lane == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
+    __syncwarp();
+    if (oz_elect()) oz_commit(done);  // arrives when every MMA issued above has completed
+    __syncwarp();
   }
-  __syncwarp();
+  // the exponents of this thread's outputs, while the products run
+  const int quarter = warp & 3, c0 = (warp >> 2) * HB, m = m0 + 32 * quarter + lane;
+  const int ea = (m < p.M) ? p.expA[(size_t)bA * p.RpadA + m] : 0;
+  int eb[HB];
+#pragma unroll
+  for (int j = 0; j < HB; ++j) {
+    const int n = n0 + c0 + j;
+    eb[j] = (n < p.N) ? p.expB[(size_t)bB * p.RpadB + n] : 0;
+  }
+  double old[HB];  // real outputs that are updated: read while the products run too
+  const bool upd = p.omode == OZ_OUT_REALZ && p.osub != 0;
+  if (upd) {
+    const zd* o = (const zd*)p.out + (size_t)b * p.sout;
+#pragma unroll
+    for (int j = 0; j < HB; ++j)
+      old[j] = (m < p.M && n0 + c0 + j < p.N) ? o[m * p.ldr + (n0 + c0 + j) * p.ldc].x : 0.0;
+  }
   const bool done_ok = oz_mbar_wait(done, tpar);
   oz_fence_after();
   __syncthreads();
   if (!done_ok && lane == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
   if (done_ok && !*abort_flag) {
-    const int quarter = warp & 3, half = warp >> 2;
-    const int c0 = half * HB;  // first tile column of this thread
-    long long Z[HB];
+    // The diagonals in two exact 64-bit words, the last lg of them in the low one.
+    long long Zh[HB], Zl[HB];
 #pragma unroll
-    for (int j = 0; j < HB; ++j) Z[j] = 0;
-    const int L = p.L;
-    for (int d = 0; d < ND; ++d) {
-      uint32_t r[HB];
-      oz_tmem_ld<HB>(tbase + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(d * BN + c0), r);
-      const int sh = L - p.bits * (d + 2);
+    for (int j = 0; j < HB; ++j) { Zh[j] = 0; Zl[j] = 0; }
+    const int lg = p.lg;
+    const uint32_t tcol = tbase + ((uint32_t)(32 * quarter) << 16) + (uint32_t)c0;
+    // The diagonals d, d + 1 first meet in one 32-bit word where it holds them (p.pair).
+    auto f2i = [](uint32_t u) { return __float2int_rn(__uint_as_float(u)); };
+    double v[HB];
+    if (p.L > 0) {
+      // one word, the low diagonals cut to its unit
 #pragma unroll
-      for (int j = 0; j < HB; ++j) {
-        const long long v = (long long)oz_f2i(r[j]);
-        Z[j] += sh >= 0 ? v * (1ll << sh) : ((v + (1ll << (-sh - 1))) >> (-sh));  // rounded
+      for (int j = 0; j < HB; ++j) Zl[j] = 0;
+      auto add = [&](long long& z, long long w, int sh) {
+        z += sh >= 0 ? w << sh : w >> -sh;
+      };
+      for (int d = 0; d < ND; d += 2) {
+        uint32_t r0[HB], r1[HB];
+        const bool two = d + 1 < ND;
+        oz_tmem_ld_async<HB>(tcol + (uint32_t)(d * BN), r0);
+        if (two) oz_tmem_ld_async<HB>(tcol + (uint32_t)((d + 1) * BN), r1);
+        oz_tmem_wait<HB>(r0, r1);
+        const int sh0 = p.L - p.bits * (d + 2), sh1 = sh0 - p.bits;
+        if (two && p.pair) {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) add(Zl[j], (long long)((f2i(r0[j]) << p.bits) + f2i(r1[j])), sh1);
+        } else {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) add(Zl[j], (long long)f2i(r0[j]), sh0);
+          if (two)
+#pragma unroll
+            for (int j = 0; j < HB; ++j) add(Zl[j], (long long)f2i(r1[j]), sh1);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < HB; ++j) v[j] = oz_round1(Zl[j], ea + eb[j] - p.L);
+    } else {
+    for (int d = 0; d < ND; d += 2) {  // two diagonals' loads in flight
+      uint32_t r0[HB], r1[HB];
+      const bool two = d + 1 < ND;
+      oz_tmem_ld_async<HB>(tcol + (uint32_t)(d * BN), r0);
+      if (two) oz_tmem_ld_async<HB>(tcol + (uint32_t)((d + 1) * BN), r1);
+      oz_tmem_wait<HB>(r0, r1);
+      if (two && p.pair) {
+        if (d < ND - lg) {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zh[j] = (Zh[j] << (2 * p.bits)) + (long long)((f2i(r0[j]) << p.bits) + f2i(r1[j]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zl[j] = (Zl[j] << (2 * p.bits)) + (long long)((f2i(r0[j]) << p.bits) + f2i(r1[j]));
+        }
+      } else {
+        if (d < ND - lg) {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zh[j] = (Zh[j] << p.bits) + (long long)f2i(r0[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zl[j] = (Zl[j] << p.bits) + (long long)f2i(r0[j]);
+        }
+        if (two && d + 1 < ND - lg) {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zh[j] = (Zh[j] << p.bits) + (long long)f2i(r1[j]);
+        } else if (two) {
+#pragma unroll
+          for (int j = 0; j < HB; ++j) Zl[j] = (Zl[j] << p.bits) + (long long)f2i(r1[j]);
+        }
       }
     }
-    const int m = m0 + 32 * quarter + lane;
-    const int ea = (m < p.M) ? p.expA[(size_t)bA * p.RpadA + m] : 0;
-    double v[HB];
 #pragma unroll
-    for (int j = 0; j < HB; ++j) {
-      const int n = n0 + c0 + j;
-      const int eb = (n < p.N) ? p.expB[(size_t)bB * p.RpadB + n] : 0;
-      v[j] = oz_i64_to_f64(Z[j], ea + eb - L);
+    for (int j = 0; j < HB; ++j) v[j] = oz_round(Zh[j], Zl[j], p.bits * lg, ea + eb[j] - p.bits * (ND + 1));
     }
     if (p.rsc && m < p.M) {
       const double s = p.rsc[(size_t)b * p.srsc + m].x;
 #pragma unroll
       for (int j = 0; j < HB; ++j) v[j] *= s;
     }
-    if (p.csc) {  // OZ_OUT_ROWS: real column n is complex column n
+    if (p.csc) {  // OZ_OUT_ROWS, OZ_OUT_REALZ: real column n is output column n
 #pragma unroll
       for (int j = 0; j < HB; ++j) {
         const int n = n0 + c0 + j;
         if (n < p.N) v[j] *= p.csc[(size_t)b * p.scsc + n].x;
       }
     }
+    if (p.omode == OZ_OUT_REALZ) {  // real result, complex128 storage
+      zd* o = (zd*)p.out + (size_t)b * p.sout;
+      if (m < p.M)
+#pragma unroll
+        for (int j = 0; j < HB; ++j)
+          if (n0 + c0 + j < p.N) {
+            const double x = !upd ? v[j] : (p.osub > 0 ? old[j] - v[j] : old[j] + v[j]);
+            o[m * p.ldr + (n0 + c0 + j) * p.ldc] = zmk(x, 0.0);
+          }
+    } else
     if (p.omode == OZ_OUT_REAL) {
       double* o = (double*)p.out + (size_t)b * p.sout;
-      if (m < p.M)
+      if (p.ldc == 1 && !p.osub && !(p.ldr & 1) && !(p.sout & 1) && n0 + c0 + HB <= p.N) {  // rows: 16-byte stores
+        if (m < p.M) {
+          double2* w = reinterpret_cast<double2*>(o + m * p.ldr + n0 + c0);
+#pragma unroll
+          for (int j = 0; j < HB / 2; ++j) w[j] = make_double2(v[2 * j], v[2 * j + 1]);
+        }
+      } else if (m < p.M)
 #pragma unroll
         for (int j = 0; j < HB; ++j)
           if (n0 + c0 + j < p.N) {
@@ -740,40 +864,50 @@ static inline int oz_tmap(CUtensorMap* m, void* base, int Kpad, long long rows_t
              : 1;
 }
 
-// Digit width and count for a K extent: every diagonal partial sum stays an integer below
-// 2^24 (S pairs at most, each below K (2^b - 1)^2), and S b >= OZ_TARGET_BITS.
-static inline int oz_pick(int Kpad, int* bits, int* S) {
-  for (int b = 7; b >= 4; --b) {
-    const int s = (OZ_TARGET_BITS + b - 1) / b;
-    const double bound = (double)s * Kpad * (double)((1 << b) - 1) * (double)((1 << b) - 1);
-    if (bound < 16777216.0) { *bits = b; *S = s; return 0; }
+// Digit width and count for a K extent: every diagonal partial sum stays an integer of at most
+// 2^24 (S pairs, each at most K 4^(b-1)), and target < S b <= 63.
+static inline int oz_pick(int Kpad, int* bits, int* S, int target = OZ_TARGET_BITS) {
+  for (int b = 8; b >= 4; --b) {
+    const int s = (target + b) / b;
+    const double bound = (double)s * Kpad * (double)(1 << (2 * (b - 1)));
+    if (s * b <= 63 && bound <= 16777216.0) { *bits = b; *S = s; return 0; }
   }
   return 1;
 }
 
-static inline int oz_round(int x, int m) { return (x + m - 1) / m * m; }
+// The words of the epilogue: ND - lg diagonals (an even number) in the high one, |acc| <= 2^24 and
+// lg b <= 40 keep each below 2^62; pair: |acc| (2^b + 1) < 2^31.
+static inline void oz_words(int Kpad, int bits, int S, int nd, int* lg, int* pair) {
+  *lg = (nd + 1) / 2;
+  if ((nd - *lg) & 1) --*lg;
+  *pair = (double)S * Kpad * (double)(1 << (2 * (bits - 1))) * ((1 << bits) + 1) < 2147483648.0;
+}
 
-// Largest L such that sum_D |acc_D| 2^(L - b D) < 2^62 for any inputs (|acc_D| below
-// min(2^24, pairs(D) K (2^b - 1)^2)): the combined integer keeps as many low bits as
-// 64 bits allow.
+// One word: the largest L with sum_D |acc_D| 2^(L - b D) < 2^62.  The low diagonals are cut to its unit,
+// 2^-L of the scales (about 2^-53 of the largest products).  For the mixed form on small grids with
+// K <= 128 alone: the shorter epilogue is on the critical path there (mean Precision Green 7e-11 at N = 64,
+// 4 chains, beta = 4).
 static inline int oz_shift(int Kpad, int b, int S, int nd) {
   double z = 0.0;
   for (int D = 2; D < nd + 2; ++D) {
     const int pairs = std::min(D - 1, std::min(S, 2 * S + 1 - D));
-    const double acc = std::min(16777216.0, (double)pairs * Kpad * (double)((1 << b) - 1) * ((1 << b) - 1));
-    z += std::ldexp(acc, -b * D);
+    z += std::ldexp(std::min(16777216.0, (double)pairs * Kpad * (double)(1 << (2 * (b - 1)))), -b * D);
   }
   return (int)std::floor(62.0 - std::log2(z));
 }
 
-// Tile width and ring depth that fit 227 KB of shared memory; 1 when none does.  A CTA's
-// time is dominated by the latency of streaming its A chunks, so a grid that does not fill
-// the GPU (narrow = 1) takes BN = 16: half the resident B and twice the ring depth.
-static inline int oz_pick_tile(int S, int nkc, int* bn, int* nst, int narrow = 0) {
-  const size_t cap = 232448;
-  const int w0 = narrow ? 16 : 32;
-  for (int w = w0; w >= 16; w -= 16)
-    for (int st = 8; st >= 2; --st)
+static inline int oz_roundup(int x, int m) { return (x + m - 1) / m * m; }
+
+// Tile width and ring depth.  pairs: 16-wide tiles (32-wide where the accumulators of two CTAs fit
+// TMEM) with shared memory for two CTAs per SM; else the widest tile whose accumulators fit TMEM
+// (512 columns), 16 with narrow, with the deepest ring.  1 when none fits.
+static inline int oz_pick_tile(int S, int nkc, int* bn, int* nst, int narrow = 0, int pairs = 0) {
+  const size_t cap = pairs ? 113 * 1024 : 232448;
+  const int tcols = pairs ? 256 : 512;
+  for (int w = narrow ? 16 : 32; w >= 16; w -= 16) {
+    if ((S + 1) * w > tcols) continue;
+    for (int st = 10; st >= 2; --st)
       if (oz_smem_bytes(w, S, nkc, st) <= cap) { *bn = w; *nst = st; return 0; }
+  }
   return 1;
 }

@@ -334,7 +334,7 @@ template <class A>
 static inline void bqr_apply(const BQRApply& ap, dim3 grid, cudaStream_t st) {
   const int rows = ap.N - ap.j0;
   const long long cols = (long long)grid.x * grid.y;
-  if (A::kReal) {
+  if constexpr (A::kReal) {
     // The FP64 instructions per reflector of the busiest sub-partition, for w warps per column:
     // ceil(cols w / 608) warps, each 2 ceil(blocks / w) products, five shuffle additions, w - 1
     // additions over the warps and the factor (one column's registers hold any number of rows).

@@ -194,6 +194,7 @@ template <class A>
 __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
   typedef typename A::Z Z;
   constexpr int KM = UPD_KMAX, LD = UPD_KMAX + 1, NW = UPD_THREADS / 32;
+  constexpr bool FOLD = A::kReal && !A::kDoubleFloat;  // K joins a position's factors (FP64)
   const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int N = p.N, F = p.F, M = p.M, nq = p.nq;
   extern __shared__ __align__(16) unsigned char upd_raw[];
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
   Z* Tc = Gh + 2 * KM * LD;               // [F][KM][KM]
   // per position
   __shared__ Z s_mye[2][KM], s_dlt[2][KM], s_rD[2][KM];
-  __shared__ Z s_myk[2][A::kReal ? KM : 1], s_dlk[2][A::kReal ? KM : 1];  // real: K folded in
+  __shared__ Z s_myk[2][FOLD ? KM : 1], s_dlk[2][FOLD ? KM : 1];  // real FP64: K folded in
   __shared__ int s_psite[KM], s_pvis[KM], s_pkind[KM], s_acc[KM], s_accq[NW][KM];
   __shared__ int s_psite2[KM];      // vector positions: site b, else -1
   __shared__ double s_pc[KM][2];    // vector positions: (c_a, c_b)
@@ -278,8 +279,8 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
         const Z me = A::mk(e[(long long)f * M * 15].myexp[I]), dl = A::mk(e[(long long)f * M * 15].dlt[I]);
         s_mye[f][p0 + I] = me;
         s_dlt[f][p0 + I] = dl;
-        // real: K joins the first flavour's factor of a single position (the last factor of a pair)
-        if (A::kReal && I == w - 1) {
+        // real FP64: K joins the first flavour's factor of a single position (the last factor of a pair)
+        if (FOLD && I == w - 1) {
           s_myk[f][p0 + I] = f == 0 ? A::mul(me, A::mk(K)) : me;
           s_dlk[f][p0 + I] = f == 0 ? A::mul(dl, A::mk(K)) : dl;
         }
@@ -334,17 +335,17 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
         const int vi = s_pvis[v], prop = s_prop[vi];
         zd Rt = zmk(0.0, 0.0);
         // Mat(1,1) = myexp - Delta G(P,P), and for the first position of a pair the 2x2
-        // determinant D_a (myexp_b - Delta_b G'_bb); the real form has K in its last factor
+        // determinant D_a (myexp_b - Delta_b G'_bb); the real FP64 form has K in its last factor
         Z Rm;
         if (kind == 0) {
-          const Z me = A::kReal ? s_myk[fo][v] : s_mye[fo][v], dl = A::kReal ? s_dlk[fo][v] : s_dlt[fo][v];
+          const Z me = FOLD ? s_myk[fo][v] : s_mye[fo][v], dl = FOLD ? s_dlk[fo][v] : s_dlt[fo][v];
           Z g = Gh[(fo * KM + v) * LD + v];
           const Z tq = Tc[(fo * KM + qs) * KM + v], row = Gh[(fo * KM + qs) * LD + v];
           if (acc) g = A::mac(g, tq, row);
           Rm = A::mac(me, A::neg(dl), g);
         } else {
           const int w = v + 1, ra = v + ((lane >> 1) & 1), rb = v + ((lane >> 2) & 1);
-          const Z me = A::kReal ? s_myk[fo][w] : s_mye[fo][w], dl = A::kReal ? s_dlk[fo][w] : s_dlt[fo][w];
+          const Z me = FOLD ? s_myk[fo][w] : s_mye[fo][w], dl = FOLD ? s_dlk[fo][w] : s_dlt[fo][w];
           Z g = Gh[(fo * KM + ra) * LD + rb];
           if (acc) g = A::mac(g, Tc[(fo * KM + q) * KM + ra], Gh[(fo * KM + q) * LD + rb]);
           const Z gvv = A::shfl(g, fo), gwv = A::shfl(g, fo + 2), gvw = A::shfl(g, fo + 4), gww = A::shfl(g, fo + 6);
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
             // non-negative numbers compare like their bits
             double r = A::wide(Rm).x;
             if (F == 2) r *= __shfl_xor_sync(0xffffffffu, r, 1);
+            if (!FOLD) r *= s_K[vi].x;
             if (p.NSUN != 1) {
               double rp = r;
               for (int e = 1; e < p.NSUN; ++e) rp *= r;

@@ -52,8 +52,11 @@ enum {
   ALFGPU_ERROR_SIZE = 105           /* size above a fixed maximum (see alfgpu_decompose_noalloc) */
 };
 
-/* Precision forms.  FP64: complex128 throughout; every product on the FP64 pipes
- * (mma.sync m8n8k4 f64), the per-visit Metropolis chain, QRs, solves and phases in FP64.
+/* Precision forms.  FP64: complex128 throughout; the per-visit Metropolis chain, QRs, solves and
+ * phases in FP64 arithmetic, products on the FP64 pipes (mma.sync m8n8k4 f64) or, where their time
+ * there is longer, as 62-bit digit-sliced products on the BF16 tensor cores, whose error is below the
+ * roundings of an FP64 product (ALFGPU_FLAG_NO_TENSOR_GEMM keeps all of them on the FP64 pipes).
+ * Models whose vertices are all real run the FP64 kernels in real arithmetic.
  * MIXED: G and all state stay complex128.  By default the G wraps through exp(-dtau T),
  * the UDV propagation products and the stabilisation's complex products (CGR's
  * U_R^H U_L and D_R V_R V_L D_L, the products with Q, decompose's R P V) run on the BF16
@@ -96,8 +99,8 @@ enum { ALFGPU_FLAG_DF_STAB_QR = 16, ALFGPU_FLAG_DF_STAB_GEMM = 32, ALFGPU_FLAG_D
  * use the stream path.  ALFGPU_FLAG_NO_GRAPH always uses the stream path. */
 enum { ALFGPU_FLAG_NO_GRAPH = 64 };
 /* Mixed form: the G wraps and delayed-update flushes run as digit-sliced BF16 products on
- * the tensor cores (tcgen05), exact to ~2^-54 like FP64 (N_dim <= 448); this flag selects
- * the double-float GEMMs on the FP32 pipes instead. */
+ * the tensor cores (tcgen05), exact to ~2^-54 like FP64 (N_dim <= 512); this flag selects
+ * the double-float GEMMs on the FP32 pipes instead.  FP64 form: every product on the FP64 pipes. */
 enum { ALFGPU_FLAG_NO_TENSOR_GEMM = 128 };
 /* Mixed form: the complex products inside the stabilisation (CGR's U_R^H U_L and
  * D_R V_R V_L D_L, the products with Q and the pivot permutations, decompose's R P V) run on
@@ -138,9 +141,8 @@ enum { ALFGPU_FLAG_FP64_VISITS = 65536 };
 /* Mixed form: the K = N_dim tensor-core products (G wraps, UDV propagation, stabilisation
  * products) on 16-wide tiles with the deeper A ring of one-chain grids, also on batched grids. */
 enum { ALFGPU_FLAG_OZ_DEEP_RING = 131072 };
-/* Mixed form, grids of several chains: the K = 64 tensor-core products as persistent CTAs, one
- * per SM, each over a contiguous range of output tiles whose A digit slices stay in shared
- * memory from one tile to the next (no overlap of the visits with the flush). */
+/* Mixed form, grids of several chains: accepted, without effect (it selected persistent K = 64 products
+ * that kept their A digit slices from one tile to the next; the paired tiles replaced them). */
 enum { ALFGPU_FLAG_OZ_FLUSH_RESIDENT = 262144 };
 /* The exact pivoted QR applies each step's reflector and forms the next step's partial sums in
  * two passes over the rows (by default one pass does both, the next pivot chosen first). */
@@ -152,10 +154,10 @@ enum { ALFGPU_FLAG_COMPLEX_ARITH = 1048576 };
 
 /* dims.reserved[1] / dims.reserved[2] (mixed form, tensor-core products only): target bits of
  * the digit-sliced products of the G wraps and TAU_M's propagation (reserved[1]) and of the
- * UDV propagation (reserved[2]); 0 keeps the full count (~54 bits, FP64-class).  The digits
- * are b bits wide (b = 7 for N_dim <= 128, 6 up to 448, 5 beyond), so a target rounds up to whole
- * digits; S digits cost (S + 1)(S + 2)/2 - 2 BF16 products per product (53 for S = 9, 43
- * for S = 8) and bound the error by 2^-(b S) of the row / column scales. */
+ * UDV propagation (reserved[2]); 0 keeps the full count (55 bits and a sign, FP64-class).  The digits
+ * are b bits wide (b = 8 for N_dim <= 128, 7 beyond), so a target rounds up to whole
+ * digits; S digits cost (S + 1)(S + 2)/2 - 2 BF16 products per product (43 for S = 8, 34
+ * for S = 7) and bound the error by 2^-(b S - 1) of the row / column scales. */
 enum { ALFGPU_DIMS_WRAP_BITS = 1, ALFGPU_DIMS_PROPAGATE_BITS = 2 };  /* indices into dims.reserved */
 
 typedef struct alfgpu_s alfgpu_t;

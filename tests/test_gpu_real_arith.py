@@ -163,3 +163,29 @@ def test_real_products(chains, L1, L2):
     assert all(np.array_equal(x, y) for x, y in zip(fa, fb))
     assert all(_relmax(x, y) <= 1e-10 for x, y in zip(ga, gb))
     assert np.max(np.abs(pa - pb)) <= 1e-10
+
+
+# the tensor-core products of the FP64 form (62-bit digits): forced on (FLAG_TENSOR_WIDE) against the
+# FP64 pipes (FLAG_NO_TENSOR_GEMM), real and complex, N around the digit widths' and tiles' edges
+# (16, 32, 64, 128), one and several matrices per launch; accept sequences equal, G to 1e-10
+@pytest.mark.parametrize("chains,L1,L2", [(1, 3, 5), (3, 8, 8), (2, 5, 13), (1, 8, 16), (2, 3, 43)])
+@pytest.mark.parametrize("flags", [0, FLAG_COMPLEX_ARITH])
+def test_fp64_tensor_products(chains, L1, L2, flags):
+    from alf_gb300.sweep import FLAG_NO_TENSOR_GEMM, FLAG_TENSOR_WIDE
+    m = mdl.hubbard("square", L1, L2, U=4.0, beta=0.4, dtau=0.1, nwrap=2)
+    u = np.stack([rng.sweep_uniforms(13, c, m.n_op, m.ltrot, 0) for c in range(chains)])
+    out = []
+    for fl in (FLAG_TENSOR_WIDE, FLAG_NO_TENSOR_GEMM):
+        g = Chains(m, n_chains=chains, flags=fl | flags, ltau=1)
+        for c in range(chains):
+            g.set_fields(c, rng.initial_fields(13, c, m.n_op, m.ltrot))
+        g.init_state()
+        g.set_recording(True)
+        _, tau = g.sweep(u, measure=True, keep=lambda k, c, nt: k == 1)
+        out.append(([g.record(c) for c in range(chains)], tau))
+        g.close()
+    for a, b in zip(out[0][0], out[1][0]):
+        assert np.array_equal(a["acc"], b["acc"])
+        assert _relmax(a["G"], b["G"]) <= 1e-10
+    for (c, nt, qa, _), (_, _, qb, _) in zip(out[0][1], out[1][1]):
+        assert all(_relmax(x, y) <= 1e-10 for x, y in zip(qa, qb))
