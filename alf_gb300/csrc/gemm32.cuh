@@ -6,7 +6,7 @@
 // ~2^-44 relative rounding instead of FP32's 2^-24.  On GB300 the FP32 pipes
 // run 64x the FP64 rate (66 vs 1.0 TFLOP/s measured); a double-float
 // multiply-accumulate costs ~14 FP32 operations.  Same operation and options
-// as k_zgemm (gemm.cuh); operands and output may be stored as complex128 or
+// as k_gemm16 (gemm.cuh); operands and output may be stored as complex128 or
 // real64.  The FP32 exponent range (|x| < 3.4e38) suffices for the G wraps and
 // flushes (|G_ij| = O(1), |expT| = O(1)); the graded UDV products stay FP64.
 #pragma once

@@ -183,14 +183,14 @@ def digit_pairs(n: int):
 def roofline(precision: str, chains: int, m, prof):
     """Roofline object of the G-wrap GEMM, the largest consumer of the complex products with a
     clean algorithmic count (2 real x complex N^3 products per flavour per slice, 2 L slices
-    per sweep).  FP64 form: k_zgemm against the measured FP64 MMA rate.  Mixed form:
+    per sweep).  FP64 form: k_gemm16 against the measured FP64 MMA rate.  Mixed form:
     k_oz_slice + k_oz_gemm (digit-sliced BF16 on tcgen05) against the measured BF16 peak; the
     algorithmic count is the same as FP64's, the BF16 products actually executed are
     reported beside it (tensor_op_tflops)."""
     hop_ms, hop_n = prof.get("hop", (0.0, 0))
     flops = algorithmic_flops(m, "hop", hop_n, 0) * chains
     if precision == "fp64":
-        roof = {"bound": "tensor", "kernel": "k_zgemm (G wraps, FP64 mma.sync)", "achieved": None,
+        roof = {"bound": "tensor", "kernel": "k_gemm16 (G wraps, FP64 mma.sync)", "achieved": None,
                 "peak": FP64_DMMA_TFLOPS, "unit": "TFLOP/s", "frac": None,
                 "traffic": HOP_TRAFFIC_BYTES * chains if m.ndim == 256 else None,
                 "algorithmic_flops_per_launch": chains * m.n_fl * 4.0 * m.ndim ** 3,

@@ -189,3 +189,22 @@ def test_fp64_tensor_products(chains, L1, L2, flags):
         assert _relmax(a["G"], b["G"]) <= 1e-10
     for (c, nt, qa, _), (_, _, qb, _) in zip(out[0][1], out[1][1]):
         assert all(_relmax(x, y) <= 1e-10 for x, y in zip(qa, qb))
+
+
+# the complex FP64 products of a model with complex vertices: one and two slices of K, few and many
+# tiles, remainders of 16 and 32: against the oracle
+@pytest.mark.parametrize("chains,L1,L2", [(1, 1, 3), (1, 3, 3), (2, 5, 3), (6, 5, 4), (114, 8, 8)])
+def test_complex_products(chains, L1, L2):
+    from alf_gb300.sweep import FLAG_NO_TENSOR_GEMM
+    m = mdl.kondo(L1, L2, JK=1.5, Uf=2.0, beta=0.4, dtau=0.1, nwrap=2)
+    f0 = rng.initial_fields(15, 0, m.n_op, m.ltrot)
+    u = rng.sweep_uniforms(15, 0, m.n_op, m.ltrot, 0)
+    r, _ = _record(m, FLAG_NO_TENSOR_GEMM, f0, u, chains=chains)
+    o = oracle.Oracle(m)
+    o.set_fields(f0)
+    o.init_state()
+    o.record(1)
+    o.sweep(u)
+    ro = o.recorded()
+    for k in (0, chains - 1):
+        compare_record(r[k], ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=1e-10, relative=True, exact_sequence=True)
