@@ -1303,6 +1303,30 @@ static LattObsParams latt_params(alfgpu_s* h, int kind) {
   return p;
 }
 
+// A cluster of eight CTAs per chain once the kinetic sum has more than a few elements per thread of one
+// (N = 12, two flavours: 288 elements).
+static int launch_obs_scal(alfgpu_s* h, const zd* G) {
+  const long long NN = (long long)h->N * h->N;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  const int CL = NN * h->F > 1024 ? 8 : 1;
+  cfg.gridDim = dim3(CL, h->C, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = h->st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  h->launches++;
+  const zd* ph = h->phase;
+  const double *HT = h->obs_HT, *tr = h->obs_trH, *U = h->obs_U;
+  if (real_model(h))
+    CK(cudaLaunchKernelEx(&cfg, k_obs_scal<true>, G, ph, HT, tr, U, h->N, h->F, (int)h->obs_nsun, h->obs_acc));
+  else
+    CK(cudaLaunchKernelEx(&cfg, k_obs_scal<false>, G, ph, HT, tr, U, h->N, h->F, (int)h->obs_nsun, h->obs_acc));
+  return 0;
+}
+
 static int obs_eq(alfgpu_s* h, alfgpu_obs_cb cb, void* ctx, int ntau1, int pending) {
   if (!cb && !h->obs_scal && !h->obs_latt) return 0;
   const long long NN = (long long)h->N * h->N;
@@ -1318,13 +1342,12 @@ static int obs_eq(alfgpu_s* h, alfgpu_obs_cb cb, void* ctx, int ntau1, int pendi
     src = h->Gw;
   }
   if (h->obs_scal) {
-    k_obs_scal<<<h->C, 256, 0, h->st>>>(src, h->phase, h->obs_HT, h->obs_trH, h->obs_U, h->N, h->F, h->obs_nsun,
-                                        h->obs_acc);
-    CKL();
+    RET(launch_obs_scal(h, src));
   }
   if (h->obs_latt) {
-    const int nout = h->lo_ncell * h->lo_norb * h->lo_norb;
-    k_obs_latt_eq<<<dim3((nout + 127) / 128, h->C), 128, 0, h->st>>>(src, latt_params(h, 0));
+    const dim3 grid(h->lo_ncell * h->lo_norb * h->lo_norb + h->lo_norb, h->C);
+    if (real_model(h)) k_obs_latt_eq<ArRe><<<grid, 128, 0, h->st>>>(src, latt_params(h, 0));
+    else k_obs_latt_eq<ArD><<<grid, 128, 0, h->st>>>(src, latt_params(h, 0));
     CKL();
   }
   if (!cb) return 0;
@@ -1346,8 +1369,9 @@ static int obs_tau(alfgpu_s* h, alfgpu_obs_cb cb, void* ctx, int nt) {
   CKL();
   RET(rotate_out(h, h->Gq, 4 * h->B));
   if (h->obs_latt) {
-    const int nout = h->lo_ncell * h->lo_norb * h->lo_norb;
-    k_obs_latt_tau<<<dim3((nout + 127) / 128, h->C), 128, 0, h->st>>>(h->Gq, nt, latt_params(h, 1));
+    const dim3 lgrid(h->lo_ncell * h->lo_norb * h->lo_norb + h->lo_norb, h->C);
+    if (real_model(h)) k_obs_latt_tau<ArRe><<<lgrid, 128, 0, h->st>>>(h->Gq, nt, latt_params(h, 1));
+    else k_obs_latt_tau<ArD><<<lgrid, 128, 0, h->st>>>(h->Gq, nt, latt_params(h, 1));
     CKL();
   }
   if (!cb) return 0;

@@ -265,51 +265,69 @@ __global__ void k_rot_cols(zd* G, int N, const int* pairs, int npairs, double u0
 //   Part = N_SUN sum_f sum_i GRC_f(i,i),  Ener = Kin + Pot
 // acc[c] += {ZP ZS Kin, ZP ZS Pot, ZP ZS Part, ZP ZS Ener} (complex), ZS, 1.
 // HT holds H_f transposed (HT_f[j + i N] = H_f(i,j)), so sum_ij H(i,j) G(j,i) is the
-// elementwise sum over the two column-major arrays.  One CTA (256 threads) per chain, fixed
-// summation order.
+// elementwise sum over the two column-major arrays.  A cluster of CTAs (256 threads) per chain, each
+// with its stretch of the elements and sites, the partial sums added in a fixed order.  The FP64 pipe
+// bounds it: the kinetic sum is F N^2 multiply-adds (twice that in complex arithmetic) at 32 per 64
+// cycles and sub-partition.  N = 64, four chains: one CTA per chain, complex, 19.6 us; this 10.9 us, most
+// of it the latency of the final weights.
+template <bool RE>
 __global__ void __launch_bounds__(256) k_obs_scal(const zd* G, const zd* phase, const double* HT, const double* trH,
                                                   const double* U, int N, int F, int nsun, double* acc) {
-  const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ncl = gridDim.x, rank = blockIdx.x;  // one cluster per chain
   const long long NN = (long long)N * N;
   double kr = 0.0, ki = 0.0, pr = 0.0, pi = 0.0;
   for (int f = 0; f < F; ++f) {
     const zd* g = G + ((long long)c * F + f) * NN;
     const double* ht = HT + (long long)f * NN;
-    for (long long e = tid; e < NN; e += 256) {
+    for (long long e = rank * 256 + tid; e < NN; e += 256 * ncl) {
       const zd v = g[e];
       kr = fma(ht[e], v.x, kr);
-      ki = fma(ht[e], v.y, ki);
+      if (!RE) ki = fma(ht[e], v.y, ki);
     }
   }
   // Pot and Part need the diagonals of both flavours at the same site
   double rr = 0.0, ri = 0.0;
-  for (int i = tid; i < N; i += 256) {
+  for (int i = rank * 256 + tid; i < N; i += 256 * ncl) {
     const zd g1 = G[((long long)c * F) * NN + i + (long long)i * N];
-    const zd a = zmk(1.0 - g1.x, -g1.y);  // GRC_1(i,i)
+    const zd a = zmk(1.0 - g1.x, RE ? 0.0 : -g1.y);  // GRC_1(i,i)
     zd b = a;
     if (F == 2) {
       const zd g2 = G[((long long)c * F + 1) * NN + i + (long long)i * N];
-      b = zmk(1.0 - g2.x, -g2.y);
-      rr += b.x; ri += b.y;
+      b = zmk(1.0 - g2.x, RE ? 0.0 : -g2.y);
+      rr += b.x;
+      if (!RE) ri += b.y;
     }
-    rr += a.x; ri += a.y;
-    const zd ab = zmul(a, b);
+    rr += a.x;
+    if (!RE) ri += a.y;
+    const zd ab = RE ? zmk(a.x * b.x, 0.0) : zmul(a, b);
     pr = fma(U[i], ab.x, pr);
-    pi = fma(U[i], ab.y, pi);
+    if (!RE) pi = fma(U[i], ab.y, pi);
   }
   double v[6] = {kr, ki, pr, pi, rr, ri};
 #pragma unroll
-  for (int q = 0; q < 6; ++q) v[q] = warp_sum(v[q]);
-  __shared__ double wsum[6][8];
+  for (int q = 0; q < 6; ++q)
+    if (!RE || q % 2 == 0) v[q] = warp_sum(v[q]);
+  __shared__ double wsum[6][8], csum[6];
   if (lane == 0)
     for (int q = 0; q < 6; ++q) wsum[q][warp] = v[q];
   __syncthreads();
-  if (tid == 0) {
+  double sq = 0.0;  // thread q < 6: total of v[q] over this CTA, then over the cluster
+  if (tid < 6) {
+    for (int w = 0; w < 8; ++w) sq += wsum[tid][w];
+    csum[tid] = sq;
+  }
+  if (ncl > 1) {
+    cluster_sync();
+    if (rank == 0 && tid < 6)
+      for (int r = 1; r < ncl; ++r) sq += dsmem_ld_f64(dsmem_addr(&csum[tid], r));
+    cluster_sync();  // no CTA leaves while its sums may still be read
+  }
+  if (rank == 0 && warp == 0) {
     double s[6];
-    for (int q = 0; q < 6; ++q) {
-      s[q] = 0.0;
-      for (int w = 0; w < 8; ++w) s[q] += wsum[q][w];
-    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q) s[q] = __shfl_sync(0xffffffffu, sq, q);
+    if (tid != 0) return;
     double trh = 0.0;
     for (int f = 0; f < F; ++f) trh += trH[f];
     const zd kin = zmk(nsun * (trh - s[0]), -nsun * s[1]);
