@@ -373,12 +373,12 @@ static int qrr_plan(int N, int CL, int B, int flags, int dev, int* CLout) {
 // N x N, 0 where it is not used: the columns do not fit, or (complex) the clusters of a batched
 // launch need a second wave, where k_qrp_rows' global rows win (32 matrices, N = 256: 5.7 ms
 // against 6.7 ms).  Measured (ms, one QR, real unless said otherwise):
-//   2 matrices   N = 64: CL 4 0.200, 8 0.199;  144: 4 0.574, 8 0.513, 16 0.574;  256: 8 1.19, 16 1.17;
-//                288: 8 1.53, 16 1.40;  complex 256: 8 2.68, 16 2.23
-//   8 matrices   144: 8 0.512, 16 0.619;  256: 8 1.19, 16 1.33;  288: 8 1.53, 16 1.61
-//   32 matrices  144: 4 0.577, 8 0.626;  196: 8 1.05, 16 1.58;  256: 8 1.64, 16 2.23
-// so: eight CTAs, sixteen for a few large matrices, four where eight would need more CTAs than
-// SMs and four hold the work (N <= 160), fewer for small N.
+//   2 matrices   N = 36: CL 2 0.098, 4 0.096;  64: 4 0.170, 8 0.167;  144: 4 0.481, 8 0.418, 16 0.393;
+//                196: 8 0.672, 16 0.592;  256: 8 1.01, 16 0.82;  complex 256: 8 2.45, 16 1.67
+//   8 matrices   144: 8 0.417, 16 0.414;  196: 8 0.671, 16 0.729;  256: 8 1.01, 16 0.99
+//   32 matrices  144: 4 0.481, 8 0.481;  196: 8 0.861, 16 1.06;  256: 8 1.40, 16 1.50
+// so: eight CTAs, sixteen for a few matrices that are not small, four where eight would need more CTAs
+// than SMs and four hold the work (N <= 160), fewer for small N.
 static int qrc_plan(int N, int B, int real, int flags, int dev) {
   if (flags & (ALFGPU_FLAG_QR_GLOBAL_ROWS | ALFGPU_FLAG_QR_HALF_CLUSTER | ALFGPU_FLAG_QR_FULL_CLUSTER |
                ALFGPU_FLAG_QR_TWO_PASS))
@@ -388,7 +388,7 @@ static int qrc_plan(int N, int B, int real, int flags, int dev) {
   const int zb = real ? 8 : 16;
   int cl = N >= 96 ? 8 : (N >= 32 ? 4 : (N >= 16 ? 2 : 1));
   if (cl == 8 && N <= 160 && 8 * B > nsm) cl = 4;
-  if (N > 224 && 16 * B <= nsm / 2) cl = 16;
+  if (N >= 128 && 16 * B <= nsm / 2) cl = 16;
   for (; cl <= 16; cl *= 2) {
     const size_t sm = qrc_smem_bytes(N, cl, zb);
     if (sm > 227 * 1024) continue;
@@ -425,7 +425,7 @@ static int launch_qrc(alfgpu_s* h, const zd* Ain, zd* A, int N, int CL, int real
   memset(&q, 0, sizeof(q));
   q.Ain = Ain; q.A = A; q.lda = N; q.sA = NN; q.N = N;
   q.colscale = colscale; q.sCS = N;
-  q.tau = tau; q.sT = N; q.jpvt = jpvt; q.sP = N; q.D = D; q.sD = N; q.info = info;
+  q.tau = tau; q.sT = N; q.jpvt = jpvt; q.sP = N; q.D = D; q.sD = N; q.info = info; q.err = h->err;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(CL, h->B, 1);

@@ -72,6 +72,24 @@ def test_decompose_sizes(N, side):
     assert np.max(np.abs(U.conj().T @ U - np.eye(N))) < 1e-12
 
 
+# reflectors that are the identity, and norms that tie (the first column wins): the oracle's pivots,
+# so the same factors
+@pytest.mark.parametrize("N", [2, 17, 40, 130])
+@pytest.mark.parametrize("kind", ["identity", "permutation", "upper"])
+def test_decompose_ties(N, kind):
+    X = np.eye(N, dtype=complex)
+    if kind == "permutation":
+        X = X[np.random.default_rng(N).permutation(N)]
+    if kind == "upper":  # columns of equal norm, all of whose reflectors are trivial
+        X = np.triu(np.ones((N, N)), 0) / np.sqrt(np.arange(1, N + 1))[None, :] * (1.0 + 0j)
+    one, V = np.ones(N, dtype=complex), np.eye(N, dtype=complex)
+    U, d, W = gpu_decompose("r", X.copy(), one, V)
+    Uo, do, Wo = oracle.decompose("r", X.copy(), one, V)
+    assert _relmax(U @ np.diag(d) @ W, X) < 1e-12
+    if kind != "upper":  # norms equal to the last bit
+        assert np.max(np.abs(U - Uo)) < 1e-14 and np.max(np.abs(W - Wo)) < 1e-14
+
+
 # right-hand sides per CTA (2, 4, 8), row blocks of 32 and their remainders, both solve
 # directions, complex factors
 @pytest.mark.parametrize("N", [1, 5, 31, 32, 33, 64, 100, 257, 320])
