@@ -20,6 +20,7 @@
 #include "gemm32.cuh"
 #include "qr_blocked.cuh"
 #include "qr_cols.cuh"
+#include "q_apply.cuh"
 #include "kernels_misc.cuh"
 #include "linalg.cuh"
 #include "update.cuh"
@@ -932,18 +933,72 @@ static int orgqr_wy(alfgpu_s* h, const zd* F, zd* Q) {
   return 0;
 }
 
+// FP64 instructions per reflector on the busiest sub-partition: a warp per cw columns (k_q_apply), and
+// four warps per column (k_bqr_apply), which complex columns want while few of them leave sub-partitions idle.
+template <class A>
+static long long q_apply_cost(long long cols, int blocks, int cw) {
+  constexpr int c = A::kReal ? 1 : 4, a = A::kReal ? 1 : 2;
+  if (cw == 0) return ((cols * 4 + 607) / 608) * (2 * c * ((blocks + 3) / 4) + 9 * a + c) + 12;  // a barrier, tau
+  const int red = cw * a >= 4 ? 6 : 5;
+  return ((cols + cw * 608 - 1) / (cw * 608)) * (2ll * c * blocks * cw + (A::kReal ? red : red + (cw == 1)) + c);
+}
+template <class A, int QW, int CW>
+static int q_apply_launch(alfgpu_s* h, const QApplyParams& p, size_t sm) {
+  // four warps per CTA while several CTAs share an SM or all of them run at once, else eight
+  const int warps = (p.N + 4 * CW - 1) / (4 * CW) * (long long)h->B <= 152 || sm <= 76 * 1024 ? 4 : 8;
+  CK(raise_smem_limit(k_q_apply<A, QW, CW>, sm));
+  k_q_apply<A, QW, CW><<<dim3((p.N + warps * CW - 1) / (warps * CW), h->B), 32 * warps, sm, h->st>>>(p);
+  CKL();
+  return 0;
+}
+// Q of the factored n x n matrices F applied to C, or formed in C (init), in one launch; *done = 0 where
+// the panels do not fit in shared memory or four warps per column are faster.
+template <class A>
+static int q_apply(alfgpu_s* h, const zd* F, const zd* tau, zd* C, int n, int init, int* done) {
+  const long long nn = (long long)n * n, cols = (long long)n * h->B;
+  const int blocks = (n + 31) / 32;
+  const size_t sm = qap_smem_bytes(n, (int)sizeof(typename A::Z));
+  *done = 0;
+  if (blocks > (A::kReal ? 24 : 14) || sm > 220 * 1024) return 0;
+  int cw = 1;
+  for (int w = 2; w <= (blocks <= 12 ? 4 : 2) && w <= (A::kReal ? 4 : 2); w *= 2)
+    if (q_apply_cost<A>(cols, blocks, w) < q_apply_cost<A>(cols, blocks, cw)) cw = w;
+  if (!A::kReal && blocks > 8) cw = 1;
+  if (q_apply_cost<A>(cols, blocks, 0) < q_apply_cost<A>(cols, blocks, cw)) return 0;
+  QApplyParams p;
+  p.V = F; p.ldv = n; p.sV = nn; p.tau = tau; p.sT = n;
+  p.C = C; p.ldc = n; p.sC = nn; p.N = n; p.init = init;
+  *done = 1;
+  if constexpr (A::kReal) {
+    if (blocks <= 8) return cw == 4 ? q_apply_launch<A, 8, 4>(h, p, sm) : (cw == 2 ? q_apply_launch<A, 8, 2>(h, p, sm) : q_apply_launch<A, 8, 1>(h, p, sm));
+    if (blocks <= 12) return cw == 4 ? q_apply_launch<A, 12, 4>(h, p, sm) : (cw == 2 ? q_apply_launch<A, 12, 2>(h, p, sm) : q_apply_launch<A, 12, 1>(h, p, sm));
+    return cw == 2 ? q_apply_launch<A, 24, 2>(h, p, sm) : q_apply_launch<A, 24, 1>(h, p, sm);
+  } else {
+    if (blocks <= 8) return cw == 2 ? q_apply_launch<A, 8, 2>(h, p, sm) : q_apply_launch<A, 8, 1>(h, p, sm);
+    return q_apply_launch<A, 14, 1>(h, p, sm);
+  }
+}
+
 static int orgqr_any(alfgpu_s* h, const zd* F, zd* Q) {
   const int N = h->N, B = h->B;
   const long long NN = (long long)N * N;
   // compact WY pays on batched grids of complex matrices; one chain's grid is too small for its
   // launch chain, and real columns take a quarter of the FP64 instructions (16 chains, N = 256,
-  // per sweep: compact WY 110 ms, real columns 70 ms)
+  // per sweep: compact WY 110 ms, real columns 49 ms)
   if (h->mixed && h->oz_stab && !h->oz_narrow && !h->qr_df && !real_model(h) && N <= 32 * BQR_LROWS) return orgqr_wy(h, F, Q);
   if (N > 32 * BQR_LROWS) {  // beyond the rows a lane of k_bqr_apply holds
     RET(copy_mats(h, Q, F, (size_t)B * NN));
     return launch_orgqr(h, Q, B);
   }
   prof_begin(h, ALFGPU_PROF_ORGQR);
+  if (!h->qr_df) {
+    int done = 0;
+    RET(real_model(h) ? q_apply<ArRe>(h, F, h->tau, Q, N, 1, &done) : q_apply<ArD>(h, F, h->tau, Q, N, 1, &done));
+    if (done) {
+      prof_end(h);
+      return 0;
+    }
+  }
   for (int j0 = ((N - 1) / BQR_NB) * BQR_NB; j0 >= 0; j0 -= BQR_NB) {
     const int w = (N - j0 < BQR_NB) ? N - j0 : BQR_NB;
     BQRApply ap;
@@ -1414,6 +1469,9 @@ static int qrp_n(alfgpu_s* h, zd* A, int N2, zd* tau, int* jpvt, double* D, doub
 // Q C for the reflectors of the factored N2 x N2 matrix F (ZUNMQR 'L','N'), all columns of C.
 static int unmqr_n(alfgpu_s* h, const zd* F, const zd* tau, zd* Cm, int N2) {
   const long long NN2 = (long long)N2 * N2;
+  int done = 0;
+  RET(real_model(h) ? q_apply<ArRe>(h, F, tau, Cm, N2, 0, &done) : q_apply<ArD>(h, F, tau, Cm, N2, 0, &done));
+  if (done) return 0;
   for (int j0 = ((N2 - 1) / BQR_NB) * BQR_NB; j0 >= 0; j0 -= BQR_NB) {
     const int w = (N2 - j0 < BQR_NB) ? N2 - j0 : BQR_NB;
     BQRApply ap;

@@ -89,6 +89,26 @@ ALF_DEV double warp_max(double v) {
 }
 ALF_DEV zd warp_zsum(zd v) { return zmk(warp_sum(v.x), warp_sum(v.y)); }
 
+// Sum over the warp of M values (a power of two <= 32): lane l returns the total of v[l / (32 / M)].
+template <int M>
+ALF_DEV double warp_sum_packed(double (&v)[M]) {
+  const int lane = threadIdx.x & 31;
+  int off = 16;
+#pragma unroll
+  for (int m = M / 2; m > 0; m >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int q = 0; q < m; ++q) {
+      const double keep = up ? v[q + m] : v[q], send = up ? v[q] : v[q + m];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  double s = v[0];
+#pragma unroll
+  for (int o = 16 / M; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // Counter-based uniform stream shared with the oracle's harness:
 // u = (splitmix64(key(seed, chain) + (counter+1)*golden) >> 11) * 2^-53.
 ALF_HD uint64_t alf_mix64(uint64_t z) {

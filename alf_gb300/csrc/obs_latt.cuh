@@ -36,26 +36,6 @@ ALF_DEV zd lobs_weight(zd ph, double* zs) {
   return zmk(ph.x / ph.x * s, ph.y / ph.x * s);  // (Phase / Re Phase) ZS
 }
 
-// Sum over the warp of M values (a power of two <= 32): lane l returns the total of v[l / (32 / M)].
-template <int M>
-ALF_DEV double lobs_warp_sum(double (&v)[M]) {
-  const int lane = threadIdx.x & 31;
-  int off = 16;
-#pragma unroll
-  for (int m = M / 2; m > 0; m >>= 1, off >>= 1) {
-    const bool up = lane & off;
-#pragma unroll
-    for (int q = 0; q < m; ++q) {
-      const double keep = up ? v[q + m] : v[q], send = up ? v[q] : v[q + m];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  double s = v[0];
-#pragma unroll
-  for (int o = 16 / M; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
-
 // Totals of NV values over the CTA's 128 threads, known to the threads of warp 0 when it returns.
 template <class A, int NV>
 ALF_DEV void lobs_cta_sum(typename A::Z (&v)[NV]) {
@@ -70,7 +50,7 @@ ALF_DEV void lobs_cta_sum(typename A::Z (&v)[NV]) {
     x[q * P] = A::re(v[q]);
     if (P == 2) x[q * P + P - 1] = A::im(v[q]);
   }
-  const double s = lobs_warp_sum<M>(x);
+  const double s = warp_sum_packed<M>(x);
   if (lane % (32 / M) == 0) red[warp][lane / (32 / M)] = s;
   __syncthreads();
   if (warp != 0) return;

@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(32 * WPC) k_bqr_apply(BQRApply p) {
       vn[q] = (r < kc || r >= N) ? A::zero() : (r == kc ? A::one() : A::ld(v[r]));
     }
   };
+  const zd tl = lane < nb ? tau[j0 + lane] : zmk(0.0, 0.0);  // lane k: tau of reflector k
   load_v(p.conj_tau ? 0 : nb - 1);
   int par = 0;  // parity of the reduction buffer: flips once per barrier
   for (int kk = 0; kk < nb; ++kk) {
@@ -291,8 +292,8 @@ __global__ void __launch_bounds__(32 * WPC) k_bqr_apply(BQRApply p) {
 #pragma unroll
     for (int q = 0; q < BQR_QW; ++q) vr[q] = vn[q];
     if (kk + 1 < nb) load_v(p.conj_tau ? kk + 1 : nb - 2 - kk);
-    zd t = tau[kc];
-    if (t.x == 0.0 && t.y == 0.0) continue;  // uniform over the block
+    zd t = zmk(__shfl_sync(0xffffffffu, tl.x, k), __shfl_sync(0xffffffffu, tl.y, k));
+    if (((__double_as_longlong(t.x) | __double_as_longlong(t.y)) << 1) == 0) continue;  // uniform over the block
     if (p.conj_tau) t.y = -t.y;
     Z s = A::zero();
 #pragma unroll

@@ -226,3 +226,10 @@ def test_complex_products(chains, L1, L2):
     ro = o.recorded()
     for k in (0, chains - 1):
         compare_record(r[k], ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=1e-10, relative=True, exact_sequence=True)
+
+
+# Q over all panels in one launch: 9 and 13 row blocks per column (12 and 24 held by a lane), one and
+# several columns per warp, an explicit Q and CGR2_2's application to general columns; against the complex products
+@pytest.mark.parametrize("chains,L1,L2", [(1, 13, 10), (1, 20, 10), (6, 13, 10)])
+def test_real_q_of_large_systems(chains, L1, L2):
+    test_real_tau_matches_complex_products(chains, L1, L2)
