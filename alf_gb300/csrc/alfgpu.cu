@@ -151,6 +151,8 @@ struct alfgpu_s {
   // families of disjoint bonds; replaces the dense hopping products
   int cb = 0, cb_ncheck = 0;
   std::vector<int> cb_fam;
+  int* cb_famd = nullptr;  // the same on the device, cb_nfamd entries
+  int cb_nfamd = 0;
   int* cb_P = nullptr;
   double *cb_mat = nullptr, *cb_inv = nullptr;
   std::vector<double> h_expT, h_expTinv;      // hopping exponentials as uploaded (original basis)
@@ -1103,34 +1105,35 @@ static int vtx_right_inv(alfgpu_s* h, zd* X, int nt1) {
 }
 
 // Checkerboard hopping on the B matrices X (Hop_mod.F90:143-250 with the bond operators in Op_T
-// order): each family's disjoint bonds in one launch, families in the order of the routine.
+// order): each family's disjoint bonds, families in the order of the routine, and the slice's vertex
+// scalings before or after them in the same launch.
 enum { CB_MMTHR, CB_MMTHR_M1, CB_MMTHL, CB_MMTHL_M1, CB_MMTHLC };
-static int cb_apply(alfgpu_s* h, zd* X, int which) {
+template <class A>
+static int cb_launch(alfgpu_s* h, zd* X, bool rows, bool inv, bool reverse, const BondScale& sc) {
+  const int N = h->N;
+  int T = 1;  // columns (rows) per CTA: the most, up to eight, that leave no SM without one
+  while (T < 8 && (long long)((N + 2 * T - 1) / (2 * T)) * h->B >= 152) T *= 2;
+  const int th = std::min(256, std::max(32, (N / 2 * T + 31) / 32 * 32));
+  while (T > 1 && (size_t)T * N * sizeof(typename A::Z) > 200 * 1024) T /= 2;
+  const size_t sm = (size_t)T * N * sizeof(typename A::Z);
+  const dim3 grid((N + T - 1) / T, h->B);
+  const double* E = inv ? h->cb_inv : h->cb_mat;
   const int nfam = (int)h->cb_fam.size() - 1;
+  if (rows) {
+    CK(raise_smem_limit(k_bonds<A, true>, sm));
+    k_bonds<A, true><<<grid, th, sm, h->st>>>(X, N, h->F, h->cb_P, E, h->cb_ncheck, h->cb_famd, nfam, reverse, T, sc);
+  } else {
+    CK(raise_smem_limit(k_bonds<A, false>, sm));
+    k_bonds<A, false><<<grid, th, sm, h->st>>>(X, N, h->F, h->cb_P, E, h->cb_ncheck, h->cb_famd, nfam, reverse, T, sc);
+  }
+  CKL();
+  return 0;
+}
+static int cb_apply(alfgpu_s* h, zd* X, int which, const BondScale& sc = BondScale()) {
   const bool rows = which == CB_MMTHR || which == CB_MMTHR_M1 || which == CB_MMTHLC;
   const bool inv = which == CB_MMTHR_M1 || which == CB_MMTHL_M1;
   const bool reverse = which == CB_MMTHR || which == CB_MMTHL_M1;  // the last family first
-  const long long NN = (long long)h->N * h->N;
-  for (int q = 0; q < nfam; ++q) {
-    const int fm = reverse ? nfam - 1 - q : q;
-    const int b0 = h->cb_fam[fm], b1 = h->cb_fam[fm + 1];
-    if (b1 <= b0) continue;
-    const dim3 grid((unsigned)(((long long)h->N * (b1 - b0) + 255) / 256), h->B);
-    if (rows)
-      k_bond_rows<<<grid, 256, 0, h->st>>>(X, NN, h->N, h->F, h->cb_P, inv ? h->cb_inv : h->cb_mat, h->cb_ncheck, b0,
-                                           b1);
-    else
-      k_bond_cols<<<grid, 256, 0, h->st>>>(X, NN, h->N, h->F, h->cb_P, inv ? h->cb_inv : h->cb_mat, h->cb_ncheck, b0,
-                                           b1);
-    CKL();
-  }
-  return 0;
-}
-static int scale_rc(alfgpu_s* h, zd* X, const zd* rs, int rconj, const zd* cs) {
-  const dim3 grid((unsigned)(((long long)h->N * h->N + 255) / 256), h->B);
-  k_scale_rc<<<grid, 256, 0, h->st>>>(X, h->N, rs, rconj, cs);
-  CKL();
-  return 0;
+  return real_model(h) ? cb_launch<ArRe>(h, X, rows, inv, reverse, sc) : cb_launch<ArD>(h, X, rows, inv, reverse, sc);
 }
 
 // WRAPUR (wrapur_mod.F90:101-124): U <- prod_nt [D_nt expT] U, then decompose (side R)
@@ -1139,13 +1142,13 @@ static int wrapur_u(alfgpu_s* h, UDVSet& u, int ntau, int ntau1) {
   prof_begin(h, ALFGPU_PROF_PROPAGATE);
   for (int nt = ntau + 1; nt <= ntau1; ++nt) {
     if (h->cb) {  // U <- P (B_T U) with the bond operators (Hop_mod_mmthr), then the vertices
-      RET(cb_apply(h, u.U, CB_MMTHR));
-      if (h->pairblock) {
-        RET(vtx_left(h, u.U, nt));
-      } else {
+      BondScale sc;
+      if (!h->pairblock) {
         RET(slice_scale(h, nt));
-        RET(scale_rc(h, u.U, h->S, 0, nullptr));
+        sc.rs1 = h->S;
       }
+      RET(cb_apply(h, u.U, CB_MMTHR, sc));
+      if (h->pairblock) RET(vtx_left(h, u.U, nt));
       continue;
     }
     if (h->pairblock) {  // U <- P (expT U): the product, then the slice's explicit vertex phases
@@ -1185,13 +1188,14 @@ static int wrapul(alfgpu_s* h, int ntau1, int ntau) {
   prof_begin(h, ALFGPU_PROF_PROPAGATE);
   for (int nt = ntau1; nt >= ntau + 1; --nt) {
     if (h->cb) {  // U <- B_T^T (P^dagger U): the vertices, then the bonds (Hop_mod_mmthlc)
+      BondScale sc;
       if (h->pairblock) {
         RET(vtx_left_adj(h, h->udvl.U, nt));
       } else {
         RET(slice_scale(h, nt));
-        RET(scale_rc(h, h->udvl.U, h->S, 1, nullptr));
+        sc.rs0 = h->S; sc.conj0 = 1;
       }
-      RET(cb_apply(h, h->udvl.U, CB_MMTHLC));
+      RET(cb_apply(h, h->udvl.U, CB_MMTHLC, sc));
       continue;
     }
     if (h->pairblock) {  // U <- expT (P^dagger U): the slice's explicit vertex phases, then the product
@@ -1594,14 +1598,16 @@ static int tau_m(alfgpu_s* h, alfgpu_obs_cb cb, void* ctx) {
       zd* Xs[3] = {h->GT0, h->G0T, h->GTT};
       for (int k = 0; k < 3; ++k) {
         if (k >= 1) {  // PROPRM1 (G0T, then the first half of GTT)
-          RET(cb_apply(h, Xs[k], CB_MMTHL_M1));
+          BondScale sc;
+          if (!pb) sc.cs1 = h->Sinv;
+          RET(cb_apply(h, Xs[k], CB_MMTHL_M1, sc));
           if (pb) RET(vtx_right_inv(h, Xs[k], NT1));
-          else RET(scale_rc(h, Xs[k], nullptr, 0, h->Sinv));
         }
         if (k != 1) {  // PROPR (GT0, then the second half of GTT)
-          RET(cb_apply(h, Xs[k], CB_MMTHR));
+          BondScale sc;
+          if (!pb) sc.rs1 = h->S;
+          RET(cb_apply(h, Xs[k], CB_MMTHR, sc));
           if (pb) RET(vtx_left(h, Xs[k], NT1));
-          else RET(scale_rc(h, Xs[k], h->S, 0, nullptr));
         }
       }
     } else if (oz_tau(h)) {
@@ -1675,8 +1681,9 @@ static int hop(alfgpu_s* h, int up, int with_scale) {
 static int hop_impl(alfgpu_s* h, int up, int with_scale) {
   const int N = h->N, F = h->F, B = h->B;
   if (h->cb) {  // WRAPGRUP: mmthr, mmthl_m1; WRAPGRDO: mmthl, mmthr_m1 (bond passes, both forms)
-    if (with_scale) RET(scale_rc(h, h->G, up ? h->S : h->Sinv, 0, up ? h->Sinv : h->S));
-    RET(cb_apply(h, h->G, up ? CB_MMTHR : CB_MMTHL));
+    BondScale sc;
+    if (with_scale) { sc.rs0 = up ? h->S : h->Sinv; sc.cs0 = up ? h->Sinv : h->S; }
+    RET(cb_apply(h, h->G, up ? CB_MMTHR : CB_MMTHL, sc));
     return cb_apply(h, h->G, up ? CB_MMTHL_M1 : CB_MMTHR_M1);
   }
   if (h->oz && !(with_scale && h->eexp_complex) && oz_pays(h, N, N, 2, OZ_MIN_US)) {
@@ -3274,6 +3281,11 @@ int alfgpu_upload_checkerboard(alfgpu_t* h, int32_t ncheck, int32_t nfam, const 
     r |= dalloc(h, &h->cb_mat, 4ull * F * ncheck); r |= dalloc(h, &h->cb_inv, 4ull * F * ncheck);
     if (r) return ALFGPU_ERROR_CUDA;
   }
+  if (nfam + 1 > h->cb_nfamd) {
+    if (dalloc(h, &h->cb_famd, nfam + 1)) return ALFGPU_ERROR_CUDA;
+    h->cb_nfamd = nfam + 1;
+  }
+  CK(cudaMemcpy(h->cb_famd, fam, (nfam + 1) * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->cb_P, P, 2ull * F * ncheck * sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->cb_mat, mat, 4ull * F * ncheck * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->cb_inv, inv, 4ull * F * ncheck * sizeof(double), cudaMemcpyHostToDevice));

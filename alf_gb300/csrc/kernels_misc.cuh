@@ -434,49 +434,71 @@ __global__ void k_copy_fields(const int8_t* fields, int L, int M, int nt1, int8_
     out[(long long)c * M + n] = fields[(long long)c * L * M + (long long)(nt1 - 1) * M + n];
 }
 
-// ---- checkerboard hopping: bond operators of one family ------------------------------------
-// Bonds [b0, b1) of a family are disjoint two-site operators (P [F][ncheck][2], E [F][ncheck][4]
+// ---- checkerboard hopping: bond operators --------------------------------------------------
+// The bonds [fam[q], fam[q + 1]) of a family are disjoint two-site operators (P [F][ncheck][2], E [F][ncheck][4]
 // real, column-major 2 x 2); batch entry b uses flavour b % F.  The RealExpOpT lmult / rmult of
-// each bond (Prog/OpTTypes_mod.F90:135-304): rows (X <- E X) or columns (X <- X E).
-// grid (ceil(N (b1 - b0) / 256), B)
-__global__ void k_bond_rows(zd* X, long long sX, int N, int F, const int* P, const double* E, int ncheck, int b0,
-                            int b1) {
-  const int b = blockIdx.y, f = b % F;
-  const long long e = blockIdx.x * 256ll + threadIdx.x;
-  if (e >= (long long)N * (b1 - b0)) return;
-  const int j = (int)(e % N), nc = b0 + (int)(e / N);
-  const long long k = (long long)f * ncheck + nc;
-  const int a = P[2 * k], c = P[2 * k + 1];
-  const double* m = E + 4 * k;
-  zd* col = X + b * sX + (long long)j * N;
-  const zd xa = col[a], xc = col[c];
-  col[a] = zadd(zscale(xa, m[0]), zscale(xc, m[2]));
-  col[c] = zadd(zscale(xa, m[1]), zscale(xc, m[3]));
-}
-__global__ void k_bond_cols(zd* X, long long sX, int N, int F, const int* P, const double* E, int ncheck, int b0,
-                            int b1) {
-  const int b = blockIdx.y, f = b % F;
-  const long long e = blockIdx.x * 256ll + threadIdx.x;
-  if (e >= (long long)N * (b1 - b0)) return;
-  const int i = (int)(e % N), nc = b0 + (int)(e / N);
-  const long long k = (long long)f * ncheck + nc;
-  const int a = P[2 * k], c = P[2 * k + 1];
-  const double* m = E + 4 * k;
-  zd* Xb = X + b * sX;
-  const zd xa = Xb[i + (long long)a * N], xc = Xb[i + (long long)c * N];
-  Xb[i + (long long)a * N] = zadd(zscale(xa, m[0]), zscale(xc, m[1]));
-  Xb[i + (long long)c * N] = zadd(zscale(xa, m[2]), zscale(xc, m[3]));
-}
-
-// X(i, j) *= rs(i) (conjugated with rconj) * cs(j); rs or cs may be null.  grid (ceil(N N / 256), B)
-__global__ void k_scale_rc(zd* X, int N, const zd* rs, int rconj, const zd* cs) {
-  const int b = blockIdx.y;
-  const long long NN = (long long)N * N;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < NN; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % N), j = (int)(e / N);
-    zd v = X[b * NN + e];
-    if (rs) v = zmul(rconj ? zconj(rs[(long long)b * N + i]) : rs[(long long)b * N + i], v);
-    if (cs) v = zmul(v, cs[(long long)b * N + j]);
-    X[b * NN + e] = v;
+// each bond (Prog/OpTTypes_mod.F90:135-304): rows (X <- E X) or columns (X <- X E), family by family.
+// X(i, j) is multiplied by rs0(i) (conjugated with conj0) and cs0(j) before and rs1(i), cs1(j) after
+// (null: not).
+//
+// Row operators act within a column of X and column operators within a row, so a CTA holds its T columns
+// (rows) in shared memory through all families and the scalings: one launch where each family and
+// the scaling took one of ~4 us, most of it launch and memory latency (N = 36, eight matrices, four
+// families and the scaling: 20 us, this 6.7).  The next family's bonds are loaded ahead.
+// Arithmetic A: ArD or ArRe.  grid (ceil(N / T), B), shared memory T N values.
+struct BondScale {
+  const zd *rs0 = nullptr, *cs0 = nullptr, *rs1 = nullptr, *cs1 = nullptr;
+  int conj0 = 0;
+};
+template <class A, bool ROWS>
+__global__ void __launch_bounds__(256) k_bonds(zd* X, int N, int F, const int* P, const double* E, int ncheck,
+                                               const int* fam, int nfam, int reverse, int T, BondScale sc) {
+  typedef typename A::Z Z;
+  const int b = blockIdx.y, t0 = blockIdx.x * T, nt = min(T, N - t0), tid = threadIdx.x, nth = blockDim.x;
+  const int2* Pf = reinterpret_cast<const int2*>(P) + (long long)(b % F) * ncheck;
+  const double2* Ef = reinterpret_cast<const double2*>(E) + 2ll * (b % F) * ncheck;
+  zd* Xb = X + (long long)b * N * N;
+  const long long bN = (long long)b * N;
+  extern __shared__ __align__(16) unsigned char bonds_raw[];
+  Z* tile = reinterpret_cast<Z*>(bonds_raw);  // [t][operator index]
+  auto bond = [&](int q, int e, int2& ac, double2& m02, double2& m13) {  // entry e of family q: bond e / nt
+    const int f = reverse ? nfam - 1 - q : q, b0 = fam[f];
+    if (e >= (fam[f + 1] - b0) * nt) { ac = make_int2(-1, 0); return; }
+    const int k = b0 + e / nt;
+    const double2 u = Ef[2 * k], v = Ef[2 * k + 1];
+    ac = Pf[k];
+    m02 = make_double2(u.x, ROWS ? v.x : u.y);  // of the first site's new value
+    m13 = make_double2(ROWS ? u.y : v.x, v.y);
+  };
+  int2 ac, an;
+  double2 p0, p1, n0, n1;
+  bond(0, tid, an, n0, n1);
+  for (int e = tid; e < N * nt; e += nth) {
+    const int t = ROWS ? e / N : e % nt, o = ROWS ? e % N : e / nt, i = ROWS ? o : t0 + t, j = ROWS ? t0 + t : o;
+    zd v = Xb[i + (long long)j * N];
+    Z z = A::mk(v);
+    if (sc.rs0) z = A::mul(sc.conj0 ? A::conj(A::mk(sc.rs0[bN + i])) : A::mk(sc.rs0[bN + i]), z);
+    if (sc.cs0) z = A::mul(z, A::mk(sc.cs0[bN + j]));
+    tile[t * N + o] = z;
+  }
+  __syncthreads();
+  for (int q = 0; q < nfam; ++q) {
+    ac = an; p0 = n0; p1 = n1;
+    if (q + 1 < nfam) bond(q + 1, tid, an, n0, n1);
+    for (int e = tid; ac.x >= 0; bond(q, e, ac, p0, p1)) {
+      Z* x = tile + (e % nt) * N;
+      const Z xa = x[ac.x], xc = x[ac.y];
+      x[ac.x] = A::add(A::scale(xa, p0.x), A::scale(xc, p0.y));
+      x[ac.y] = A::add(A::scale(xa, p1.x), A::scale(xc, p1.y));
+      e += nth;
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < N * nt; e += nth) {
+    const int t = ROWS ? e / N : e % nt, o = ROWS ? e % N : e / nt, i = ROWS ? o : t0 + t, j = ROWS ? t0 + t : o;
+    Z z = tile[t * N + o];
+    if (sc.rs1) z = A::mul(A::mk(sc.rs1[bN + i]), z);
+    if (sc.cs1) z = A::mul(z, A::mk(sc.cs1[bN + j]));
+    Xb[i + (long long)j * N] = A::wide(z);
   }
 }

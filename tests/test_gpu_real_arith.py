@@ -233,3 +233,23 @@ def test_complex_products(chains, L1, L2):
 @pytest.mark.parametrize("chains,L1,L2", [(1, 13, 10), (1, 20, 10), (6, 13, 10)])
 def test_real_q_of_large_systems(chains, L1, L2):
     test_real_tau_matches_complex_products(chains, L1, L2)
+
+
+# checkerboard bonds, all families and the scalings in one launch: one and eight columns (rows) per CTA
+# (1 and 24 chains), remainders, real and complex arithmetic: against the oracle
+@pytest.mark.parametrize("flags", [0, FLAG_COMPLEX_ARITH])
+@pytest.mark.parametrize("lattice,chains,L1,L2", [("square", 1, 4, 2), ("square", 24, 6, 6), ("honeycomb", 2, 3, 3),
+                                                  ("honeycomb", 24, 4, 3)])
+def test_bond_launches(lattice, chains, L1, L2, flags):
+    m = mdl.hubbard(lattice, L1, L2, U=4.0, chem=0.2, beta=0.6, dtau=0.1, nwrap=3, checkerboard=True)
+    f0 = rng.initial_fields(17, 0, m.n_op, m.ltrot)
+    u = rng.sweep_uniforms(17, 0, m.n_op, m.ltrot, 0)
+    r, _ = _record(m, flags, f0, u, chains=chains)
+    o = oracle.Oracle(m)
+    o.set_fields(f0)
+    o.init_state()
+    o.record(1)
+    o.sweep(u)
+    ro = o.recorded()
+    for k in (0, chains - 1):
+        compare_record(r[k], ro, u, m.n_op, m.ltrot, m.nwrap, g_tol=1e-10, relative=True, exact_sequence=True)
