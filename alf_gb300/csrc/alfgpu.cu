@@ -1779,7 +1779,7 @@ static int hop_impl(alfgpu_s* h, int up, int with_scale) {
 // The slice's delayed-update blocks.  Per block: the Metropolis visits (k_update), the flush
 // operands (k_flush_xy) and the flush G -= X Y.  With h->overlap (no vector vertices, no phase
 // profile) the visits of block k + 1 run on the second stream while the flush of block k runs on
-// st: before the flush, k_sub_gather snapshots G over block k + 1's positions, and k_sub_stage
+// st: beside block k's visits, k_sub_gather snapshots G over block k + 1's positions, and k_sub_stage
 // applies block k's updates to that snapshot (the same Woodbury form), so block k + 1 starts from
 // its submatrix without waiting for the full-matrix flush.  The rank array m is kept per block
 // parity because the flush of block k reads it while block k + 1 writes its own.
@@ -1805,13 +1805,25 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
   for (size_t blk = 0; blk < nblk; ++blk) {
     int* mb = h->m + (ov ? (long long)(blk & 1) * msz : 0);
     cudaStream_t su = ov ? h->st2 : h->st;
+    // Snapshots alternate between two sets: block blk + 1's is taken on st after the flush of block
+    // blk - 1, beside block blk's visits, while its own may still be read.  Between the visits (after
+    // k_flush_xy) it was 8 us of every block's serial chain.
+    zd* snap[2] = {h->Gsnap, h->Gsnap + (size_t)h->B * UPD_KMAX * UPD_KMAX};
+    int* posn[2] = {h->posn, h->posn + (size_t)h->C * UPD_KMAX};
+    int* npos[2] = {h->npos, h->npos + h->C};
+    const int now = (int)(blk & 1), next = now ^ 1;
+    if (ov && blk + 1 < nblk) {
+      k_sub_gather<<<h->B, 256, 0, h->st>>>(h->G, F * NN, N, F, M, V, dir, h->blk_start[dir][blk + 1],
+                                            h->blk_cnt[dir][blk + 1], snap[next], posn[next], npos[next]);
+      CKL();
+    }
     if (ov && blk > 0) {  // block blk's submatrix after block blk - 1's updates
       // FP64 in both forms: this submatrix is the block's G0, whose Gamma^-1 sets the next flush
       // (double-float here raised the mixed form's largest Precision Green from 9e-6 to 6e-5)
       const int* mprev = h->m + (long long)((blk - 1) & 1) * msz;
       const dim3 gs(UPD_KMAX / 4, h->B), bs(32, 4);
-      if (real) k_sub_stage<ArRe><<<gs, bs, 0, su>>>(h->Gsnap, h->posn, h->npos, mprev, N, F, h->X, h->Y, h->Gsub);
-      else k_sub_stage<ArD><<<gs, bs, 0, su>>>(h->Gsnap, h->posn, h->npos, mprev, N, F, h->X, h->Y, h->Gsub);
+      if (real) k_sub_stage<ArRe><<<gs, bs, 0, su>>>(snap[now], posn[now], npos[now], mprev, N, F, h->X, h->Y, h->Gsub);
+      else k_sub_stage<ArD><<<gs, bs, 0, su>>>(snap[now], posn[now], npos[now], mprev, N, F, h->X, h->Y, h->Gsub);
       CKL();
     }
     UpdParams u;
@@ -1858,10 +1870,7 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
     else
       k_flush_xy<ArD><<<gxy, 256, 0, h->st>>>(h->G, F * NN, N, F, mb, h->sites, h->W, h->X, h->Y, s2o, co);
     CKL();
-    if (ov && blk + 1 < nblk) {  // snapshot for the next block, then let its visits start
-      k_sub_gather<<<h->B, 256, 0, h->st>>>(h->G, F * NN, N, F, M, V, dir, h->blk_start[dir][blk + 1],
-                                            h->blk_cnt[dir][blk + 1], h->Gsnap, h->posn, h->npos);
-      CKL();
+    if (ov && blk + 1 < nblk) {  // the next block's visits may start
       CK(cudaEventRecord(h->ev_fork, h->st));
       CK(cudaStreamWaitEvent(h->st2, h->ev_fork, 0));
     }
@@ -2181,8 +2190,8 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   r |= dalloc(h, &h->info, B); r |= dalloc(h, &h->dphase, B); r |= dalloc(h, &h->cmp, 2 * B);
   r |= dalloc(h, &h->opang, B);
   r |= dalloc(h, &h->m, 2 * (C + B)); r |= dalloc(h, &h->sites, C * UPD_KMAX);  // m: one set per block parity
-  r |= dalloc(h, &h->Gsnap, B * UPD_KMAX * UPD_KMAX); r |= dalloc(h, &h->Gsub, B * UPD_KMAX * UPD_KMAX);
-  r |= dalloc(h, &h->posn, C * UPD_KMAX); r |= dalloc(h, &h->npos, C);
+  r |= dalloc(h, &h->Gsnap, 2 * B * UPD_KMAX * UPD_KMAX); r |= dalloc(h, &h->Gsub, B * UPD_KMAX * UPD_KMAX);
+  r |= dalloc(h, &h->posn, 2 * C * UPD_KMAX); r |= dalloc(h, &h->npos, 2 * C);
   r |= dalloc(h, &h->W, C * 2 * UPD_KMAX * UPD_KMAX);
   r |= dalloc(h, &h->X, C * 2 * N * UPD_KMAX); r |= dalloc(h, &h->Y, C * 2 * N * UPD_KMAX);
   r |= dalloc(h, &h->phase, C); r |= dalloc(h, &h->cnt, 4 * C); r |= dalloc(h, &h->stat, 8 * C);

@@ -104,7 +104,7 @@ ALF_DEV int block_positions(const VertexDev& V, int c, int M, int dir, int q0, i
   return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// Snapshot of G over the positions of the next block, taken before the current block's flush
+// Snapshot of G over the positions of the next block, taken beside the current block's visits, before its flush
 // writes G: Gsnap[chain][f][a][l] = G(P_a, P_l).  Also stores the positions (pos[chain][KMAX],
 // npos[chain]).  grid (chains * F), 256 threads.
 __global__ void k_sub_gather(const zd* G, long long sG, int N, int F, int M, VertexDev V, int dir, int q0, int nq,
