@@ -1821,7 +1821,7 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       // FP64 in both forms: this submatrix is the block's G0, whose Gamma^-1 sets the next flush
       // (double-float here raised the mixed form's largest Precision Green from 9e-6 to 6e-5)
       const int* mprev = h->m + (long long)((blk - 1) & 1) * msz;
-      const dim3 gs(UPD_KMAX / 4, h->B), bs(32, 4);
+      const dim3 gs((UPD_KMAX + 7) / 8, h->B), bs(32, 8);
       if (real) k_sub_stage<ArRe><<<gs, bs, 0, su>>>(snap[now], posn[now], npos[now], mprev, N, F, h->X, h->Y, h->Gsub);
       else k_sub_stage<ArD><<<gs, bs, 0, su>>>(snap[now], posn[now], npos[now], mprev, N, F, h->X, h->Y, h->Gsub);
       CKL();

@@ -133,37 +133,21 @@ __global__ void k_sub_gather(const zd* G, long long sG, int N, int F, int M, Ver
 // The next block's submatrix after the current block's accepted updates, from the snapshot
 // and the flush operands: Gsub(a, l) = Gsnap(a, l) - sum_k X(P_a, k) Y(k, P_l), k < m (the same
 // Woodbury form the flush applies to all of G).
-// The next block's visits wait for it, so what counts is its latency: a warp per row, one warp per
-// sub-partition, every load in flight at once (N = 256, one chain: eight warps per CTA and a loop of
-// dependent loads 9.7 us, this 7.0; 16 chains 12.3, 8.1).
-// grid (KMAX / 4, chains * F), block (32, 4): (l, a).
+// grid (ceil(KMAX / 8), chains * F), block (32, 8): (l, a).
 template <class A>
-__global__ void __launch_bounds__(128) k_sub_stage(const zd* Gsnap, const int* pos, const int* npos, const int* m_in,
-                                                   int N, int F, const zd* X, const zd* Y, zd* Gsub) {
+__global__ void k_sub_stage(const zd* Gsnap, const int* pos, const int* npos, const int* m_in, int N, int F,
+                            const zd* X, const zd* Y, zd* Gsub) {
   typedef typename A::Z Z;
   const int b = blockIdx.y, c = b / F, f = b % F;
-  const int l = threadIdx.x, a = blockIdx.x * 4 + threadIdx.y;
+  const int l = threadIdx.x, a = blockIdx.x * 8 + threadIdx.y;
   const int np = npos[c], m = m_in[c];
-  const int* ps = pos + (long long)c * UPD_KMAX;
-  const int la = l < np ? l : 0;
-  const int pa = ps[a < np ? a : 0], pl = ps[la];
-  if (a >= np) return;  // the whole warp
-  const long long o = (long long)b * UPD_KMAX * UPD_KMAX + a * UPD_KMAX + la;
-  const zd *Xf = X + ((long long)c * 2 + f) * N * UPD_KMAX + pa, *Yf = Y + ((long long)c * 2 + f) * N * UPD_KMAX + (long long)pl * UPD_KMAX;
-  const Z g = A::mk(Gsnap[o]), xl = l < m ? A::mk(Xf[(long long)l * N]) : A::zero();  // lane k: X(P_a, k)
+  if (a >= np || l >= np) return;
+  const long long o = (long long)b * UPD_KMAX * UPD_KMAX + a * UPD_KMAX + l;
+  const int pa = pos[(long long)c * UPD_KMAX + a], pl = pos[(long long)c * UPD_KMAX + l];
+  const long long xy = ((long long)c * 2 + f) * N * UPD_KMAX;
   Z acc = A::zero();
-#pragma unroll
-  for (int k0 = 0; k0 < UPD_KMAX; k0 += 16) {
-    Z y[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) y[u] = k0 + u < m ? A::mk(Yf[k0 + u]) : A::zero();
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const Z x = A::shfl(xl, k0 + u);
-      if (k0 + u < m) acc = A::mac(acc, x, y[u]);
-    }
-  }
-  if (l < np) Gsub[o] = A::wide(A::sub(g, acc));
+  for (int k = 0; k < m; ++k) acc = A::mac(acc, A::mk(X[xy + pa + (long long)k * N]), A::mk(Y[xy + k + (long long)pl * UPD_KMAX]));
+  Gsub[o] = A::wide(A::sub(A::mk(Gsnap[o]), acc));
 }
 
 ALF_DEV int nranf3(double r) {
