@@ -47,11 +47,8 @@ PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # FP64 peak of a GB300: a register-only loop of independent mma.sync m8n8k4 f64 accumulators
 # (608 CTAs x 256 threads) measured 1.048 TFLOP/s; DFMA gives 1.006.
 FP64_DMMA_TFLOPS = 1.048
-# DRAM bytes (read + write) of one G-wrap GEMM launch (N_dim = 256, two flavours, one chain),
-# from an ncu capture of the 16x16 workload (dram__bytes_read.sum + dram__bytes_write.sum)
-HOP_TRAFFIC_BYTES = 3.28e6
-# the same for the mixed form's G-wrap k_oz_gemm launch of the 16-chain handle (78.1 MB read,
-# 8.3 MB written: the digit slices of G and the output), per chain
+# DRAM bytes (read + write) of the mixed form's G-wrap k_oz_gemm launch on the 16x16 workload's 16-chain
+# handle, per chain, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
 OZ_HOP_TRAFFIC_BYTES_PER_CHAIN = 86.5e6 / 16
 # default chains per GPU of each workload (the batched forms of the benchmark configurations)
 DEFAULT_CHAINS = {"hubbard4x4": 1, "hubbard16x16": 16, "honeycomb12x12": 8, "kondo12x12": 32, "batch128": 128}
@@ -154,61 +151,58 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(self.samples)}
 
 
-def algorithmic_flops(m, phase: str, launches: int, n_acc: int) -> float:
-    """Algorithmic FLOPs of one phase over `launches` launch groups of one chain (real-flop
-    convention: complex MAC = 8, real x complex MAC = 4; LAPACK counts for QR)."""
-    N, F = m.ndim, m.n_fl
-    if phase == "hop":        # 2 real x complex N^3 products per flavour per group
-        return launches * 2 * F * 4.0 * N ** 3
-    if phase == "propagate":  # per group: Nwrap (or fewer) slices of one real x complex product per flavour
-        return None
-    if phase in ("qr", "orgqr"):
-        return launches * F * (16.0 / 3.0) * N ** 3
-    if phase == "solve":
-        return launches * F * 4.0 * N ** 3
-    if phase == "flush":
-        return 8.0 * N * N * n_acc * 1.0  # rank-1 equivalents, both flavours counted in n_acc per flavour
-    return None
-
-
-def digit_pairs(n: int):
-    """(bits, slices, digit-pair products per algorithmic product) of the digit-sliced
-    tensor-core GEMM at inner dimension n, as the library picks them (ozaki.cuh oz_pick)."""
+def digit_pairs(n: int, target: int = 54):
+    """(bits, slices, digit products per algorithmic product) of the digit-sliced tensor-core GEMM
+    at inner dimension n, as the library picks them (ozaki.cuh oz_pick); target 54 in the mixed
+    form, 61 in the FP64 form."""
     kpad = (n + 63) // 64 * 64
-    bits, S = next((b, (54 + b - 1) // b) for b in range(7, 3, -1)
-                   if ((54 + b - 1) // b) * kpad * ((1 << b) - 1) ** 2 < 2 ** 24)
+    bits, S = next((b, (target + b) // b) for b in range(8, 3, -1)
+                   if (target + b) // b * b <= 63 and (target + b) // b * kpad * 4 ** (b - 1) <= 2 ** 24)
     return bits, S, S * (S + 1) // 2 + (S - 1)
 
 
+def real_model(m) -> bool:
+    """Whether every vertex exponential is real: the library then runs on real matrices."""
+    return not np.any(np.imag(np.asarray(m.pack()["op_Eexp"])))
+
+
+def wraps_on_tensor(m, chains: int, precision: str) -> bool:
+    """Whether the G wraps run on the tensor cores: always in the mixed form, in the FP64 form where
+    the FP64 MMAs of one product would take 8 us or more (alfgpu.cu oz_pays)."""
+    n8, b = (m.ndim + 7) // 8, chains * m.n_fl
+    return precision != "fp64" or n8 * n8 * ((m.ndim + 3) // 4) * b * (1 if real_model(m) else 2) * 0.30 / 608 >= 8.0
+
+
 def roofline(precision: str, chains: int, m, prof):
-    """Roofline object of the G-wrap GEMM, the largest consumer of the complex products with a
-    clean algorithmic count (2 real x complex N^3 products per flavour per slice, 2 L slices
-    per sweep).  FP64 form: k_gemm16 against the measured FP64 MMA rate.  Mixed form:
-    k_oz_slice + k_oz_gemm (digit-sliced BF16 on tcgen05) against the measured BF16 peak; the
-    algorithmic count is the same as FP64's, the BF16 products actually executed are
-    reported beside it (tensor_op_tflops)."""
+    """Roofline object of the G wraps, the largest consumer of the dense products with a clean
+    algorithmic count (2 N^3 products per flavour per slice: 2 N^3 FLOPs each on real matrices,
+    4 N^3 with a real exponential and a complex G), over the event-timed hop phase.  On the tensor cores:
+    k_oz_slice + k_oz_gemm (digit-sliced BF16 on tcgen05) against the measured BF16 peak, the BF16
+    products actually executed beside it (tensor_op_tflops); else k_gemm16 against the measured FP64
+    MMA rate."""
     hop_ms, hop_n = prof.get("hop", (0.0, 0))
-    flops = algorithmic_flops(m, "hop", hop_n, 0) * chains
-    if precision == "fp64":
-        roof = {"bound": "tensor", "kernel": "k_gemm16 (G wraps, FP64 mma.sync)", "achieved": None,
-                "peak": FP64_DMMA_TFLOPS, "unit": "TFLOP/s", "frac": None,
-                "traffic": HOP_TRAFFIC_BYTES * chains if m.ndim == 256 else None,
-                "algorithmic_flops_per_launch": chains * m.n_fl * 4.0 * m.ndim ** 3,
+    per_product = (2.0 if real_model(m) else 4.0) * m.ndim ** 3 * m.n_fl * chains
+    flops = hop_n * 2 * per_product
+    tensor = wraps_on_tensor(m, chains, precision)
+    if not tensor:
+        roof = {"bound": "fp64", "kernel": "k_gemm16 (G wraps, FP64 mma.sync)", "achieved": None,
+                "peak": FP64_DMMA_TFLOPS, "unit": "TFLOP/s", "frac": None, "traffic": None,
+                "algorithmic_flops_per_launch": per_product,
                 "peak_source": "FP64 mma.sync m8n8k4 throughput measured on a GB300 with a register-only "
                                "loop; MEASURED_PEAKS.json has no FP64 figure"}
     else:
         peak, src = measured_bf16_peak()
-        _, _, pairs = digit_pairs(m.ndim)
+        _, _, pairs = digit_pairs(m.ndim, 61 if precision == "fp64" else 54)
         roof = {"bound": "tensor", "kernel": "k_oz_slice + k_oz_gemm (G wraps, digit-sliced BF16 on tcgen05)",
                 "achieved": None, "peak": peak, "unit": "TFLOP/s", "frac": None,
-                "traffic": OZ_HOP_TRAFFIC_BYTES_PER_CHAIN * chains if m.ndim == 256 else None,
-                "algorithmic_flops_per_launch": chains * m.n_fl * 4.0 * m.ndim ** 3,
+                "traffic": OZ_HOP_TRAFFIC_BYTES_PER_CHAIN * chains if m.ndim == 256 and precision != "fp64" else None,
+                "algorithmic_flops_per_launch": per_product,
                 "bf16_products_per_algorithmic_product": pairs,
                 "peak_source": src + "; of measured"}
     if flops and hop_ms > 0:
         roof["achieved"] = flops / (hop_ms / 1e3) / 1e12
         roof["frac"] = roof["achieved"] / roof["peak"]
-        if precision != "fp64":
+        if tensor:
             # the BF16 digit products the tensor cores execute, against the same BF16 peak, and the
             # FP64-accurate algorithmic rate against the FP64 rate it replaces
             roof["tensor_op_tflops"] = roof["achieved"] * roof["bf16_products_per_algorithmic_product"]
@@ -274,7 +268,8 @@ def sweep_roofline_groups(groups, ms_per_step: float, precision: str, p_fp64: fl
             "achieved_tflops": total / (ms_per_step / 1e3) / 1e12 if ms_per_step > 0 else None,
             "peaks_tflops": {"fp64": p_fp64, "bf16": p_bf16},
             "basis": "FP64 phases at the measured FP64 MMA rate" + (
-                "" if precision == "fp64" else "; wraps, propagation and flushes at the measured BF16 peak")}
+                "" if precision == "fp64" else "; wraps, propagation and flushes at the measured BF16 peak") +
+            "; the FLOPs are the reference's complex operations, of which real models execute a quarter to a half"}
 
 
 def workload_model(name: str):
