@@ -49,7 +49,7 @@ PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FP64_DMMA_TFLOPS = 1.048
 # DRAM bytes (read + write) of the mixed form's G-wrap k_oz_gemm launch on the 16x16 workload's 16-chain
 # handle, per chain, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
-OZ_HOP_TRAFFIC_BYTES_PER_CHAIN = 86.5e6 / 16
+OZ_HOP_TRAFFIC_BYTES_PER_CHAIN = 35.8e6 / 16
 # default chains per GPU of each workload (the batched forms of the benchmark configurations)
 DEFAULT_CHAINS = {"hubbard4x4": 1, "hubbard16x16": 16, "honeycomb12x12": 8, "kondo12x12": 32, "batch128": 128}
 L2_NOTE = "GPU arm: L2 flushed between timed steps (256 MB write); host arm: not applicable"
