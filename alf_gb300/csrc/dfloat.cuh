@@ -25,8 +25,10 @@ ALF_DEV dff df_qts(float a, float b) {  // |a| >= |b| or a == 0
   return dff{s, __fsub_rn(b, __fsub_rn(s, a))};
 }
 // FP64 <-> double-float.  The conversion instructions run on the FP64 pipe (64 cycles per warp each),
-// so in the range of FP32 the bits are moved on the integer pipes: x = hi (24 bits, truncated) +
-// the other 29 bits as a float; and the exponent of a float rebiased for the way back.
+// so in the range of FP32 the bits are moved on the integer pipes: x = h + l with h the nearest float
+// (a carry of the rounding runs on into the exponent; a tie goes away from zero, where l is exact)
+// and l the signed 29-bit rest as a float, off by 2^-49 |x| at most, as h = float(x), l = float(x - h)
+// are; and the exponent of a float rebiased for the way back.
 ALF_DEV dff df_make(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), sg = hi & 0x80000000u;
   if (((hi << 1) | lo) == 0u) return dff{0.f, 0.f};
@@ -37,9 +39,10 @@ ALF_DEV dff df_make(double x) {
     v.l = __double2float_rn(x - (double)v.h);
     return v;
   }
-  const float h = __uint_as_float(sg | ((unsigned)(e + 127) << 23) | (((hi << 3) | (lo >> 29)) & 0x7fffffu));
-  const float l = __uint2float_rn(lo & 0x1fffffffu) * __uint_as_float(sg | ((unsigned)(e + 75) << 23));
-  return df_qts(h, l);
+  const unsigned lr = lo + 0x10000000u, hr = hi + (lr < lo ? 1u : 0u);
+  const float h = __uint_as_float(sg | ((((hr << 3) | (lr >> 29)) - 0xc0000000u) & 0x7fffffffu));
+  const float l = __int2float_rn((int)(lo << 3) >> 3) * __uint_as_float(sg | ((unsigned)(e + 75) << 23));
+  return dff{h, l};
 }
 ALF_DEV double df_f2d(float f) {
   const unsigned u = (unsigned)__float_as_int(f), e = (u >> 23) & 0xffu;
