@@ -615,7 +615,6 @@ static int oz_gemm(alfgpu_s* h, const CUtensorMap& ta, const CUtensorMap& tb, in
   p.csc = csc; p.scsc = scsc;
   p.Kv = ((kvalid > 0 ? kvalid : Kpad) + 15) / 16;
   oz_words(kvalid > 0 ? kvalid : Kpad, bits, S, p.nd, &p.lg, &p.pair);
-  if (h->mixed && h->oz_narrow && h->oz_Kpad <= 128) p.L = oz_shift(Kpad, bits, S, p.nd);
   p.RpadA = RpadA; p.RpadB = RpadB; p.modA = modA; p.modB = modB; p.expA = expA; p.expB = expB;
   p.omode = omode; p.osub = osub; p.out = out; p.ldr = ldr; p.ldc = ldc; p.sout = sout; p.err = h->err;
   p.rsc = rsc; p.srsc = srsc;

@@ -377,22 +377,6 @@ ALF_DEV double oz_round(long long zh, long long zl, int sh, int sc) {
   return __longlong_as_double((long long)(u | ((unsigned long long)(unsigned)neg << 63)));
 }
 
-// z 2^sc rounded to the nearest FP64 (ties to even), |z| < 2^63.
-ALF_DEV double oz_round1(long long z, int sc) {
-  const unsigned long long nl = (unsigned long long)(z >> 63);
-  const unsigned long long a = ((unsigned long long)z ^ nl) - nl;
-  const int n = __clzll((long long)a);
-  const unsigned long long m = a << (n & 63);
-  const unsigned rem = (unsigned)m & 0x7ffu;
-  unsigned long long r = m >> 11;
-  r += (rem > 0x400u || (rem == 0x400u && (r & 1ull))) ? 1ull : 0ull;
-  const int be = 63 - n + sc + 1023;
-  unsigned long long u = ((unsigned long long)(unsigned)(be - 1) << 52) + r;
-  if (be <= 0 || !a) u = 0ull;
-  if (be >= 2047 && a) u = 0x7ff0000000000000ull;
-  return __longlong_as_double((long long)(u | (nl & 0x8000000000000000ull)));
-}
-
 // ---------------------------------------------------------------------------------------
 // GEMM
 // ---------------------------------------------------------------------------------------
@@ -400,7 +384,6 @@ struct OzGemmParams {
   int M, N;                  // logical rows of A and of B (valid extents)
   int nkc, S, bits, nst;     // K chunks (Kpad / 64), slices, bits per slice, ring stages
   int nd;                    // diagonals accumulated: s + t < nd (0-based digit indices), nd = S + 1
-  int L;                     // > 0: one 64-bit word with 2^-L as its unit instead of two (oz_words)
   int lg, pair;              // diagonals in the low word (ND - lg even); two diagonals fit 32 bits (oz_words)
   int Kv;                    // K steps of 16 that hold digits (the rest of Kpad is zero)
   int RpadA, RpadB;
@@ -652,34 +635,6 @@ __global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_
     // The diagonals d, d + 1 first meet in one 32-bit word where it holds them (p.pair).
     auto f2i = [](uint32_t u) { return __float2int_rn(__uint_as_float(u)); };
     double v[HB];
-    if (p.L > 0) {
-      // one word, the low diagonals cut to its unit
-#pragma unroll
-      for (int j = 0; j < HB; ++j) Zl[j] = 0;
-      auto add = [&](long long& z, long long w, int sh) {
-        z += sh >= 0 ? w << sh : w >> -sh;
-      };
-      for (int d = 0; d < ND; d += 2) {
-        uint32_t r0[HB], r1[HB];
-        const bool two = d + 1 < ND;
-        oz_tmem_ld_async<HB>(tcol + (uint32_t)(d * BN), r0);
-        if (two) oz_tmem_ld_async<HB>(tcol + (uint32_t)((d + 1) * BN), r1);
-        oz_tmem_wait<HB>(r0, r1);
-        const int sh0 = p.L - p.bits * (d + 2), sh1 = sh0 - p.bits;
-        if (two && p.pair) {
-#pragma unroll
-          for (int j = 0; j < HB; ++j) add(Zl[j], (long long)((f2i(r0[j]) << p.bits) + f2i(r1[j])), sh1);
-        } else {
-#pragma unroll
-          for (int j = 0; j < HB; ++j) add(Zl[j], (long long)f2i(r0[j]), sh0);
-          if (two)
-#pragma unroll
-            for (int j = 0; j < HB; ++j) add(Zl[j], (long long)f2i(r1[j]), sh1);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < HB; ++j) v[j] = oz_round1(Zl[j], ea + eb[j] - p.L);
-    } else {
     for (int d = 0; d < ND; d += 2) {  // two diagonals' loads in flight
       uint32_t r0[HB], r1[HB];
       const bool two = d + 1 < ND;
@@ -713,7 +668,6 @@ __global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_
     }
 #pragma unroll
     for (int j = 0; j < HB; ++j) v[j] = oz_round(Zh[j], Zl[j], p.bits * lg, ea + eb[j] - p.bits * (ND + 1));
-    }
     if (p.rsc && m < p.M) {
       const double s = p.rsc[(size_t)b * p.srsc + m].x;
 #pragma unroll
@@ -881,19 +835,6 @@ static inline void oz_words(int Kpad, int bits, int S, int nd, int* lg, int* pai
   *lg = (nd + 1) / 2;
   if ((nd - *lg) & 1) --*lg;
   *pair = (double)S * Kpad * (double)(1 << (2 * (bits - 1))) * ((1 << bits) + 1) < 2147483648.0;
-}
-
-// One word: the largest L with sum_D |acc_D| 2^(L - b D) < 2^62.  The low diagonals are cut to its unit,
-// 2^-L of the scales (about 2^-53 of the largest products).  For the mixed form on small grids with
-// K <= 128 alone: the shorter epilogue is on the critical path there (mean Precision Green 7e-11 at N = 64,
-// 4 chains, beta = 4).
-static inline int oz_shift(int Kpad, int b, int S, int nd) {
-  double z = 0.0;
-  for (int D = 2; D < nd + 2; ++D) {
-    const int pairs = std::min(D - 1, std::min(S, 2 * S + 1 - D));
-    z += std::ldexp(std::min(16777216.0, (double)pairs * Kpad * (double)(1 << (2 * (b - 1)))), -b * D);
-  }
-  return (int)std::floor(62.0 - std::log2(z));
 }
 
 static inline int oz_roundup(int x, int m) { return (x + m - 1) / m * m; }
