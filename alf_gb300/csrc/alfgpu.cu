@@ -2580,9 +2580,9 @@ static int check_err(alfgpu_s* h) {
   CK(cudaMemcpy(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
     CK(cudaMemset(h->err, 0, sizeof(int)));
+    if (e & 4) return ALFGPU_ERROR_TIMEOUT;  // first: the others may be what it left behind
     if (e & 1) return ALFGPU_ERROR_NAN;
     if (e & 2) return ALFGPU_ERROR_UNSTABLE_MATRIX;
-    if (e & 4) return ALFGPU_ERROR_TIMEOUT;
     return ALFGPU_ERROR_GENERIC;
   }
   return 0;

@@ -8,6 +8,9 @@
 
 #define QRC_WORK 256                 // threads that carry FP64 work: two warps per sub-partition
 #define QRC_THREADS (QRC_WORK + 32)  // and one warp of integer bookkeeping
+#ifndef QRC_WAIT_CYCLES
+#define QRC_WAIT_CYCLES (1ll << 31)  // a wait's limit in SM cycles: one second
+#endif
 
 struct QRColsParams {
   const zd* Ain;             // input (may equal A)
@@ -38,7 +41,7 @@ static inline size_t qrc_smem_bytes(int N, int CL, int zb) {
 }
 
 ALF_DEV uint32_t qrc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// Wait for a phase of an mbarrier of this CTA; gives up after ~2^31 SM cycles (one second).
+// Wait for a phase of an mbarrier of this CTA; gives up after QRC_WAIT_CYCLES.
 ALF_DEV bool qrc_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -53,7 +56,7 @@ ALF_DEV bool qrc_wait(uint32_t bar, uint32_t parity) {
   if (qrc_try(bar, parity)) return true;
   const long long t0 = clock64();
   while (!qrc_try(bar, parity))
-    if (clock64() - t0 > (1ll << 31)) return false;
+    if (clock64() - t0 > QRC_WAIT_CYCLES) return false;
   return true;
 }
 ALF_DEV void qrc_expect(uint32_t bar, uint32_t bytes) {
@@ -188,7 +191,9 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
   __shared__ QRCand cand[2][16];                      // the CTAs' candidates, pushed by them
   __shared__ QRCand wc[QRC_WORK / 32];                // the warps' candidates: col is the index in the active list
   __shared__ __align__(8) unsigned long long mb[4];   // cand[0], cand[1], xb[0], xb[1] complete
-  __shared__ struct { int lw, nact, lanes, dead; } st;  // step j: own slot chosen or -1, active columns, lanes
+  // step j: own slot chosen or -1, active columns, lanes; dead: 1 + the step whose exchange gave up, gone:
+  // some CTA of the cluster has given up
+  __shared__ struct { int lw, nact, lanes, dead, gone; } st;
   __shared__ struct { Z tau, scal; double ib; int trivial; } rf;  // the reflector of step j
   const double tol3z = 1.0536712127723509e-08;  // sqrt(dlamch('Epsilon'))
   const zd* Ab = p.Ain + b * p.sA;
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(qrc_smem(mb + i)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    st.dead = 0;
+    st.dead = st.gone = 0;
   }
   for (int lc = warp; lc < nmine; lc += QRC_THREADS / 32) {
     const int c = (int)rank + lc * (int)CL;
@@ -289,19 +294,20 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
     if (join) qrc_bar_join();
     qrc_fence_async();  // the column as the work warps left it, for the copy engine
     if (q.col >= 0) q.col = (int)rank + (act[q.col] << lgC);
-    bool ok = qrc_wait(cbar, (unsigned)(j >> 1) & 1u);
-    unsigned long long key = 0;
-    int pw = 0x7fffffff, w = -1;
-    if (lane < (int)CL) {
-      if (lane != (int)rank) q = cand[par][lane];
-      key = q.key; pw = q.pos; w = q.col;
-    }
-    qrc_argmax(key, pw, w);
-    if (w < 0) { ok = false; w = 0; }  // only if a candidate did not come
-    const bool own = (w & ((int)CL - 1)) == (int)rank;
-    const int lw = w >> lgC, i0 = j & ~(ZA - 1);
+    const int i0 = j & ~(ZA - 1);
     const uint32_t bytes = (uint32_t)((N - i0 + ZA - 1) & ~(ZA - 1)) * ZB;
+    bool armed = false, ok = __all_sync(0xffffffffu, qrc_wait(cbar, (unsigned)(j >> 1) & 1u));
     if (ok) {
+      unsigned long long key = 0;
+      int pw = 0x7fffffff, w = -1;
+      if (lane < (int)CL) {
+        if (lane != (int)rank) q = cand[par][lane];
+        key = q.key; pw = q.pos; w = q.col;
+      }
+      qrc_argmax(key, pw, w);
+      const bool own = (w & ((int)CL - 1)) == (int)rank;
+      const int lw = w >> lgC;
+      armed = true;
       if (own) {
         const uint32_t src = qrc_smem(cols + (size_t)lw * ld + i0);
         if (lane < (int)CL && lane != (int)rank)
@@ -310,23 +316,28 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
       } else if (lane == 0) {
         qrc_expect(xbar, bytes);
       }
+      for (int t = lane; t < nact; t += 32) {  // positions and the active list
+        const int lc = act[t];
+        if (pos[lc] == j) pos[lc] = pw;
+        if (j > 0 || (own && lc == lw)) an[t] = own && lc == lw ? last : lc;  // past the new end: never read
+      }
+      if (pw != j) sign = -sign;
+      if (lane == 0) {
+        if (own) fin[lw] = j;
+        st.lw = own ? lw : -1;
+        st.nact = nact - (own ? 1 : 0); st.lanes = own ? ln1 : ln0;
+        if (rank == 0) p.jpvt[b * p.sP + j] = w + 1;
+      }
+      ok = __all_sync(0xffffffffu, qrc_wait(xbar, (unsigned)(j >> 1) & 1u));
     }
-    for (int t = lane; t < nact; t += 32) {  // positions and the active list
-      const int lc = act[t];
-      if (pos[lc] == j) pos[lc] = pw;
-      if (j > 0 || (own && lc == lw)) an[t] = own && lc == lw ? last : lc;  // past the new end: never read
-    }
-    if (pw != j) sign = -sign;
-    if (lane == 0) {
-      if (own) fin[lw] = j;
-      st.lw = own ? lw : -1;
-      st.nact = nact - (own ? 1 : 0); st.lanes = own ? ln1 : ln0;
-      if (rank == 0) p.jpvt[b * p.sP + j] = w + 1;
-    }
-    if (ok) ok = qrc_wait(xbar, (unsigned)(j >> 1) & 1u);
-    if (!__all_sync(0xffffffffu, ok) && lane == 0) {
-      st.dead = 1;
-      if (p.err) atomicOr(p.err, 4);
+    if (!ok) {
+      if (lane < (int)CL) asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(dsmem_addr(&st.gone, lane)) : "memory");
+      if (lane == 0) {
+        st.dead = j + 1;
+        if (!armed) qrc_expect(xbar, bytes);  // what may still come: this step's messages, the next candidates
+        qrc_expect(qrc_smem(mb + (par ^ 1)), 16u * (CL - 1));
+        if (p.err) atomicOr(p.err, 4);
+      }
     }
   };
 
@@ -467,6 +478,21 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
   }
   __syncwarp();
   cluster_sync();  // no CTA leaves while a peer may still write to it
+  if (st.gone) {
+    // Nothing is sent any more.  A CTA that gave up waits until what its peers had sent has landed in its
+    // shared memory (a message that was never sent costs the limit), and none leaves before.  No column is
+    // written, but the pivots stay indices: the kernels that run before the host reads the error use them.
+    if (rank == 0 && st.dead)
+      for (int i = tid; i < N; i += QRC_THREADS) p.jpvt[b * p.sP + i] = i + 1;
+    if (rank == 0 && tid == QRC_WORK) p.info[b].psign = sign;
+    if (st.dead && tid < 3) {
+      const int s = st.dead - 1 + (tid == 1);
+      qrc_wait(qrc_smem(mb + (tid == 2 ? 2 : 0) + (s & 1)), (unsigned)(s >> 1) & 1u);
+    }
+    __syncwarp();
+    cluster_sync();
+    return;
+  }
   for (int lc = warp; lc < nmine; lc += QRC_THREADS / 32) {
     const int j = fin[lc];
     const Z sc = scl[lc];
