@@ -2926,6 +2926,15 @@ static int oneshot_handle(int N, alfgpu_s** out) {
   return alfgpu_create(out, &d);
 }
 
+// The end of a one-shot call: a wait that gave up is an error, and the caller's buffers stay as they were (a NaN in
+// the factors is the caller's, and goes through as it does in the reference).
+static int oneshot_wait(alfgpu_s* h) {
+  int e = 0;
+  CK(cudaStreamSynchronize(h->st));
+  CK(cudaMemcpy(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost));
+  return e & 4 ? ALFGPU_ERROR_TIMEOUT : 0;
+}
+
 int alfgpu_cgr(int32_t ndim, int32_t nvar, const double* UR, const double* DR, const double* VR, const double* UL,
                const double* DL, const double* VL, double* G, double* phase) {
   if (ndim < 1 || !UR || !DR || !VR || !UL || !DL || !VL || !G || !phase) return ALFGPU_ERROR_ARGUMENT;
@@ -2963,7 +2972,7 @@ int alfgpu_cgr(int32_t ndim, int32_t nvar, const double* UR, const double* DR, c
     sp.phase = h->phase; sp.stat = h->stat; sp.err = h->err;
     k_stab_finish<<<1, 32, 0, h->st>>>(sp);
     CKL();
-    CK(cudaStreamSynchronize(h->st));
+    RET(oneshot_wait(h));
     CK(cudaMemcpy(G, h->G, NN * sizeof(zd), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(phase, h->phase, sizeof(zd), cudaMemcpyDeviceToHost));
     return 0;
@@ -2987,7 +2996,7 @@ int alfgpu_decompose(int32_t ndim, char side, double* U, double* D, double* V) {
     CK(cudaMemcpy(s.V, V, NN * sizeof(zd), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s.D, dd.data(), N * sizeof(double), cudaMemcpyHostToDevice));
     RET(decompose(h, s, left));
-    CK(cudaStreamSynchronize(h->st));
+    RET(oneshot_wait(h));
     CK(cudaMemcpy(U, s.U, NN * sizeof(zd), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(V, s.V, NN * sizeof(zd), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(dd.data(), s.D, N * sizeof(double), cudaMemcpyDeviceToHost));

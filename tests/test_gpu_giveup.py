@@ -3,13 +3,14 @@ the call reports it, and the device stays usable.
 
 The library is built once more from a copy of its sources in which CTA 1 of a cluster never posts
 its candidate column, with waits of about two milliseconds: every wait on it runs out."""
+import ctypes
 import os
 import shutil
 
 import numpy as np
 import pytest
 
-from alf_gb300 import _lib, build, model as mdl, rng
+from alf_gb300 import _lib, build, model as mdl, rng, sweep
 from alf_gb300.sweep import Chains
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,28 @@ def test_init_state_reports_a_missing_candidate(silent, L):
                 _start(L)
             assert e.value.code == 104
     assert np.array_equal(_start(L), G)
+
+
+# the one-shot calls on host buffers: the error, and the outputs untouched
+@pytest.mark.parametrize("N", [40, 100, 144])
+def test_one_shot_calls_report_it(silent, N):
+    r = np.random.default_rng(N)
+    U = np.linalg.qr(r.standard_normal((N, N)) + 1j * r.standard_normal((N, N)))[0]
+    V = np.eye(N, dtype=complex)
+    D = np.exp(np.linspace(3.0, -3.0, N)).astype(complex)
+    want = sweep.cgr(1, U, D, V, U, D, V), sweep.decompose("r", U, D, V)
+    with silent:
+        with pytest.raises(_lib.AlfGpuError) as e:
+            sweep.cgr(1, U, D, V, U, D, V)
+        assert e.value.code == 104
+        with pytest.raises(_lib.AlfGpuError) as e:
+            sweep.decompose("r", U, D, V)
+        assert e.value.code == 104
+        u, d, v = U.T.copy(), D.copy(), V.T.copy()
+        kept = u.copy(), d.copy(), v.copy()
+        p = lambda a: ctypes.c_void_p(a.ctypes.data)
+        assert _lib.lib().alfgpu_decompose(N, ctypes.c_char(b"r"), p(u), p(d), p(v)) == 104
+        assert all(np.array_equal(a, b) for a, b in zip((u, d, v), kept))
+    (G, ph), dec = sweep.cgr(1, U, D, V, U, D, V), sweep.decompose("r", U, D, V)
+    assert np.array_equal(G, want[0][0]) and ph == want[0][1]
+    assert all(np.array_equal(a, b) for a, b in zip(dec, want[1]))
