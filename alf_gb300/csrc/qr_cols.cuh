@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
         const double ar = A::re(alpha);
         t2 = A::abs2add(alpha, xn2);
         if (alf_normal(t2)) {
-          ib = -copysign(alf_rsqrt_n(t2), ar);
+          ib = -copysign(rsqrt(t2), ar);
           tau = A::mkz(fma(-ar, ib, 1.0), -A::im(alpha) * ib);  // 1 <= |tau|^2 <= 4
           if constexpr (A::kReal) scal = -ib * alf_rcp_n(tau);
           else scal = A::scale(A::conj(tau), -ib * alf_rcp_n(A::abs2(tau)));
@@ -405,14 +405,7 @@ __global__ void __launch_bounds__(QRC_THREADS) k_qrp_cols(QRColsParams p) {
     if (!work && lw >= 0) {  // beta, needed at the end only
       double beta = A::re(alpha);
       if (!plain) {
-        double s;
-        if (alf_normal(t2)) {
-          const double r = fabs(ib);
-          s = t2 * r;
-          s = fma(fma(-s, s, t2), alf_half(r), s);
-        } else {
-          s = sqrt(t2);
-        }
+        const double s = alf_normal(t2) ? alf_sqrt_n(t2, fabs(ib)) : sqrt(t2);
         beta = -copysign(s, beta);
       }
       if (lane == 0) {

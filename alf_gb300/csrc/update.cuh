@@ -28,7 +28,7 @@
 // weight test and the phase are FP64 in both forms.  GB300's FP64 dependent
 // latency (63-76 cycles, ~560 for a division) sets the cost of every visit, so
 // the chain avoids divisions and square roots: the Metropolis test is
-// division-free, the reciprocal is a Newton iteration, and the phase stays
+// division-free, the reciprocal is one step of an iteration (arith.cuh), and the phase stays
 // unnormalised until the block ends.
 #pragma once
 #include "common.cuh"

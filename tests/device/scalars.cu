@@ -40,3 +40,18 @@ extern "C" int chk_df_make(const double* x, float* hi, float* lo, double* back, 
   bh.out(); bl.out(); bb.out();
   return rc;
 }
+
+// out: [5][n] the approximation, this library's and CUDA's reciprocal of x, this library's and CUDA's root of |x|
+extern "C" int chk_roots(const double* x, double* out, int n) {
+  Buf<double> bx(x, n), bo(out, 5 * n);
+  const double* p = bx.d;
+  double* o = bo.d;
+  const long long m = n;
+  const int rc = each(n, [=] __device__(int i) {
+    const double y = p[i], t = fabs(y);
+    o[i] = alf_rcp_seed(y); o[m + i] = alf_rcp(y); o[2 * m + i] = 1.0 / y;
+    o[3 * m + i] = alf_sqrt_n(t, rsqrt(t)); o[4 * m + i] = sqrt(t);
+  });
+  bo.out();
+  return rc;
+}

@@ -36,3 +36,50 @@ def test_df_make(dev, lo, hi):
     ln = (x - hn.astype(np.float64)).astype(np.float32)
     assert np.array_equal(h[~tie], hn[~tie]) and np.array_equal(l[~tie], ln[~tie])
     assert np.array_equal(back, s)
+
+
+def _roots(dev, x):
+    out = np.empty((5, len(x)))
+    assert dev.chk_roots(_p(np.ascontiguousarray(x)), _p(out), len(x)) == 0
+    return out
+
+
+def _ulps(a, exact):
+    """|a - exact| in units in the last place of the rounded exact value."""
+    return float(np.max(np.abs(a.astype(np.longdouble) - exact) / np.spacing(np.abs(exact).astype(np.float64))))
+
+
+# Every upper word of the mantissa, both exponent parities, the lower word at its ends: the approximation
+# within 2^-19, so the reciprocal within half an ulp for its rounding and e^3 / 2^-53 = 1/16 at most; the
+# root's Newton step leaves the rounding and the square of a few ulp.  Exact values in extended precision
+# (64 or 113 bits: 2^-11 ulp or less).
+@pytest.mark.parametrize("low", [0, 1, 0x80000000, 0xffffffff])
+@pytest.mark.parametrize("e", [0, 1])
+def test_reciprocal_and_root_all_mantissas(dev, e, low):
+    hi = np.arange(1 << 20, dtype=np.uint64)
+    x = (((1023 + e) << 52) | (hi << 32) | low).astype(np.uint64).view(np.float64)
+    o = _roots(dev, x)
+    xl = x.astype(np.longdouble)
+    seed = float(np.max(np.abs(1 - xl * o[0])))
+    u, v = _ulps(o[1], 1 / xl), _ulps(o[3], np.sqrt(xl))
+    print(f"e = {e}, low = {low:#x}: approximation 2^{np.log2(seed):.2f}, reciprocal {u:.4f} ulp (CUDA's "
+          f"{_ulps(o[2], 1 / xl):.4f}), root {v:.4f} ({_ulps(o[4], np.sqrt(xl)):.4f})")
+    assert seed <= 2.0 ** -19 and u <= 0.57 and v <= 0.51
+
+
+# the whole range of the corrected forms, its edges from both sides, signs; beyond it the reciprocal is CUDA's
+@pytest.mark.parametrize("lo,hi", [(-900, -890), (-899, 899), (890, 900)])
+def test_reciprocal_and_root_range(dev, lo, hi):
+    r = np.random.default_rng(hi + 1000)
+    x = np.ldexp(1.0 + r.random(200000), r.integers(lo, hi, 200000))
+    x = np.concatenate([x, np.ldexp([1.0, 1.0 + 2.0 ** -52, 2.0 - 2.0 ** -52], lo), np.ldexp([1.0, 2.0 - 2.0 ** -52], hi - 1)])
+    o, n = _roots(dev, np.concatenate([x, -x])), len(x)
+    xl = x.astype(np.longdouble)
+    assert _ulps(o[1, :n], 1 / xl) <= 0.57 and np.array_equal(o[1, n:], -o[1, :n])
+    assert _ulps(o[3, :n], np.sqrt(xl)) <= 0.51
+
+
+def test_reciprocal_outside(dev):
+    x = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 2.0 ** -1022, 2.0 ** -1000, -2.0 ** 1000, 1.7e308])
+    with np.errstate(divide="ignore", over="ignore"):
+        assert np.array_equal(_roots(dev, x)[1], 1.0 / x, equal_nan=True)
