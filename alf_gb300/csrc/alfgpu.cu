@@ -1954,8 +1954,8 @@ const char* alfgpu_error_string(int code) {
   }
 }
 
-// Buffers, tensor maps and tile shapes of the tensor-core GEMMs of the mixed form; leaves
-// h->oz = 0 (double-float GEMMs) when a size does not fit.
+// Buffers, tensor maps and tile shapes of the tensor-core GEMMs; leaves h->oz = 0 when a size does not
+// fit (mixed form: double-float GEMMs), and in the FP64 form when the buffers do not (FP64 pipes).
 static int oz_setup(alfgpu_s* h) {
   const int N = h->N;
   const size_t B = h->B, F = h->F;
@@ -2001,6 +2001,7 @@ static int oz_setup(alfgpu_s* h) {
   }
   if (!oz_encoder()) return 0;
   const size_t S = h->oz_S, Sf = h->ozf_S, Kp = h->oz_Kpad, Kf = 2 * UPD_KMAX, RpN = h->oz_RpN, Rp2 = h->oz_Rp2N;
+  const size_t before = h->allocs.size();
   int r = 0;
   for (int a = 0; a < 4; ++a) { r |= dalloc(h, &h->ozE[a], F * S * RpN * Kp); r |= dalloc(h, &h->ozEe[a], F * RpN); }
   r |= dalloc(h, &h->ozGA, B * S * Rp2 * Kp); r |= dalloc(h, &h->ozGAe, B * Rp2);
@@ -2009,7 +2010,12 @@ static int oz_setup(alfgpu_s* h) {
   r |= dalloc(h, &h->ozYB, B * Sf * Rp2 * Kf); r |= dalloc(h, &h->ozYBe, B * Rp2);
   r |= dalloc(h, &h->ozGm, B * 1024); r |= dalloc(h, &h->ozTm, B * 1024);
   r |= dalloc(h, &h->ozWm, B * 32 * (size_t)N); r |= dalloc(h, &h->ozXm, B * 32 * (size_t)N);
-  if (r) return ALFGPU_ERROR_CUDA;
+  if (r && h->mixed) return ALFGPU_ERROR_CUDA;
+  if (r) {
+    while (h->allocs.size() > before) { cudaFree(h->allocs.back()); h->allocs.pop_back(); }
+    cudaGetLastError();
+    return 0;
+  }
   int t = 0;
   for (int a = 0; a < 4; ++a)
     t |= oz_tmap(&h->tmE[a], h->ozE[a], (int)Kp, (long long)(F * S * RpN), a < 2 ? OZ_BM : h->oz_bn);
@@ -2045,6 +2051,18 @@ static int oz_setup(alfgpu_s* h) {
   }
   h->oz = 1;
   return 0;
+}
+
+// FP64 form: the tensor-core buffers (at N = 16 590 KB per matrix, whose G is 4 KB) once the vertices say in
+// which arithmetic the handle runs, and only if some product of it pays there.
+static int oz_setup_fp64(alfgpu_s* h) {
+  if (h->mixed || h->oz || (h->d.reserved[0] & ALFGPU_FLAG_NO_TENSOR_GEMM)) return 0;
+  if (!oz_pays(h, h->N, h->N, 4, OZ_MIN_US) && !(real_model(h) && oz_pays(h, h->N, UPD_KMAX, 1, OZ_MIN_FLUSH_US)))
+    return 0;
+  CK(cudaSetDevice(h->dev));
+  RET(oz_setup(h));
+  h->oz_stab = h->oz;
+  return h->hop_ok ? oz_slice_expT(h) : 0;
 }
 
 int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
@@ -2198,10 +2216,10 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   r |= dalloc(h, &h->draws, C * 6 * M * L);
   r |= dalloc(h, &h->rngkey, C); r |= dalloc(h, &h->rngctr, C);
   if (r) return fail(ALFGPU_ERROR_CUDA);
-  if (!(d.reserved[0] & ALFGPU_FLAG_NO_TENSOR_GEMM)) {
+  if (h->mixed && !(d.reserved[0] & ALFGPU_FLAG_NO_TENSOR_GEMM)) {
     const int e = oz_setup(h);
     if (e) return fail(e);
-    h->oz_stab = h->oz && !(h->mixed && (d.reserved[0] & ALFGPU_FLAG_FP64_STAB_GEMM)) && !h->df_stab;
+    h->oz_stab = h->oz && !(d.reserved[0] & ALFGPU_FLAG_FP64_STAB_GEMM) && !h->df_stab;
   }
   h->h_key.assign(C, 0); h->h_ctr.assign(C, 0);
   for (size_t c = 0; c < C; ++c) { h->h_key[c] = alf_chain_key(0, c); h->h_ctr[c] = M * L; }
@@ -2520,7 +2538,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
   if (rot_changed && h->hop_ok) RET(upload_expT(h));
   drop_graphs(h);  // block partition and basis may have changed
   h->vert_ok = true;
-  return 0;
+  return oz_setup_fp64(h);
 }
 
 int alfgpu_set_fields(alfgpu_t* h, int32_t chain, const int8_t* f) {
