@@ -64,6 +64,9 @@ struct alfgpu_s {
   // ALFGPU_FLAG_COMPLEX_ARITH): otherwise every matrix of the sweep is real and the FP64 kernels
   // that have a real form run it (ArRe; the matrices stay complex128 in memory)
   int model_complex = 0;
+  // per chain: bit 0 complex exponentials, bit 1 complex exponentials or factors.  An upload sets the two
+  // flags above; alfgpu_init_state, which rebuilds every matrix from the fields, takes them back.
+  std::vector<int8_t> vcplx;
   int oz_narrow = 0;  // small grids: BN = 16 tiles; the flush keeps the double-float GEMM (measured faster there)
   int oz_stab = 0;    // the stabilisation's complex products on the tensor-core GEMM too
   zd *ozGm = nullptr, *ozTm = nullptr, *ozWm = nullptr, *ozXm = nullptr;  // compact-WY explicit Q work
@@ -2101,6 +2104,7 @@ int alfgpu_create(alfgpu_t** out, const alfgpu_dims* dims) {
   h->df_qr = h->mixed && (d.reserved[0] & ALFGPU_FLAG_DF_STAB_QR);
   h->use_graph = !(d.reserved[0] & ALFGPU_FLAG_NO_GRAPH);
   h->model_complex = (d.reserved[0] & ALFGPU_FLAG_COMPLEX_ARITH) ? 1 : 0;
+  h->vcplx.assign(h->C, 0);
   fill_tables(h->ft);
   auto fail = [&](int code) { alfgpu_destroy(h); return code; };
   if (cudaSetDevice(d.device) != cudaSuccess) return fail(ALFGPU_ERROR_CUDA);
@@ -2360,6 +2364,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
   std::vector<std::pair<int, int>> pairs;
   double U[4] = {1.0, 0.0, 0.0, 1.0};
   bool have_rot = false;
+  int8_t cplx = 0;  // as vcplx; the handle's flags change only when the upload is accepted
   for (size_t k = 0; k < K; ++k) {
     const int n = v->op_n[k], nz = v->op_nz[k];
     if (n < 1 || n > 2 || nz < 1 || nz > n) return ALFGPU_ERROR_UNSUPPORTED;
@@ -2390,7 +2395,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
       for (int s = 0; s < 5; ++s)
         ee[k * 10 + m * 5 + s] = zmk(v->op_Eexp[(k * 10 + m * 5 + s) * 2], v->op_Eexp[(k * 10 + m * 5 + s) * 2 + 1]);
     for (int s = 0; s < 10; ++s)
-      if (ee[k * 10 + s].y != 0.0) h->eexp_complex = h->model_complex = 1;
+      if (ee[k * 10 + s].y != 0.0) cplx = 3;
     if (!std::isfinite(g[k].x) || !std::isfinite(g[k].y)) return ALFGPU_ERROR_HAMILTONIAN;
   }
   // the vertices of every flavour act on the same sites
@@ -2484,7 +2489,7 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
         }
         const std::complex<double> ea = std::exp(Z1 * std::complex<double>(al[k].x, al[k].y));
         e.expal = zmk(ea.real(), ea.imag());
-        if (e.myexp[0].y != 0.0 || e.myexp[1].y != 0.0 || e.expal.y != 0.0) h->model_complex = 1;
+        if (e.myexp[0].y != 0.0 || e.myexp[1].y != 0.0 || e.expal.y != 0.0) cplx |= 2;
       }
   }
   // positions of each site, ascending (vertex n, eigen-index I) -> 2n + I, per flavour
@@ -2504,8 +2509,11 @@ int alfgpu_upload_vertices(alfgpu_t* h, int32_t chain, const alfgpu_vertices* v)
       if (site2[k] >= 0) slist[(size_t)f * 2 * M + fill[site2[k]]++] = 2 * n + 1;
     }
   }
+  if (cplx & 1) h->eexp_complex = 1;
+  if (cplx & 2) h->model_complex = 1;
   int c0 = chain < 0 ? 0 : chain, c1 = chain < 0 ? h->C : chain + 1;
   for (int c = c0; c < c1; ++c) {
+    h->vcplx[c] = cplx;
     CK(cudaMemcpy(h->v_tab + c * K * 15, tab.data(), K * 15 * sizeof(UpdTab), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->v_sptr + (size_t)c * F * (N + 1), sptr.data(), sptr.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->v_slist + (size_t)c * 2 * K, slist.data(), 2 * K * sizeof(int), cudaMemcpyHostToDevice));
@@ -2610,6 +2618,13 @@ int alfgpu_init_state(alfgpu_t* h, double* phase_out) {
   if (!h) return ALFGPU_ERROR_ARGUMENT;
   if (!h->hop_ok || !h->vert_ok || !h->fields_ok) return ALFGPU_ERROR_ARGUMENT;
   CK(cudaSetDevice(h->dev));
+  int8_t cplx = (h->d.reserved[0] & ALFGPU_FLAG_COMPLEX_ARITH) ? 2 : 0;
+  for (int8_t c : h->vcplx) cplx |= c;
+  if (h->eexp_complex != (cplx & 1) || h->model_complex != (cplx >> 1)) {
+    h->eexp_complex = cplx & 1;
+    h->model_complex = cplx >> 1;
+    drop_graphs(h);
+  }
   RET(udv_reset(h, h->udvl));
   RET(udv_reset(h, h->udvr));
   RET(udv_reset(h, h->udvst[h->Nstm - 1]));
