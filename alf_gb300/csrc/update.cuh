@@ -266,7 +266,11 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
     const UpdTab* e = tab + ((long long)n * 5 + so + 2) * 3 + ch;
     s_snew[q] = sn;
     s_prop[q] = 1.5 > u1;  // T0_proposal (Wrapgr_mod.F90:123,133); always true
-    s_u2[q] = uu2;
+    // real models compare the weight with it bit by bit: one zero, and one NaN, which no weight is above
+    long long ub = __double_as_longlong(uu2);
+    if ((ub & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) ub = 0x7ff8000000000000ll;
+    if ((ub << 1) == 0) ub = 0;
+    s_u2[q] = __longlong_as_double(ub);
     const double gr = p.ft.grat[tp - 1][so + 2][sn + 2];
     s_gr[q] = gr;
     zd K = e->expal;
@@ -369,7 +373,8 @@ __global__ void __launch_bounds__(UPD_THREADS) k_update(UpdParams p) {
             }
             Rt.x = r;
             const long long rb = __double_as_longlong(r) & 0x7fffffffffffffffll;
-            a = rb <= 0x7ff0000000000000ll && rb > __double_as_longlong(s_u2[vi]);
+            // an infinite weight is a NaN in complex products (infinity times zero), so not accepted either
+            a = rb < 0x7ff0000000000000ll && rb > __double_as_longlong(s_u2[vi]);
             if (a && __double_as_longlong(r) < 0) ph = zmk(alf_flip(ph.x), alf_flip(ph.y));
           } else {
             const zd Rm64 = A::wide(Rm);
