@@ -1966,7 +1966,7 @@ static int oz_setup(alfgpu_s* h) {
   h->oz_Kpad = oz_roundup(N, OZ_KC);
   h->oz_RpN = oz_roundup(N, OZ_BM);
   h->oz_Rp2N = oz_roundup(2 * N, OZ_BM);
-  // mixed form 55 bits of each row's scale; FP64 form 62, below the roundings of an FP64 product
+  // mixed form 55 bits of each row's scale; FP64 form 62
   const int bits = h->mixed ? OZ_TARGET_BITS : 61;
   if (h->N > 512 || oz_pick(h->oz_Kpad, &h->oz_bits, &h->oz_S, bits) ||
       oz_pick(2 * UPD_KMAX, &h->ozf_bits, &h->ozf_S, bits))

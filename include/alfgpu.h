@@ -54,8 +54,11 @@ enum {
 
 /* Precision forms.  FP64: complex128 throughout; the per-visit Metropolis chain, QRs, solves and
  * phases in FP64 arithmetic, products on the FP64 pipes (mma.sync m8n8k4 f64) or, where their time
- * there is longer, as 62-bit digit-sliced products on the BF16 tensor cores, whose error is below the
- * roundings of an FP64 product (ALFGPU_FLAG_NO_TENSOR_GEMM keeps all of them on the FP64 pipes).
+ * there is longer, as digit-sliced products on the BF16 tensor cores: 62 bits of every row's and
+ * column's scale, combined exactly and rounded once (ALFGPU_FLAG_NO_TENSOR_GEMM keeps all of them on the
+ * FP64 pipes).  Against the largest entries of the row and the column such a product is closer than
+ * an FP64 one; an entry (|A| |B|)_ij far below these (where they do not meet at one k) keeps fewer digits
+ * of its own, 2^-62 of the largest entries where an FP64 product keeps 2^-53 of (|A| |B|)_ij.
  * Models whose vertices are all real run the FP64 kernels in real arithmetic.
  * MIXED: G and all state stay complex128.  By default the G wraps through exp(-dtau T),
  * the UDV propagation products and the stabilisation's complex products (CGR's
@@ -110,7 +113,8 @@ enum { ALFGPU_FLAG_FP64_STAB_GEMM = 256 };
 /* Mixed form: the tensor-core choices made for batched grids (32-wide tiles, the flush and
  * the explicit Q on the tensor cores) also for a grid that does not fill the GPU (by
  * default one chain keeps 16-wide tiles and the double-float flush / FP64 explicit Q,
- * measured faster there). */
+ * measured faster there).  FP64 form: every product that the tensor cores can do, however small (by
+ * default those that take longer on the FP64 pipes). */
 enum { ALFGPU_FLAG_TENSOR_WIDE = 512 };
 /* The exact pivoted QR (ZGEQP3 on one thread-block cluster per matrix) takes clusters of half
  * the default size when the full-size clusters of a batched launch would put more than two
