@@ -1726,7 +1726,7 @@ static int hop_impl(alfgpu_s* h, int up, int with_scale) {
     }
     return 0;
   }
-  if (h->mixed && !(h->oz && real_model(h))) {
+  if (h->mixed) {
     const double* E1 = up ? h->expT : h->expTinv;
     const double* E2 = up ? h->expTinv : h->expT;
     if (up) {
@@ -1820,7 +1820,7 @@ static int update_slice(alfgpu_s* h, int nt1, int dir, int visit_base, const dou
       CKL();
     }
     if (ov && blk > 0) {  // block blk's submatrix after block blk - 1's updates
-      // FP64 in both forms: this submatrix is the block's G0, whose Gamma^-1 sets the next flush
+      // FP64 in both forms: this submatrix is the block's G0, which sets the next flush
       // (double-float here raised the mixed form's largest Precision Green from 9e-6 to 6e-5)
       const int* mprev = h->m + (long long)((blk - 1) & 1) * msz;
       const dim3 gs((UPD_KMAX + 7) / 8, h->B), bs(32, 8);

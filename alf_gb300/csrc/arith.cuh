@@ -55,18 +55,13 @@ struct ArD {
   static ALF_DEV Z neg(Z a) { return zmk(-a.x, -a.y); }
   static ALF_DEV Z mac(Z c, Z a, Z b) { return zfma(a, b, c); }
   static ALF_DEV Z scale(Z a, R s) { return zscale(a, s); }
-  static ALF_DEV R re_mul(Z a, Z b) { return a.x * b.x - a.y * b.y; }
   static ALF_DEV R re(Z a) { return a.x; }
-  static ALF_DEV R absr(R a) { return fabs(a); }
   static ALF_DEV R mulr(R a, R b) { return a * b; }
   static ALF_DEV bool gt(R a, R b) { return a > b; }
   static ALF_DEV Z rcp(Z a) {
     const double s = alf_rcp(a.x * a.x + a.y * a.y);
     return zmk(a.x * s, -a.y * s);
   }
-  // FP64 range holds the unnormalised phase of a block (<= 32 ratio factors); it is
-  // normalised once at block end
-  static ALF_DEV Z renorm(Z a) { return a; }
   static ALF_DEV zd unit(Z a) { const double r = sqrt(a.x * a.x + a.y * a.y); return zmk(a.x / r, a.y / r); }
   static ALF_DEV Z shfl(Z a, int src) {
     return zmk(__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src));
@@ -110,16 +105,10 @@ struct ArF {
   static ALF_DEV Z neg(Z a) { return dfz{df_neg(a.r), df_neg(a.i)}; }
   static ALF_DEV Z mac(Z c, Z a, Z b) { return dz_mac(c, a, b); }
   static ALF_DEV Z scale(Z a, R s) { return dz_scale(a, s); }
-  static ALF_DEV R re_mul(Z a, Z b) { return df_dot2(a.r, b.r, df_neg(a.i), b.i); }
   static ALF_DEV R re(Z a) { return a.r; }
-  static ALF_DEV R absr(R a) { return df_abs(a); }
   static ALF_DEV R mulr(R a, R b) { return df_mul(a, b); }
   static ALF_DEV bool gt(R a, R b) { return df_gt(a, b); }
   static ALF_DEV Z rcp(Z a) { return dz_rcp(a); }
-  static ALF_DEV Z renorm(Z a) {
-    const float m2 = a.r.h * a.r.h + a.i.h * a.i.h;
-    return (m2 > 0.f && m2 < 3e38f) ? dz_scale(a, df_f(rsqrtf(m2))) : a;
-  }
   static ALF_DEV zd unit(Z a) { return dz_wide(dz_unit(a)); }
   static ALF_DEV Z shfl(Z a, int src) {
     Z r;

@@ -34,12 +34,6 @@ ALF_HD zd zdiv(zd a, zd b) {
     return zmk((a.x * r + a.y) / d, (a.y * r - a.x) / d);
   }
 }
-ALF_HD zd zexp(zd a) {
-  double e = exp(a.x);
-  double s, c;
-  sincos(a.y, &s, &c);
-  return zmk(e * c, e * s);
-}
 ALF_HD zd zinv(zd a) { return zdiv(zmk(1.0, 0.0), a); }
 
 // ---------------------------------------------------------------------------

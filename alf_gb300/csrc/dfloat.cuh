@@ -18,8 +18,6 @@ struct dfz {
   dff r, i;
 };
 
-ALF_DEV dff df_f(float x) { return dff{x, 0.f}; }
-
 ALF_DEV dff df_qts(float a, float b) {  // |a| >= |b| or a == 0
   const float s = __fadd_rn(a, b);
   return dff{s, __fsub_rn(b, __fsub_rn(s, a))};
@@ -59,7 +57,6 @@ ALF_DEV dff df_ts(float a, float b) {
   return dff{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
 }
 ALF_DEV dff df_neg(dff a) { return dff{-a.h, -a.l}; }
-ALF_DEV dff df_abs(dff a) { return a.h < 0.f ? df_neg(a) : a; }
 ALF_DEV dff df_add(dff a, dff b) {
   dff s = df_ts(a.h, b.h);
   return df_qts(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
@@ -74,10 +71,6 @@ ALF_DEV float df_perr(dff a, dff b, float p) {
 ALF_DEV dff df_mul(dff a, dff b) {
   const float p = __fmul_rn(a.h, b.h);
   return df_qts(p, df_perr(a, b, p));
-}
-ALF_DEV dff df_mulf(dff a, float b) {
-  const float p = __fmul_rn(a.h, b);
-  return df_qts(p, fmaf(a.l, b, fmaf(a.h, b, -p)));
 }
 // a*b + c*d
 ALF_DEV dff df_dot2(dff a, dff b, dff c, dff d) {

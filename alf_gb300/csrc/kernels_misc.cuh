@@ -217,11 +217,6 @@ __global__ void k_real_to_complex2(const double* a, const double* b, zd* oa, zd*
     ob[i] = zmk(b[i], 0.0);
   }
 }
-// per-batch flush rank: out[c*F + f] = m[c]
-__global__ void k_expand_m(const int* m, int* out, int C, int F) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < C * F) out[b] = m[b / F];
-}
 __global__ void k_count_sweep(double* stat, int C) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < C) stat[8 * c + 7] += 1.0;

@@ -433,8 +433,8 @@ ALF_DEV void oz_tmem_wait(uint32_t (&r)[HB], uint32_t (&q)[HB]) {
   for (int j = 0; j < HB; ++j) asm volatile("" : "+r"(r[j]), "+r"(q[j]));
 }
 
-// 256 threads.  Warp 0 lane 0 is the TMA producer (per K chunk the B slices into one of two
-// buffers, then the A slices into the ring, as they free up), warp 1 lane 0 issues the MMAs and
+// 256 threads.  Warp 0, one elected lane issuing, is the TMA producer (per K chunk the B slices into one of two
+// buffers, then the A slices into the ring, as they free up), warp 1 issues the MMAs the same way and
 // commits each buffer back to the producer; then all eight warps read TMEM: warp w takes TMEM
 // lanes 32 (w % 4) .. + 31 (its sub-partition's) and columns (w / 4) BN/2 .. + BN/2 - 1.
 // Holding one chunk's B slices instead of all of them leaves room, at 16-wide tiles, for two CTAs per

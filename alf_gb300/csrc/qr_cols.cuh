@@ -7,7 +7,7 @@
 #include "linalg.cuh"
 
 #define QRC_WORK 256                 // threads that carry FP64 work: two warps per sub-partition
-#define QRC_THREADS (QRC_WORK + 32)  // and one warp of integer bookkeeping
+#define QRC_THREADS (QRC_WORK + 32)  // and one warp for a step's scalars (FP64) and its exchange
 #ifndef QRC_WAIT_CYCLES
 #define QRC_WAIT_CYCLES (1ll << 31)  // a wait's limit in SM cycles: one second
 #endif

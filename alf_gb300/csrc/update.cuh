@@ -14,16 +14,15 @@
 // vertices.  The kernel keeps Ghat = G(Sblk, Sblk) in shared memory and applies
 // every accepted Sherman-Morrison update to Ghat only; each visit's ratio is
 // then Upgrade2's Mat(1,1) = 1 + Delta (1 - Ghat_jj) read directly.  The effect
-// on the full matrix is the Woodbury form of the same updates,
-//   G = G0 - G0(:,S) Delta_S Gamma^-1 (E_S - G0(S,:)),
-//   Gamma = 1 + (1 - G0(S,S)) Delta_S   (S = accepted sites, in accept order),
-// applied by one rank-m GEMM flush; W = Delta_S Gamma^-1 is formed at block
-// end by the same kernel.
+// on the full matrix is the sum of the same updates over the accepted sites S,
+//   G = G0 - G0(:,S) Y,
+// applied by one rank-m GEMM flush; the kernel leaves the coefficients from which
+// k_flush_xy forms Y by two triangular substitutions (below), without an inverse.
 //
 // G is complex128 in both precision forms.  The per-flavour determinants
 // Mat(1,1) (or the 2x2 determinant of a two-site vertex), the Ghat rank-1 updates
-// and Gamma^-1 run in FP64 (plain form) or double-float (mixed form, dfloat.cuh,
-// ~2^-46 relative rounding).  The accumulation of the Metropolis ratio (the
+// and the coefficients run in FP64 (plain form) or double-float (mixed form,
+// dfloat.cuh, ~2^-46 relative rounding), real ones on models that are real.  The accumulation of the Metropolis ratio (the
 // product over flavours, exp(Z1 alpha), the N_SUN power and the gamma ratio), the
 // weight test and the phase are FP64 in both forms.  GB300's FP64 dependent
 // latency (63-76 cycles, ~560 for a division) sets the cost of every visit, so

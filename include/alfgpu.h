@@ -139,8 +139,8 @@ enum { ALFGPU_FLAG_NO_OVERLAP = 16384 };
  * one k_update CTA share an SM (the next block's visits overlap the flush).  This flag keeps the
  * 32-wide tiles of one CTA per SM (and the serial order of visits and flush). */
 enum { ALFGPU_FLAG_OZ_FLUSH_SINGLE = 32768 };
-/* Mixed form: the per-visit Metropolis arithmetic, the block-submatrix updates, Gamma^-1 and
- * the flush operand Y in FP64 (k_update<ArD>) instead of double-float. */
+/* Mixed form: the per-visit Metropolis arithmetic, the block-submatrix updates and the flush
+ * operand Y in FP64 (k_update, k_flush_xy) instead of double-float. */
 enum { ALFGPU_FLAG_FP64_VISITS = 65536 };
 /* Mixed form: the K = N_dim tensor-core products (G wraps, UDV propagation, stabilisation
  * products) on 16-wide tiles with the deeper A ring of one-chain grids, also on batched grids. */
