@@ -10,7 +10,9 @@ value:     aggregate sweeps/s of the batched mixed form: C chains (16 by default
            handle, all state resident on the device, timed with CUDA events on the
            library's stream (device draw stream, L2 flushed between steps).
 fp64:      the same for the plain FP64 form on the same workload and chain count, and
-           mixed_over_fp64 = value / fp64.value (the spec ratio).
+           mixed_over_fp64 = value / fp64.value.
+fp64_pipes: the plain form with every product on the FP64 pipes (ALFGPU_FLAG_NO_TENSOR_GEMM)
+           on the same chains, and mixed_over_fp64_pipes.
 per_chain: one chain per handle in both forms (the single-chain rate).
 vs_fp64:   max |G_mixed - G_fp64| after one sweep on identical fields and draws.
 e2e:       the headline through the C ABI with host buffers: each step copies every
@@ -166,11 +168,16 @@ def real_model(m) -> bool:
     return not np.any(np.imag(np.asarray(m.pack()["op_Eexp"])))
 
 
-def wraps_on_tensor(m, chains: int, precision: str) -> bool:
-    """Whether the G wraps run on the tensor cores: always in the mixed form, in the FP64 form where
-    the FP64 MMAs of one product would take 8 us or more (alfgpu.cu oz_pays)."""
+def product_on_tensor(m, chains: int, precision: str, zmul: int) -> bool:
+    """Whether an N x N x N product (zmul FP64 MMAs per complex one: 2 with a real factor, 4) runs on the
+    tensor cores: always in the mixed form, in the FP64 form where its FP64 MMAs would take 8 us or
+    more (alfgpu.cu oz_pays)."""
     n8, b = (m.ndim + 7) // 8, chains * m.n_fl
-    return precision != "fp64" or n8 * n8 * ((m.ndim + 3) // 4) * b * (1 if real_model(m) else 2) * 0.30 / 608 >= 8.0
+    return precision != "fp64" or n8 * n8 * ((m.ndim + 3) // 4) * b * (1 if real_model(m) else zmul) * 0.30 / 608 >= 8.0
+
+
+def wraps_on_tensor(m, chains: int, precision: str) -> bool:
+    return product_on_tensor(m, chains, precision, 2)
 
 
 def roofline(precision: str, chains: int, m, prof):
@@ -267,9 +274,49 @@ def sweep_roofline_groups(groups, ms_per_step: float, precision: str, p_fp64: fl
             "frac": 1e3 * t / ms_per_step if ms_per_step > 0 else None,
             "achieved_tflops": total / (ms_per_step / 1e3) / 1e12 if ms_per_step > 0 else None,
             "peaks_tflops": {"fp64": p_fp64, "bf16": p_bf16},
-            "basis": "FP64 phases at the measured FP64 MMA rate" + (
-                "" if precision == "fp64" else "; wraps, propagation and flushes at the measured BF16 peak") +
-            "; the FLOPs are the reference's complex operations, of which real models execute a quarter to a half"}
+            "basis": "the reference's complex operations (real models execute a quarter to a half of them); FP64 phases "
+                     "at the measured FP64 MMA rate" + (
+                "" if precision == "fp64" else "; wraps, propagation and flushes at the measured BF16 peak")}
+
+
+def reference_operations(groups, ms_per_step: float) -> dict:
+    """The reference's complex operations of one step and their rate: a speed-up figure, no roofline."""
+    r = sweep_roofline_groups(groups, ms_per_step, "fp64", FP64_DMMA_TFLOPS, FP64_DMMA_TFLOPS)
+    return {k: r[k] for k in ("flops_per_step", "flops_by_phase", "achieved_tflops")}
+
+
+def executed_roofline(groups, ms_per_step: float, precision: str, p_fp64: float, p_bf16: float) -> dict:
+    """Roofline of one step over the operations that are executed, groups as in
+    sweep_roofline_groups: real models run a quarter of sweep_flops' complex operations, half of
+    those of a product with a real exponential, and every phase is charged to the unit it runs
+    on.  Products (wraps, propagation, flushes, 4 of decompose's 14.7 N^3 and 29.3 of CGR's 44) at
+    the BF16 peak over the digit products per product where they run on the tensor cores; QRs, Q,
+    solves and CGR2_2 at the FP64 MMA rate.  The visits' serial chain is not in it."""
+    if isinstance(groups, Exception):
+        raise groups
+    t = {"fp64": 0.0, "tensor": 0.0}
+    fl = {"fp64": 0.0, "tensor": 0.0}
+    for m, n_acc, ltau, chains in groups:
+        f = sweep_flops(m, n_acc, ltau)
+        half, quarter = (0.5, 0.25) if real_model(m) else (1.0, 1.0)
+        _, _, pairs = digit_pairs(m.ndim, 61 if precision == "fp64" else 54) if m.ndim <= 512 else (0, 0, 0)
+        stab = 4.0 / 14.7 * f["decompose"] + 2.0 / 3.0 * f["cgr"]
+        parts = [(f["wraps"] + f["propagate"] + f.get("tau_wraps", 0.0), half, 2), (stab, quarter, 4),
+                 (f["rank1"], quarter, 2),
+                 (f["decompose"] + f["cgr"] - stab + f.get("tau_cgr2_2", 0.0), quarter, 0)]
+        for flops, share, zmul in parts:
+            unit = "tensor" if zmul and pairs and product_on_tensor(m, chains, precision, zmul) else "fp64"
+            fl[unit] += chains * flops * share
+            t[unit] += chains * flops * share / ((p_bf16 / pairs if unit == "tensor" else p_fp64) * 1e12)
+    frac = 1e3 * sum(t.values()) / ms_per_step if ms_per_step > 0 else None
+    if frac is not None and frac > 1.0:
+        raise ValueError(f"{frac:.3f} of the roofline: more operations counted than executed")
+    return {"flops_per_step": sum(fl.values()), "flops_by_unit": fl, "t_roof_ms": 1e3 * sum(t.values()),
+            "t_roof_by_unit_ms": {k: 1e3 * v for k, v in t.items()}, "ms_per_step": ms_per_step, "frac": frac,
+            "peaks_tflops": {"fp64": p_fp64, "bf16": p_bf16},
+            "basis": "operations executed (real arithmetic on real models); products at the measured BF16 peak over the "
+                     "digit products per product where they run on the tensor cores, the rest at the measured FP64 MMA "
+                     "rate; the visits' serial chain not counted"}
 
 
 def workload_model(name: str):
@@ -538,8 +585,9 @@ def form_summary(ws, r) -> dict:
                     for k, v in r["prof"].items()},
          "precision_green": r["precision_green"], "acceptance": r["acceptance"],
          "roofline": _reported(roofline, r["precision"], r["chains"], m, r["prof"]),
-         "sweep_roofline": _reported(sweep_roofline, m, r["n_acc"], r["ltau"], r["chains"], ms_step, r["precision"],
-                                     FP64_DMMA_TFLOPS, measured_bf16_peak()[0])}
+         "sweep_roofline": _reported(executed_roofline, [(m, r["n_acc"], r["ltau"], r["chains"])], ms_step,
+                                     r["precision"], FP64_DMMA_TFLOPS, measured_bf16_peak()[0]),
+         "reference_operations": _reported(reference_operations, [(m, r["n_acc"], r["ltau"], r["chains"])], ms_step)}
     if r["t_e2e"]:
         d["e2e"] = replicas.whole_job_rate(ws, r["chains"], r["steps"], r["t_e2e"])
     return d
@@ -688,8 +736,9 @@ def batch_summary(ws, rb, precision) -> dict:
     d = {"value": ws * rb["nchains"] * rb["steps"] / rb["t_dev"], "unit": "sweeps/s", "chains_per_gpu": rb["nchains"],
          "steps": rb["steps"], "ms_per_step": ms_step, "gpu_launches": int(rb["launches"]), "clocks": rb["clocks"],
          "groups": rb["groups"], "precision_green": {"xmaxG": rb["xmaxG"]},
-         "sweep_roofline": _reported(sweep_roofline_groups, rb["rgroups"], ms_step, precision, FP64_DMMA_TFLOPS,
-                                     measured_bf16_peak()[0])}
+         "sweep_roofline": _reported(executed_roofline, rb["rgroups"], ms_step, precision, FP64_DMMA_TFLOPS,
+                                     measured_bf16_peak()[0]),
+         "reference_operations": _reported(reference_operations, rb["rgroups"], ms_step)}
     if rb["t_e2e"]:
         d["e2e"] = ws * rb["nchains"] * rb["steps"] / rb["t_e2e"]
     return d
@@ -753,6 +802,7 @@ def main():
         print(json.dumps(line))
         return
 
+    from alf_gb300.sweep import FLAG_NO_TENSOR_GEMM
     other = "fp64" if args.precision == "mixed" else "mixed"
     cmp_steps, cmp_warm = min(args.steps, 5), min(args.warmup, 3)
     if args.config == "batch128":
@@ -777,7 +827,8 @@ def main():
             "e2e": {"value": head.get("e2e"), "unit": "sweeps/s", "h2d_bytes_per_step": rb["h2d"],
                     "d2h_bytes_per_step": rb["d2h"]},
             "roofline": None, "cpu_baseline": cpu, "clocks": head["clocks"], "gpu_launches": head["gpu_launches"],
-            "precision_green": head["precision_green"], "sweep_roofline": head["sweep_roofline"]})
+            "precision_green": head["precision_green"], "sweep_roofline": head["sweep_roofline"],
+            "reference_operations": head["reference_operations"]})
         if other_sum is not None:
             line[other] = other_sum
             line["mixed_over_fp64"] = (head["value"] / other_sum["value"] if args.precision == "mixed"
@@ -797,6 +848,14 @@ def main():
         extra[other] = form_summary(ws, ro)
         extra["mixed_over_fp64"] = (head["value"] / extra[other]["value"] if args.precision == "mixed"
                                     else extra[other]["value"] / head["value"])
+        # the plain form with every product on the FP64 pipes
+        pipes = argparse.Namespace(**dict(vars(args), flags=args.flags | FLAG_NO_TENSOR_GEMM, tune=0))
+        fp = _reported(lambda: form_summary(ws, run_ours(pipes, ws, rank, local, "fp64", args.chains, min(args.steps, 2), 1,
+                                                         e2e=False)))
+        extra["fp64_pipes"] = fp if "failed" in fp else {k: fp[k] for k in ("value", "unit", "steps", "ms_per_step", "clocks",
+                                                                             "precision_green")}
+        if "failed" not in fp:
+            extra["mixed_over_fp64_pipes"] = (head if args.precision == "mixed" else extra[other])["value"] / fp["value"]
         if args.chains > 1:
             pc = {}
             for prec in ("fp64", "mixed"):
@@ -826,7 +885,7 @@ def main():
         "roofline": head["roofline"], "cpu_baseline": cpu, "clocks": head["clocks"],
         "gpu_launches": head["gpu_launches"], "phases": head["phases"], "precision_green": head["precision_green"],
         "acceptance": head["acceptance"], "per_chain_sweeps_per_s": head["per_chain_sweeps_per_s"],
-        "sweep_roofline": head["sweep_roofline"]})
+        "sweep_roofline": head["sweep_roofline"], "reference_operations": head["reference_operations"]})
     if r.get("meas"):
         line["measuring_sweeps"] = r["meas"]
     line.update(extra)
