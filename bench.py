@@ -156,10 +156,12 @@ class ClockSampler:
 def digit_pairs(n: int, target: int = 54):
     """(bits, slices, digit products per algorithmic product) of the digit-sliced tensor-core GEMM
     at inner dimension n, as the library picks them (ozaki.cuh oz_pick); target 54 in the mixed
-    form, 61 in the FP64 form."""
+    form, 61 in the FP64 form.  Zeros where the library has none (n > 512; FP64 form n > 448)."""
     kpad = (n + 63) // 64 * 64
-    bits, S = next((b, (target + b) // b) for b in range(8, 3, -1)
-                   if (target + b) // b * b <= 63 and (target + b) // b * kpad * 4 ** (b - 1) <= 2 ** 24)
+    bits, S = next(((b, (target + b) // b) for b in range(8, 3, -1) if n <= 512 and
+                    (target + b) // b * b <= 63 and (target + b) // b * kpad * 4 ** (b - 1) <= 2 ** 24), (0, 0))
+    if not S:
+        return 0, 0, 0
     return bits, S, S * (S + 1) // 2 + (S - 1)
 
 
@@ -172,6 +174,8 @@ def product_on_tensor(m, chains: int, precision: str, zmul: int) -> bool:
     """Whether an N x N x N product (zmul FP64 MMAs per complex one: 2 with a real factor, 4) runs on the
     tensor cores: always in the mixed form, in the FP64 form where its FP64 MMAs would take 8 us or
     more (alfgpu.cu oz_pays)."""
+    if not digit_pairs(m.ndim, 61 if precision == "fp64" else 54)[1]:
+        return False
     n8, b = (m.ndim + 7) // 8, chains * m.n_fl
     return precision != "fp64" or n8 * n8 * ((m.ndim + 3) // 4) * b * (1 if real_model(m) else zmul) * 0.30 / 608 >= 8.0
 
@@ -299,13 +303,13 @@ def executed_roofline(groups, ms_per_step: float, precision: str, p_fp64: float,
     for m, n_acc, ltau, chains in groups:
         f = sweep_flops(m, n_acc, ltau)
         half, quarter = (0.5, 0.25) if real_model(m) else (1.0, 1.0)
-        _, _, pairs = digit_pairs(m.ndim, 61 if precision == "fp64" else 54) if m.ndim <= 512 else (0, 0, 0)
+        _, _, pairs = digit_pairs(m.ndim, 61 if precision == "fp64" else 54)
         stab = 4.0 / 14.7 * f["decompose"] + 2.0 / 3.0 * f["cgr"]
         parts = [(f["wraps"] + f["propagate"] + f.get("tau_wraps", 0.0), half, 2), (stab, quarter, 4),
                  (f["rank1"], quarter, 2),
                  (f["decompose"] + f["cgr"] - stab + f.get("tau_cgr2_2", 0.0), quarter, 0)]
         for flops, share, zmul in parts:
-            unit = "tensor" if zmul and pairs and product_on_tensor(m, chains, precision, zmul) else "fp64"
+            unit = "tensor" if zmul and product_on_tensor(m, chains, precision, zmul) else "fp64"
             fl[unit] += chains * flops * share
             t[unit] += chains * flops * share / ((p_bf16 / pairs if unit == "tensor" else p_fp64) * 1e12)
     frac = 1e3 * sum(t.values()) / ms_per_step if ms_per_step > 0 else None

@@ -41,3 +41,18 @@ def test_reported_beside_each_other():
     json.dumps(bench.executed_roofline([(mdl.config("hubbard4x4"), 100.0, 0, 1)], 4.5, "fp64", 1.0, 1900.0))
     assert set(bench.reference_operations([(mdl.config("hubbard4x4"), 100.0, 0, 1)], 4.5)) == {
         "flops_per_step", "flops_by_phase", "achieved_tflops"}
+
+
+# digits as the library picks them, and none where it has none
+@pytest.mark.parametrize("n,target,want", [(16, 54, (8, 7, 34)), (128, 54, (8, 7, 34)), (256, 54, (7, 8, 43)),
+                                           (512, 54, (7, 8, 43)), (513, 54, (0, 0, 0)), (256, 61, (7, 9, 53)),
+                                           (448, 61, (7, 9, 53)), (449, 61, (0, 0, 0))])
+def test_digit_pairs(n, target, want):
+    assert bench.digit_pairs(n, target) == want
+
+
+def test_large_systems_on_the_fp64_pipes():
+    m = mdl.hubbard("square", 22, 22, beta=0.2)  # N = 484: no 62-bit digits
+    r = bench.executed_roofline([(m, 100.0, 0, 8)], 1e6, "fp64", 1.0, 1900.0)
+    assert r["flops_by_unit"]["tensor"] == 0.0
+    assert bench.executed_roofline([(m, 100.0, 0, 8)], 1e6, "mixed", 1.0, 1900.0)["flops_by_unit"]["tensor"] > 0.0
