@@ -116,15 +116,17 @@ enum { ALFGPU_FLAG_FP64_STAB_GEMM = 256 };
  * measured faster there).  FP64 form: every product that the tensor cores can do, however small (by
  * default those that take longer on the FP64 pipes). */
 enum { ALFGPU_FLAG_TENSOR_WIDE = 512 };
-/* The exact pivoted QR (ZGEQP3 on one thread-block cluster per matrix) takes clusters of half
- * the default size when the full-size clusters of a batched launch would put more than two
- * CTAs on every SM; these flags force the half-size or the full-size cluster. */
+/* The exact pivoted QR (ZGEQP3 on one thread-block cluster per matrix) keeps columns in its CTAs' shared
+ * memory where they fit; else, for batched complex matrices whose clusters would need a second
+ * wave, and with any of the QR flags below, it is the row-distributed kernel (complex arithmetic).
+ * That one takes clusters of half the default size when the full-size clusters of a batched launch
+ * would put more than two CTAs on every SM; these flags force the half-size or the full-size cluster. */
 enum { ALFGPU_FLAG_QR_HALF_CLUSTER = 1024, ALFGPU_FLAG_QR_FULL_CLUSTER = 2048 };
 /* Mixed form, grids of several chains: the delayed-update flush G -= X Y on the double-float
  * GEMM, whose loop stops at the block's accepted count, instead of the tensor-core GEMM
  * (K padded to 64, digit-sliced). */
 enum { ALFGPU_FLAG_DF_FLUSH = 4096 };
-/* The exact pivoted QR keeps each CTA's rows in a global (L2-resident) workspace even where
+/* The row-distributed QR keeps each CTA's rows in a global (L2-resident) workspace even where
  * they fit in shared memory.  A CTA then needs little shared memory, so several clusters share
  * an SM; by default this layout is taken when it needs fewer waves of clusters than rows in
  * shared memory (batched grids), and this flag takes it always. */
@@ -148,7 +150,7 @@ enum { ALFGPU_FLAG_OZ_DEEP_RING = 131072 };
 /* Mixed form, grids of several chains: accepted, without effect (it selected persistent K = 64 products
  * that kept their A digit slices from one tile to the next; the paired tiles replaced them). */
 enum { ALFGPU_FLAG_OZ_FLUSH_RESIDENT = 262144 };
-/* The exact pivoted QR applies each step's reflector and forms the next step's partial sums in
+/* The row-distributed QR applies each step's reflector and forms the next step's partial sums in
  * two passes over the rows (by default one pass does both, the next pivot chosen first). */
 enum { ALFGPU_FLAG_QR_TWO_PASS = 524288 };
 /* Models whose vertex exponentials and transition factors are all real keep every matrix of the
