@@ -292,12 +292,15 @@ ALF_DEV bool oz_mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after ~2^31 SM cycles (about one second) and returns false.
+#ifndef OZ_WAIT_CYCLES
+#define OZ_WAIT_CYCLES (1ll << 31)  // a wait's limit in SM cycles: one second
+#endif
+// Bounded wait: gives up after OZ_WAIT_CYCLES and returns false.
 ALF_DEV bool oz_mbar_wait(uint32_t bar, uint32_t parity) {
   if (oz_mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   while (!oz_mbar_try(bar, parity))
-    if (clock64() - t0 > (1ll << 31)) return false;
+    if (clock64() - t0 > OZ_WAIT_CYCLES) return false;
   return true;
 }
 // The same for a converged warp: one answer for all its lanes.
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_
     if (!ok && lane == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
     __syncwarp();
     if (__any_sync(0xffffffffu, *abort_flag)) {  // let every copy issued by this warp land before the CTA exits
-      for (int q = gb0; q < gb0 + bloaded; ++q) oz_mbar_wait(bfull0 + 8u * (uint32_t)(q % NB), (uint32_t)((q / NB) & 1));
+      for (int q = gb0 + max(0, bloaded - NB); q < gb0 + bloaded; ++q) oz_mbar_wait(bfull0 + 8u * (uint32_t)(q % NB), (uint32_t)((q / NB) & 1));
       for (int q = g0 + *consumed_sh; q < g0 + loaded; ++q)
         oz_mbar_wait(full0 + 8u * (uint32_t)(q % NST), (uint32_t)((q / NST) & 1));
     }
@@ -625,10 +628,10 @@ __global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_
     for (int j = 0; j < HB; ++j)
       old[j] = (m < p.M && n0 + c0 + j < p.N) ? o[m * p.ldr + (n0 + c0 + j) * p.ldc].x : 0.0;
   }
-  const bool done_ok = oz_mbar_wait(done, tpar);
+  const bool mine_ok = oz_mbar_wait(done, tpar);
   oz_fence_after();
-  __syncthreads();
-  if (!done_ok && lane == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
+  const bool done_ok = __syncthreads_and(mine_ok) != 0;  // one answer for the CTA: TMEM loads are warp-wide
+  if (!done_ok && tid == 0) { atomicOr(p.err, 4); *abort_flag = 1; }
   if (done_ok && !*abort_flag) {
     // The diagonals in two exact 64-bit words, the last lg of them in the low one.
     long long Zh[HB], Zl[HB];

@@ -1,8 +1,9 @@
-"""Bounded waits of the column-distributed pivoted QR: a cluster that misses a message gives up,
-the call reports it, and the device stays usable.
+"""Bounded waits of the column-distributed pivoted QR and of the tensor-core product: a cluster (a CTA)
+that misses a message gives up, the call reports it, and the device stays usable.
 
 The library is built once more from a copy of its sources in which CTA 1 of a cluster never posts
-its candidate column, with waits of about two milliseconds: every wait on it runs out."""
+its candidate column, and products with 77 rows never signal their end, with waits of about two
+milliseconds: every wait on these runs out."""
 import ctypes
 import os
 import shutil
@@ -15,7 +16,9 @@ from alf_gb300.sweep import Chains
 
 pytestmark = pytest.mark.gpu
 
-POST = "if (lane < (int)CL && lane != (int)rank) qrc_push16("
+PATCHES = {"qr_cols.cuh": ("if (lane < (int)CL && lane != (int)rank) qrc_push16(",
+                           "if (rank != 1 && lane < (int)CL && lane != (int)rank) qrc_push16("),
+           "ozaki.cuh": ("if (oz_elect()) oz_commit(done);", "if (p.M != 77 && oz_elect()) oz_commit(done);")}
 
 
 @pytest.fixture(scope="module")
@@ -26,14 +29,15 @@ def silent():
     shutil.rmtree(root, ignore_errors=True)
     shutil.copytree(build.CSRC, os.path.join(root, "alf_gb300", "csrc"))
     shutil.copytree(os.path.dirname(_lib.HEADER), os.path.join(root, "include"))
-    qr = os.path.join(root, "alf_gb300", "csrc", "qr_cols.cuh")
-    with open(qr) as f:
-        txt = f.read()
-    assert txt.count(POST) == 1
-    with open(qr, "w") as f:
-        f.write(txt.replace(POST, POST.replace("(lane <", "(rank != 1 && lane <")))
+    for name, (old, new) in PATCHES.items():
+        path = os.path.join(root, "alf_gb300", "csrc", name)
+        with open(path) as f:
+            txt = f.read()
+        assert txt.count(old) == 1
+        with open(path, "w") as f:
+            f.write(txt.replace(old, new))
     load("silent", os.path.join(root, "alf_gb300", "csrc", "alfgpu.cu"),
-         ("-DQRC_WAIT_CYCLES=(1ll<<22)", "-Xptxas", "-O1"))
+         ("-DQRC_WAIT_CYCLES=(1ll<<22)", "-DOZ_WAIT_CYCLES=(1ll<<22)", "-Xptxas", "-O1"))
     path = os.path.join(HERE, "_build", "silent.so")
 
     class Use:
@@ -91,3 +95,24 @@ def test_one_shot_calls_report_it(silent, N):
     (G, ph), dec = sweep.cgr(1, U, D, V, U, D, V), sweep.decompose("r", U, D, V)
     assert np.array_equal(G, want[0][0]) and ph == want[0][1]
     assert all(np.array_equal(a, b) for a, b in zip(dec, want[1]))
+
+
+# one and several tiles, one and several K chunks; a product with another row count ends as ever
+@pytest.mark.parametrize("n,k", [(5, 9), (300, 200), (64, 448)])
+def test_products_report_a_missing_end(silent, n, k):
+    r = np.random.default_rng(n + k)
+
+    def product(m):
+        A, B = np.asfortranarray(r.standard_normal((m, k))), np.asfortranarray(r.standard_normal((k, n)))
+        C = np.full((m, n), 7.0, order="F")
+        p = lambda a: ctypes.c_void_p(a.ctypes.data)
+        rc = _lib.lib().alfgpu_oz_dgemm(m, n, k, p(A), m, p(B), k, p(C), m, 0)
+        return rc, C, A @ B
+
+    with silent:
+        rc, C, _ = product(77)
+        assert rc == 104 and np.all(C == 7.0)
+        rc, C, want = product(78)
+        assert rc == 0 and np.max(np.abs(C - want)) < 1e-12 * k
+    rc, C, want = product(77)
+    assert rc == 0 and np.max(np.abs(C - want)) < 1e-12 * k
