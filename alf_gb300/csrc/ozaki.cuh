@@ -445,6 +445,9 @@ ALF_DEV void oz_tmem_wait(uint32_t (&r)[HB], uint32_t (&q)[HB]) {
 // pairs 64 us, 32-wide with nine stages 67 us; two matrices 16 us and 19 us (start: 32-wide tiles with all B
 // slices resident and one issuing thread, 105 us per real half of a complex product).  The ring's depth
 // (2 .. 9) makes no difference: a chunk of 4 K steps takes ~450 cycles to issue.
+// <16, true> has 104 registers a thread: two CTAs leave 12,288 of the SM's, what a CTA of the real visits in
+// double-float takes (48 a thread), so the next block's visits start beside a flush.  With 105 (allocated as
+// 112) they waited for it: 16 chains of 16 x 16, mixed, 317 ms a sweep for 306.
 template <int BN, bool PERSIST = false>
 __global__ void __launch_bounds__(256, BN == 16 ? 2 : 1) k_oz_gemm(const __grid_constant__ CUtensorMap tmA,
                                                     const __grid_constant__ CUtensorMap tmB, OzGemmParams p) {
